@@ -108,17 +108,14 @@ class WarmStartNet:
         return {k: v.detach().cpu().numpy().astype(np.float64) for k, v in self.p.items()}
 
     # ---------------------------------------------------------------- layers
-    def _conv(self, name, X, Y, N, H, W, relu=True):
-        """Y slice = act(conv3x3(X slice)); X, Y = (tensor, channel stride, offset, channels)."""
+    def _conv(self, name, X, Y, N, H, W, relu=True, up=None):
+        """Y slice = act(conv3x3(X slice)); X, Y = (tensor, channel stride, offset, channels). up (tensor, channel
+        stride, offset): also the x2 nearest-neighbour upsampled Y."""
         xt, xcs, xc0, ci = X; yt, ycs, yc0, co = Y
-        P = N * H * W; K9 = 9 * ci
-        col = self._ws('col', P * K9, torch.bfloat16)
-        call('blml_nn_im2col', xt.data_ptr(), N, H, W, xcs, xc0, ci, col.data_ptr(), 0, self.st)
-        Cm = self._ws('C', P * co, torch.float32)
-        call('blml_nn_gemm_bf16', col.data_ptr(), self.wb[name].data_ptr(), Cm.data_ptr(), P, co, K9, 1,
-             self.err.data_ptr(), self.st)
-        call('blml_nn_bias_act', Cm.data_ptr(), 1, P, co, self.p[name + '.b'].data_ptr(), int(relu), yt.data_ptr(),
-             ycs, yc0, self.st)
+        ut, ucs, uc0 = (None, 0, 0) if up is None else up
+        call('blml_nn_conv3x3', xt.data_ptr(), N, H, W, xcs, xc0, ci, self.wb[name].data_ptr(),
+             self.p[name + '.b'].data_ptr(), int(relu), co, yt.data_ptr(), ycs, yc0,
+             None if ut is None else ut.data_ptr(), ucs, uc0, self.err.data_ptr(), self.st)
 
     def _conv_bwd(self, name, X, Y, dY, dX, N, H, W):
         """Gradients of a conv + ReLU layer: weights and bias into self.g, the input's gradient into the dX slice
@@ -171,14 +168,11 @@ class WarmStartNet:
         self._conv('enc3b', (A['a3'], 128, 0, 128), (A['cat3'], 384, 256, 128), N, H4, W4)
         call('blml_nn_pool_fwd', A['cat3'].data_ptr(), N, H4, W4, 384, 256, 128, A['p3'].data_ptr(), 128, 0, st)
         self._conv('bot1', (A['p3'], 128, 0, 128), (A['b1'], 256, 0, 256), N, H8, W8)
-        self._conv('bot2', (A['b1'], 256, 0, 256), (A['b2'], 256, 0, 256), N, H8, W8)
-        call('blml_nn_up_fwd', A['b2'].data_ptr(), N, H8, W8, 256, A['cat3'].data_ptr(), 384, 0, st)
+        self._conv('bot2', (A['b1'], 256, 0, 256), (A['b2'], 256, 0, 256), N, H8, W8, up=(A['cat3'], 384, 0))
         self._conv('dec3a', (A['cat3'], 384, 0, 384), (A['d3a'], 128, 0, 128), N, H4, W4)
-        self._conv('dec3b', (A['d3a'], 128, 0, 128), (A['d3'], 128, 0, 128), N, H4, W4)
-        call('blml_nn_up_fwd', A['d3'].data_ptr(), N, H4, W4, 128, A['cat2'].data_ptr(), 192, 0, st)
+        self._conv('dec3b', (A['d3a'], 128, 0, 128), (A['d3'], 128, 0, 128), N, H4, W4, up=(A['cat2'], 192, 0))
         self._conv('dec2a', (A['cat2'], 192, 0, 192), (A['d2a'], 64, 0, 64), N, H2, W2)
-        self._conv('dec2b', (A['d2a'], 64, 0, 64), (A['d2'], 64, 0, 64), N, H2, W2)
-        call('blml_nn_up_fwd', A['d2'].data_ptr(), N, H2, W2, 64, A['cat1'].data_ptr(), 96, 0, st)
+        self._conv('dec2b', (A['d2a'], 64, 0, 64), (A['d2'], 64, 0, 64), N, H2, W2, up=(A['cat1'], 96, 0))
         self._conv('dec1a', (A['cat1'], 96, 0, 96), (A['d1a'], 32, 0, 32), N, H, W)
         self._conv('dec1b', (A['d1a'], 32, 0, 32), (A['d1'], 32, 0, 32), N, H, W)
         u = self._act('u', P1 * 2, torch.float32)

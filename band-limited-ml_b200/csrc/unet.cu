@@ -12,51 +12,9 @@
 // 128-byte-swizzled 64-deep K slices into a ring of up to 8 stages, one elected thread issuing kind::f16 MMAs (M 128,
 // N <= 256, K 16) into one of two TMEM accumulators, tcgen05.ld epilogue overlapping the next tile's MMAs. Waits are bounded: on timeout the kernel sets the caller's error word, gives
 // copies and MMAs in flight one more bounded wait, frees its tensor memory and returns.
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <string.h>
-#include <vector>
-#include "common.cuh"
+#include "nn_tc.cuh"
 
 namespace blml {
-
-constexpr int NN_BM = 128, NN_BK = 64;
-
-__device__ __forceinline__ uint32_t nn_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void nn_mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(nn_smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void nn_mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(nn_smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool nn_mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (long it = 0; it < (1L << 20); it++) {
-    uint32_t done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done) : "r"(nn_smem_u32(bar)), "r"(parity) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void nn_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-               :: "r"(nn_smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(nn_smem_u32(bar)) : "memory");
-}
-// K-major, 128-byte-swizzled operand tile: 8-row core groups 1024 bytes apart
-__device__ __forceinline__ uint64_t nn_desc(const void* p) {
-  const uint64_t addr = nn_smem_u32(p);
-  uint64_t d = 0;
-  d |= (addr >> 4) & 0x3FFFull;
-  d |= (uint64_t)(16 >> 4) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// kind::f16 instruction descriptor: D f32, A and B bf16, both K-major, M = 128, N = n
-__host__ __device__ constexpr uint32_t idesc_bf16(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(NN_BM >> 4) << 24);
-}
 
 // C[z][m][n] = sum_{k in split z} A[m][k] B[n][k]. Persistent, one CTA per SM (its shared memory keeps a second
 // one out), warp-specialised over a ring of `stages` shared-memory K slices and two TMEM accumulators:
@@ -69,31 +27,6 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int n) {
 // walked t = blockIdx.x, blockIdx.x + gridDim.x, ... with the n tile fastest, so the CTAs that share an A tile run
 // at the same time and the second read of it comes from L2. Tiles whose split has an empty K range are written as
 // zeros by the epilogue and skipped by the other roles.
-constexpr int NN_PIPE_THREADS = 192, NN_MAX_STAGES = 8;
-
-struct NNPipeShared {
-  uint64_t full[NN_MAX_STAGES], empty[NN_MAX_STAGES], tfull[2], tempty[2];
-  uint32_t tslot;
-  int abort;
-  long long issued, consumed;           // K slices loaded by the producer / taken by the MMA issuer
-};
-
-__device__ __forceinline__ bool nn_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  for (long it = 0; it < (1L << 20); it++) {
-    uint32_t done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done) : "r"(nn_smem_u32(bar)), "r"(parity) : "memory");
-    if (done) return true;
-    if ((it & 63) == 63 && abort && *abort) return false;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void nn_fail(volatile int* abort, int* err) {
-  *abort = 1;
-  atomicExch(err, 1);
-}
-
 __global__ void __launch_bounds__(NN_PIPE_THREADS, 1) k_gemm_bf16(const __grid_constant__ CUtensorMap mA,
                                                                   const __grid_constant__ CUtensorMap mB, int M, int N,
                                                                   int NT, int tcols, int nkb, int kb_per_split,
@@ -345,6 +278,34 @@ __global__ void k_pool_fwd(const __nv_bfloat16* __restrict__ X, int Nb, int H, i
   Y[q * Csy + c0y + c] = __float2bfloat16(0.25f * s);
 }
 
+// the same, 8 channels (16 bytes) per thread
+__global__ void k_pool_fwd8(const uint4* __restrict__ X, int Nb, int H, int W, int Csx, int c0x, int C,
+                            uint4* __restrict__ Y, int Csy, int c0y) {       // strides and offsets in 8-channel units
+  const int h = H / 2, w = W / 2;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (int64_t)Nb * h * w * C) return;
+  const unsigned c = (unsigned)(i % C); const int64_t q = i / C;
+  const unsigned x = (unsigned)(q % w); const int64_t r = q / w;             // r = n h + y
+  uint4 v[4];
+#pragma unroll
+  for (int a = 0; a < 2; a++)
+#pragma unroll
+    for (int b = 0; b < 2; b++) v[2 * a + b] = __ldg(X + ((2 * r + a) * W + 2 * x + b) * Csx + c0x + c);
+  uint4 o;
+  __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&v[j])[k]);
+      s.x += f.x; s.y += f.y;
+    }
+    op[k] = __floats2bfloat162_rn(0.25f * s.x, 0.25f * s.y);
+  }
+  Y[q * Csy + c0y + c] = o;
+}
+
 // its gradient, added into dX (the encoder output's gradient also receives the skip path's)
 __global__ void k_pool_bwd_add(const float* __restrict__ dY, int Nb, int H, int W, int C, float* __restrict__ dX,
                                int Csx, int c0x) {
@@ -388,6 +349,23 @@ __global__ void k_head_fwd(const __nv_bfloat16* __restrict__ X, int64_t P, int C
   for (int o = 0; o < Cout; o++) {
     float acc = b[o];
     for (int c = 0; c < Cin; c++) acc += Wt[o * Cin + c] * __bfloat162float(X[p * Cin + c]);
+    Y[p * Cout + o] = acc;
+  }
+}
+
+// the same for 32 input channels: a pixel's channels in four 16-byte loads, summed in the same order
+__global__ void k_head_fwd32(const uint4* __restrict__ X, int64_t P, const float* __restrict__ Wt,
+                             const float* __restrict__ b, int Cout, float* __restrict__ Y) {
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P) return;
+  uint4 v[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) v[j] = __ldg(X + 4 * p + j);
+  const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(v);
+  for (int o = 0; o < Cout; o++) {
+    float acc = b[o];
+#pragma unroll
+    for (int c = 0; c < 32; c++) acc += __ldg(Wt + o * 32 + c) * __bfloat162float(x[c]);
     Y[p * Cout + o] = acc;
   }
 }
@@ -495,22 +473,6 @@ __global__ void k_to_bf16(const float* __restrict__ x, int64_t n, __nv_bfloat16*
 }
 
 // ----------------------------------------------------------------------------------------------------- host side
-typedef CUresult (*NNEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static NNEncodeFn nn_encode() {
-  static NNEncodeFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<NNEncodeFn>(p);
-  }
-  return fn;
-}
-
 // a BF16 [rows x K] K-major operand, box {64, box_rows}, 128-byte swizzle, zero fill outside
 static int nn_map(CUtensorMap* m, const void* ptr, int64_t K, int64_t rows, int box_rows) {
   NNEncodeFn fn = nn_encode();
@@ -529,6 +491,7 @@ static int nn_map(CUtensorMap* m, const void* ptr, int64_t K, int64_t rows, int 
   return BLML_OK;
 }
 
+static inline bool nn_aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 static inline unsigned g1(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace blml
@@ -639,6 +602,12 @@ int blml_nn_sum_splits(const float* in, int splits, int64_t n, float* out, void*
 int blml_nn_pool_fwd(const void* X, int Nb, int H, int W, int Csx, int c0x, int C, void* Y, int Csy, int c0y,
                      void* stream) {
   if (!X || !Y || (H & 1) || (W & 1) || C < 1) { set_error("blml_nn_pool_fwd: bad arguments"); return BLML_ERR_ARG; }
+  if ((Csx | c0x | C | Csy | c0y) % 8 == 0 && nn_aligned16(X) && nn_aligned16(Y)) {
+    k_pool_fwd8<<<g1((int64_t)Nb * (H / 2) * (W / 2) * (C / 8)), 256, 0, NST>>>(
+        (const uint4*)X, Nb, H, W, Csx / 8, c0x / 8, C / 8, (uint4*)Y, Csy / 8, c0y / 8);
+    BLML_CHECK_LAUNCH("blml_nn_pool_fwd");
+    return BLML_OK;
+  }
   k_pool_fwd<<<g1((int64_t)Nb * (H / 2) * (W / 2) * C), 256, 0, NST>>>((const __nv_bfloat16*)X, Nb, H, W, Csx, c0x, C,
                                                                         (__nv_bfloat16*)Y, Csy, c0y);
   BLML_CHECK_LAUNCH("blml_nn_pool_fwd");
@@ -670,6 +639,11 @@ int blml_nn_up_bwd(const float* dY, int Nb, int h, int w, int Csy, int c0y, int 
 int blml_nn_head_fwd(const void* X, int64_t P, int Cin, const float* Wt, const float* b, int Cout, float* Y,
                      void* stream) {
   if (!X || !Wt || !b || !Y || Cout < 1 || Cout > 4) { set_error("blml_nn_head_fwd: bad arguments"); return BLML_ERR_ARG; }
+  if (Cin == 32 && nn_aligned16(X)) {
+    k_head_fwd32<<<g1(P), 256, 0, NST>>>((const uint4*)X, P, Wt, b, Cout, Y);
+    BLML_CHECK_LAUNCH("blml_nn_head_fwd");
+    return BLML_OK;
+  }
   k_head_fwd<<<g1(P), 256, 0, NST>>>((const __nv_bfloat16*)X, P, Cin, Wt, b, Cout, Y);
   BLML_CHECK_LAUNCH("blml_nn_head_fwd");
   return BLML_OK;

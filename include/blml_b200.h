@@ -362,6 +362,12 @@ int blml_start_batch_destroy(blml_start_batch runner);
  * set when a bounded wait gave up (the results are then invalid). */
 int blml_nn_gemm_bf16(const void* A, const void* B, float* C, int M, int N, int K, int splits, int* err,
                       void* stream);
+/* Y slice = act(3 x 3 convolution (pad 1) of the X slice + bias) in BF16, an implicit GEMM on tcgen05 with no im2col
+ * matrix: W [Co][9 C] BF16 with columns (ky 3 + kx) C + c, bias FP32 [Co]. With Yup also the nearest x2 upsampled
+ * result, a (Nb, 2H, 2W) slice. C = 8 or a multiple of 32, Co a multiple of 16 up to 256, strides and offsets multiples
+ * of 8 channels, 16-byte aligned pointers. */
+int blml_nn_conv3x3(const void* X, int Nb, int H, int W, int Cs, int c0, int C, const void* Wt, const float* bias,
+                    int relu, int Co, void* Y, int Ys, int y0, void* Yup, int Ups, int up0, int* err, void* stream);
 /* 3 x 3 (pad 1) im2col of a BF16 slice: col[p][(ky 3 + kx) C + c], or its transpose [9 C][p] */
 int blml_nn_im2col(const void* X, int Nb, int H, int W, int Cs, int c0, int C, void* col, int transposed,
                    void* stream);
