@@ -15,6 +15,12 @@ ENGINE_SIMT, ENGINE_TC = 0, 1
 ROUTE_AUTO, ROUTE_CONTRACT, ROUTE_FFT = 0, 1, 2
 
 
+class AdamTensor(C.Structure):
+    """blml_nn_adam_tensor"""
+    _fields_ = [('w', C.c_void_p), ('g', C.c_void_p), ('m', C.c_void_p), ('v', C.c_void_p), ('n', C.c_int64),
+                ('wb', C.c_void_p), ('wbt', C.c_void_p), ('rows', C.c_int32), ('cols', C.c_int32)]
+
+
 class BLMLError(RuntimeError):
     pass
 
@@ -84,6 +90,10 @@ _SIGS = {
     'blml_seg_dots2': (_I, [_I, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P]),
     'blml_nn_gemm_bf16': (_I, [_P, _P, _P, _I, _I, _I, _I, _P, _P]),
     'blml_nn_conv3x3': (_I, [_P, _I, _I, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _I, _P, _I, _I, _P, _P]),
+    'blml_nn_conv3x3_dgrad': (_I, [_P, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P, _P]),
+    'blml_nn_conv3x3_wgrad': (_I, [_P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P, _P, _P, _P]),
+    'blml_nn_relu_bwd_bias': (_I, [_P, _I, _I, _P, _I, _I, _L, _I, _P, _I, _P, _P, _P]),
+    'blml_nn_adam_multi': (_I, [_P, _I, C.c_float, C.c_float, C.c_float, C.c_float, _I, _P]),
     'blml_nn_im2col': (_I, [_P, _I, _I, _I, _I, _I, _I, _P, _I, _P]),
     'blml_nn_col2im': (_I, [_P, _I, _I, _I, _I, _P, _I, _I, _P]),
     'blml_nn_bias_act': (_I, [_P, _I, _L, _I, _P, _I, _P, _I, _I, _P]),

@@ -14,8 +14,8 @@ start is the real rank-1 solve with seeded phases (blml_binned.py:415-436), whic
 The network (about 1.94e6 parameters): three encoder levels of two 3 x 3 convolutions + ReLU (32, 64, 128 channels)
 with 2 x 2 average pooling, a 256-channel bottleneck, three decoder levels (nearest x2 upsampling, the skip
 concatenated after the upsampled channels, two 3 x 3 convolutions + ReLU), a 1 x 1 head to (re, im). BF16 weights
-and activations, FP32 accumulation, FP32 master weights and Adam state; every convolution is an im2col + tcgen05
-GEMM of csrc/unet.cu, in forward and backward. Inputs: 8 channels per bin -- log1p(counts) / 8, 4 fc, the one-hot
+and activations, FP32 accumulation, FP32 master weights and Adam state; every convolution is an implicit GEMM on
+tcgen05 (csrc/conv.cu), in forward and backward. Inputs: 8 channels per bin -- log1p(counts) / 8, 4 fc, the one-hot
 kernel kind (pball, slits), log10(n) / 6, zeros. Lattice sides must be multiples of 8. The loss is the phase- and
 conjugation-invariant distance of csrc/unet.cu (a fit's field is defined up to a global phase and conjugation)."""
 import ctypes as C
@@ -122,26 +122,19 @@ class WarmStartNet:
         (overwritten) unless dX is None. dY, dX = (tensor, channel stride, offset)."""
         xt, xcs, xc0, ci = X; yt, ycs, yc0, co = Y
         P = N * H * W; K9 = 9 * ci
-        dpre = self._ws('dpre', P * co, torch.bfloat16); dpreT = self._ws('dpreT', P * co, torch.bfloat16)
-        call('blml_nn_relu_bwd', dY[0].data_ptr(), dY[1], dY[2], yt.data_ptr(), ycs, yc0, P, co, dpre.data_ptr(),
-             dpreT.data_ptr(), self.st)
+        dpre = self._ws('dpre', P * co, torch.bfloat16)
         chunks = int(min(2048, max(1, P // 256)))     # ~256 rows per block
         part = self._ws('bpart', chunks * co, torch.float32)
-        call('blml_nn_bias_grad', dY[0].data_ptr(), dY[1], dY[2], yt.data_ptr(), ycs, yc0, P, co, 1, chunks,
-             part.data_ptr(), self.g[name + '.b'].data_ptr(), self.st)
-        colT = self._ws('col', P * K9, torch.bfloat16)
-        call('blml_nn_im2col', xt.data_ptr(), N, H, W, xcs, xc0, ci, colT.data_ptr(), 1, self.st)
+        call('blml_nn_relu_bwd_bias', dY[0].data_ptr(), dY[1], dY[2], yt.data_ptr(), ycs, yc0, P, co, dpre.data_ptr(),
+             chunks, part.data_ptr(), self.g[name + '.b'].data_ptr(), self.st)
         mt = (co + 127) // 128; nt = (K9 + 255) // 256; nkb = (P + 63) // 64
         splits = int(max(1, min(nkb, -(-296 // (mt * nt)))))
         Cp = self._ws('Cp', splits * co * K9, torch.float32)
-        call('blml_nn_gemm_bf16', dpreT.data_ptr(), colT.data_ptr(), Cp.data_ptr(), co, K9, P, splits,
-             self.err.data_ptr(), self.st)
-        call('blml_nn_sum_splits', Cp.data_ptr(), splits, co * K9, self.g[name + '.w'].data_ptr(), self.st)
+        call('blml_nn_conv3x3_wgrad', xt.data_ptr(), N, H, W, xcs, xc0, ci, dpre.data_ptr(), co, splits, Cp.data_ptr(),
+             self.g[name + '.w'].data_ptr(), self.err.data_ptr(), self.st)
         if dX is not None:
-            dcol = self._ws('dcol', P * K9, torch.float32)
-            call('blml_nn_gemm_bf16', dpre.data_ptr(), self.wbt[name].data_ptr(), dcol.data_ptr(), P, K9, co, 1,
-                 self.err.data_ptr(), self.st)
-            call('blml_nn_col2im', dcol.data_ptr(), N, H, W, ci, dX[0].data_ptr(), dX[1], dX[2], self.st)
+            call('blml_nn_conv3x3_dgrad', dpre.data_ptr(), N, H, W, co, self.wbt[name].data_ptr(), ci,
+                 dX[0].data_ptr(), dX[1], dX[2], self.err.data_ptr(), self.st)
 
     # ---------------------------------------------------------------- forward / backward
     def forward(self, x, N, H, W):
@@ -236,14 +229,16 @@ class WarmStartNet:
 
     def adam(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.step_ += 1
-        for k, w in self.p.items():
+        ts = (_lib.AdamTensor * len(self.p))()
+        for t, (k, w) in zip(ts, self.p.items()):
             name = k.split('.')[0]
             conv_w = k.endswith('.w') and name in self.wb
-            rows, cols = (w.shape[0], w.shape[1]) if conv_w else (0, 0)
-            call('blml_nn_adam', w.data_ptr(), self.g[k].data_ptr(), self.m[k].data_ptr(), self.v[k].data_ptr(),
-                 w.numel(), float(lr), float(b1), float(b2), float(eps), self.step_,
-                 self.wb[name].data_ptr() if conv_w else None, self.wbt[name].data_ptr() if conv_w else None,
-                 int(rows), int(cols), self.st)
+            t.w, t.g, t.m, t.v = (d[k].data_ptr() for d in (self.p, self.g, self.m, self.v))
+            t.n = w.numel()
+            if conv_w:
+                t.wb, t.wbt, t.rows, t.cols = self.wb[name].data_ptr(), self.wbt[name].data_ptr(), w.shape[0], w.shape[1]
+        call('blml_nn_adam_multi', C.cast(ts, C.c_void_p), len(self.p), float(lr), float(b1), float(b2), float(eps),
+             self.step_, self.st)
 
     def check(self):
         """Raise when a tensor-core GEMM gave up on a bounded wait since the net was made."""

@@ -3,15 +3,17 @@
 // (its start is the real rank-1 solve, blml_binned.py:415-436); the net replaces that start for the fits it covers.
 //
 // Activations are NHWC (channels innermost) in BF16, read from / written to channel slices of wider buffers so the
-// decoder's skip concatenation needs no copy; gradients are FP32 in the same layout. A 3 x 3 convolution (pad 1) is
-// an implicit GEMM over an explicit im2col matrix Col[p][(ky 3 + kx) C + c]:
-//   forward        Y[P x Cout]   = Col[P x 9C] . W[Cout x 9C]^T
+// decoder's skip concatenation needs no copy; gradients are FP32 in the same layout. The 3 x 3 convolutions run as the
+// implicit GEMMs of conv.cu; here are the plain BF16 GEMM and the explicit im2col form they reproduce bit for bit
+//   forward        Y[P x Cout]   = Col[P x 9C] . W[Cout x 9C]^T,   Col[p][(ky 3 + kx) C + c]
 //   data grad      dCol[P x 9C]  = dPre[P x Cout] . Wt[9C x Cout]^T      (then col2im gathers the 9 taps)
 //   weight grad    dW[Cout x 9C] = dPreT[Cout x P] . ColT[9C x P]^T      (split over P, partials summed in order)
-// Every GEMM is C = A B^T with A (M x K) and B (N x K) K-major BF16 and FP32 output, on tcgen05: TMA loads of
-// 128-byte-swizzled 64-deep K slices into a ring of up to 8 stages, one elected thread issuing kind::f16 MMAs (M 128,
-// N <= 256, K 16) into one of two TMEM accumulators, tcgen05.ld epilogue overlapping the next tile's MMAs. Waits are bounded: on timeout the kernel sets the caller's error word, gives
-// copies and MMAs in flight one more bounded wait, frees its tensor memory and returns.
+// and the layers between them. The GEMM is C = A B^T with A (M x K) and B (N x K) K-major BF16 and FP32 output, on
+// tcgen05: TMA loads of 128-byte-swizzled 64-deep K slices into a ring of up to 8 stages, one elected thread issuing
+// kind::f16 MMAs (M 128, N <= 256, K 16) into one of two TMEM accumulators, tcgen05.ld epilogue overlapping the next
+// tile's MMAs. Waits are bounded: on timeout the kernel sets the caller's error word, gives copies and MMAs in flight
+// one more bounded wait, frees its tensor memory and returns.
+#include <cooperative_groups.h>
 #include "nn_tc.cuh"
 
 namespace blml {
@@ -240,6 +242,76 @@ __global__ void k_relu_bwd(const float* __restrict__ dY, int Csd, int c0d, const
   dpreT[(int64_t)c * P + p] = b;
 }
 
+// through the ReLU and the bias gradient in one pass over dY: dPre = dY (Y > 0) in BF16 [P x C], and part[chunk][c] =
+// the masked FP32 gradient summed over the chunk's rows in row order (block = chunk; the sums of k_bias_grad bit for
+// bit). 8 channels per thread (two 16-byte gradient loads, one activation load, one store); the masked rows pass through
+// shared memory, kRbTile values at a time, to the C threads that sum them. HBM-bound: 4 + 2 + 2 bytes per value.
+constexpr int kRbTile = 8192;
+__global__ void __launch_bounds__(256) k_relu_bwd_bias(const float* __restrict__ dY, int Csd,
+                                                       const __nv_bfloat16* __restrict__ Y, int Csy, int64_t P, int C,
+                                                       __nv_bfloat16* __restrict__ dpre, float* __restrict__ part) {
+  __shared__ float4 sh[kRbTile / 4];
+  const int cg = C / 8, rows_t = kRbTile / C;
+  const int64_t rows = (P + gridDim.x - 1) / gridDim.x;
+  const int64_t p0 = (int64_t)blockIdx.x * rows, p1 = min(P, p0 + rows);
+  float acc = 0.0f;
+  for (int64_t q = p0; q < p1; q += rows_t) {
+    const int nr = (int)min((int64_t)rows_t, p1 - q);
+    for (int i = threadIdx.x; i < nr * cg; i += 256) {
+      const int r = i / cg, g = i - r * cg;
+      const int64_t p = q + r;
+      const float4* d = reinterpret_cast<const float4*>(dY + p * Csd) + 2 * g;
+      float4 d0 = __ldg(d), d1 = __ldg(d + 1);
+      const uint4 yv = __ldg(reinterpret_cast<const uint4*>(Y + p * Csy) + g);
+      const __nv_bfloat162* y2 = reinterpret_cast<const __nv_bfloat162*>(&yv);
+      float2 y = __bfloat1622float2(y2[0]);
+      d0.x = y.x > 0.0f ? d0.x : 0.0f; d0.y = y.y > 0.0f ? d0.y : 0.0f; y = __bfloat1622float2(y2[1]);
+      d0.z = y.x > 0.0f ? d0.z : 0.0f; d0.w = y.y > 0.0f ? d0.w : 0.0f; y = __bfloat1622float2(y2[2]);
+      d1.x = y.x > 0.0f ? d1.x : 0.0f; d1.y = y.y > 0.0f ? d1.y : 0.0f; y = __bfloat1622float2(y2[3]);
+      d1.z = y.x > 0.0f ? d1.z : 0.0f; d1.w = y.y > 0.0f ? d1.w : 0.0f;
+      uint4 o;
+      __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
+      op[0] = __floats2bfloat162_rn(d0.x, d0.y); op[1] = __floats2bfloat162_rn(d0.z, d0.w);
+      op[2] = __floats2bfloat162_rn(d1.x, d1.y); op[3] = __floats2bfloat162_rn(d1.z, d1.w);
+      reinterpret_cast<uint4*>(dpre + p * C)[g] = o;
+      sh[2 * i] = d0; sh[2 * i + 1] = d1;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < C) {
+      const float* v = reinterpret_cast<const float*>(sh) + threadIdx.x;
+#pragma unroll 8
+      for (int r = 0; r < nr; r++) acc += v[r * C];
+    }
+    __syncthreads();
+  }
+  if ((int)threadIdx.x < C) part[(size_t)blockIdx.x * C + threadIdx.x] = acc;
+}
+
+// out[i] = sum_z in[z][i] in order, for few outputs and many partials: a block stages its kSumOut outputs' partials in
+// shared memory (every load in flight at once), then one thread per output adds them
+constexpr int kSumOut = 8, kSumParts = 1024;
+__global__ void __launch_bounds__(256) k_sum_parts(const float* __restrict__ in, int parts, int n,
+                                                   float* __restrict__ out) {
+  __shared__ float sh[kSumParts * kSumOut];
+  const int i0 = blockIdx.x * kSumOut;
+  float acc = 0.0f;
+  for (int z0 = 0; z0 < parts; z0 += kSumParts) {
+    const int nz = min(kSumParts, parts - z0);
+#pragma unroll 8
+    for (int k = threadIdx.x; k < nz * kSumOut; k += 256) {
+      const int i = i0 + k % kSumOut;
+      sh[k] = i < n ? __ldg(in + (size_t)(z0 + k / kSumOut) * n + i) : 0.0f;
+    }
+    __syncthreads();
+    if (threadIdx.x < kSumOut) {
+#pragma unroll 16
+      for (int z = 0; z < nz; z++) acc += sh[z * kSumOut + threadIdx.x];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x < kSumOut && i0 + (int)threadIdx.x < n) out[i0 + threadIdx.x] = acc;
+}
+
 // bias gradient partials: part[chunk][c] = sum over the chunk's rows of dY (Y > 0); block = chunk, thread = channel
 __global__ void k_bias_grad(const float* __restrict__ dY, int Csd, int c0d, const __nv_bfloat16* __restrict__ Y,
                             int Csy, int c0y, int64_t P, int C, int relu, float* __restrict__ part) {
@@ -317,6 +389,20 @@ __global__ void k_pool_bwd_add(const float* __restrict__ dY, int Nb, int H, int 
   dX[q * Csx + c0x + c] += 0.25f * dY[((n * h + y / 2) * w + x / 2) * C + c];
 }
 
+// the same, four channels (16 bytes) per thread; strides and offsets in 4-channel units
+__global__ void k_pool_bwd_add4(const float4* __restrict__ dY, int Nb, int H, int W, int C, float4* __restrict__ dX,
+                                int Csx, int c0x) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (int64_t)Nb * H * W * C) return;
+  const unsigned c = (unsigned)(i % C); const int64_t q = i / C;
+  const unsigned x = (unsigned)(q % W); const int64_t r = q / W;             // r = n H + y, H even
+  const float4 d = __ldg(dY + ((r / 2) * (W / 2) + x / 2) * C + c);
+  float4* o = dX + q * Csx + c0x + c;
+  float4 v = *o;
+  v.x += 0.25f * d.x; v.y += 0.25f * d.y; v.z += 0.25f * d.z; v.w += 0.25f * d.w;
+  *o = v;
+}
+
 // nearest-neighbour x2 upsampling into a channel slice, and its gradient (sum of the 4 copies)
 __global__ void k_up_fwd(const __nv_bfloat16* __restrict__ X, int Nb, int h, int w, int C,
                          __nv_bfloat16* __restrict__ Y, int Csy, int c0y) {
@@ -338,6 +424,24 @@ __global__ void k_up_bwd(const float* __restrict__ dY, int Nb, int h, int w, int
   float s = 0.0f;
   for (int a = 0; a < 2; a++)
     for (int b = 0; b < 2; b++) s += dY[((n * H + 2 * y + a) * W + 2 * x + b) * Csy + c0y + c];
+  dX[q * C + c] = s;
+}
+
+// the same, four channels (16 bytes) per thread; strides and offsets in 4-channel units
+__global__ void k_up_bwd4(const float4* __restrict__ dY, int Nb, int h, int w, int Csy, int c0y, int C,
+                          float4* __restrict__ dX) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (int64_t)Nb * h * w * C) return;
+  const unsigned c = (unsigned)(i % C); const int64_t q = i / C;
+  const unsigned x = (unsigned)(q % w); const int64_t r = q / w;             // r = n h + y
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+  for (int a = 0; a < 2; a++)
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      const float4 v = __ldg(dY + ((2 * r + a) * 2 * w + 2 * x + b) * Csy + c0y + c);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
   dX[q * C + c] = s;
 }
 
@@ -395,23 +499,53 @@ __global__ void k_head_bwd_weight(const float* __restrict__ dY, const __nv_bfloa
   }
 }
 
+// the same for 32 input channels: the chunk's rows staged in shared memory kHwRows at a time, each quantity summed over
+// them in row order by one thread
+constexpr int kHwRows = 256;
+__global__ void __launch_bounds__(256) k_head_bwd_weight32(const float* __restrict__ dY, const uint4* __restrict__ X,
+                                                           int64_t P, int Cout, float* __restrict__ part) {
+  __shared__ uint4 xs[kHwRows * 4];
+  __shared__ float ds[kHwRows * 4];
+  const int nq = Cout * 33, q = threadIdx.x, o = q / 33, c = q - o * 33;
+  const int64_t rows = (P + gridDim.x - 1) / gridDim.x;
+  const int64_t p0 = (int64_t)blockIdx.x * rows, p1 = min(P, p0 + rows);
+  float acc = 0.0f;
+  for (int64_t p = p0; p < p1; p += kHwRows) {
+    const int nr = (int)min((int64_t)kHwRows, p1 - p);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nr * 4; i += 256) xs[i] = __ldg(X + p * 4 + i);
+    for (int i = threadIdx.x; i < nr * Cout; i += 256) ds[i] = __ldg(dY + p * Cout + i);
+    __syncthreads();
+    if (q < nq) {
+      const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(xs);
+#pragma unroll 8
+      for (int r = 0; r < nr; r++) acc += ds[r * Cout + o] * (c < 32 ? __bfloat162float(x[r * 32 + c]) : 1.0f);
+    }
+    __syncthreads();
+  }
+  if (q < nq) part[(size_t)blockIdx.x * nq + q] = acc;
+}
+
 // the phase- and conjugation-invariant loss per sample s (HW complex values u, target t):
 //   l_s = min over (t, conj t) and a global phase of |u - e^{i th} t|^2 / |t|^2
 //       = (|u|^2 + |t|^2 - 2 max(|<t, u>|, |<conj t, u>|)) / |t|^2
-// stats[s] = [|u|^2, |t|^2, Re a, Im a, Re b, Im b] with a = sum conj(t) u, b = sum t u (one block per sample)
-__global__ void k_loss_stats(const float* __restrict__ u, const float* __restrict__ t, int64_t HW,
-                             double* __restrict__ stats) {
-  const int s = blockIdx.x;
-  const float* us = u + (size_t)s * HW * 2;
-  const float* ts = t + (size_t)s * HW * 2;
+// stats[s] = [|u|^2, |t|^2, Re a, Im a, Re b, Im b] with a = sum conj(t) u, b = sum t u: a cluster of 8 blocks per
+// sample, the blocks' sums joined in block order through distributed shared memory
+constexpr int kLossBlocks = 8;
+__global__ void __cluster_dims__(kLossBlocks, 1, 1) __launch_bounds__(256)
+    k_loss_stats(const float2* __restrict__ u, const float2* __restrict__ t, int64_t HW, double* __restrict__ stats) {
+  const int s = blockIdx.x / kLossBlocks, part = blockIdx.x % kLossBlocks;
+  const float2* us = u + (size_t)s * HW;
+  const float2* ts = t + (size_t)s * HW;
   double v[6] = {0, 0, 0, 0, 0, 0};
-  for (int64_t i = threadIdx.x; i < HW; i += blockDim.x) {
-    const double ur = us[2 * i], ui = us[2 * i + 1], tr = ts[2 * i], ti = ts[2 * i + 1];
+  for (int64_t i = (int64_t)part * blockDim.x + threadIdx.x; i < HW; i += kLossBlocks * blockDim.x) {
+    const float2 a = us[i], b = ts[i];
+    const double ur = a.x, ui = a.y, tr = b.x, ti = b.y;
     v[0] += ur * ur + ui * ui; v[1] += tr * tr + ti * ti;
     v[2] += tr * ur + ti * ui; v[3] += tr * ui - ti * ur;       // conj(t) u
     v[4] += tr * ur - ti * ui; v[5] += tr * ui + ti * ur;       // t u
   }
-  __shared__ double sh[6][32];
+  __shared__ double sh[6][32], tot[6];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int q = 0; q < 6; q++) {
     double x = warp_sum(v[q]);
@@ -422,8 +556,17 @@ __global__ void k_loss_stats(const float* __restrict__ u, const float* __restric
     for (int q = 0; q < 6; q++) {
       double x = lane < nw ? sh[q][lane] : 0.0;
       x = warp_sum(x);
-      if (lane == 0) stats[s * 6 + q] = x;
+      if (lane == 0) tot[q] = x;
     }
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  if (part == 0 && threadIdx.x < 6) {
+    double x = 0.0;
+    for (int b = 0; b < kLossBlocks; b++) x += *cl.map_shared_rank(&tot[threadIdx.x], b);
+    stats[s * 6 + threadIdx.x] = x;
+  }
+  cl.sync();                                                    // the other blocks' sums stay until they are read
 }
 
 // loss[s] and du = dl_s / du / S (the batch mean), from the stats
@@ -461,6 +604,36 @@ __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float
   w[i] = wi;
   if (wb) wb[i] = __float2bfloat16(wi);
   if (wbt) { const int64_t r = i / cols, c = i - r * cols; wbt[c * rows + r] = __float2bfloat16(wi); }
+}
+
+// the same update of many tensors in one launch: block b takes 1024 values of the tensor it falls in (first[]: each
+// tensor's first block)
+constexpr int kAdamTensors = 32, kAdamPer = 1024;
+struct AdamArgs {
+  blml_nn_adam_tensor t[kAdamTensors];
+  int first[kAdamTensors + 1];
+  int n;
+};
+__global__ void __launch_bounds__(256) k_adam_multi(const __grid_constant__ AdamArgs a, float lr, float b1, float b2,
+                                                    float eps, float c1, float c2) {
+  int k = 0;
+  while ((int)blockIdx.x >= a.first[k + 1]) k++;
+  const blml_nn_adam_tensor& T = a.t[k];
+  __nv_bfloat16* wb = reinterpret_cast<__nv_bfloat16*>(T.wb);
+  __nv_bfloat16* wbt = reinterpret_cast<__nv_bfloat16*>(T.wbt);
+  const int64_t i0 = (int64_t)(blockIdx.x - a.first[k]) * kAdamPer;
+#pragma unroll
+  for (int j = 0; j < kAdamPer / 256; j++) {
+    const int64_t i = i0 + 256 * j + threadIdx.x;
+    if (i >= T.n) return;
+    const float gi = T.g[i];
+    const float mi = b1 * T.m[i] + (1.0f - b1) * gi, vi = b2 * T.v[i] + (1.0f - b2) * gi * gi;
+    T.m[i] = mi; T.v[i] = vi;
+    const float wi = T.w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    T.w[i] = wi;
+    if (wb) wb[i] = __float2bfloat16(wi);
+    if (wbt) { const int64_t r = i / T.cols, c = i - r * T.cols; wbt[c * T.rows + r] = __float2bfloat16(wi); }
+  }
 }
 
 __global__ void k_to_bf16(const float* __restrict__ x, int64_t n, __nv_bfloat16* __restrict__ y,
@@ -592,6 +765,24 @@ int blml_nn_bias_grad(const float* dY, int Csd, int c0d, const void* Y, int Csy,
   return BLML_OK;
 }
 
+int blml_nn_relu_bwd_bias(const float* dY, int Csd, int c0d, const void* Y, int Csy, int c0y, int64_t P, int C,
+                          void* dpre, int chunks, float* part, float* db, void* stream) {
+  if (!dY || !Y || !dpre || !part || !db || P < 1 || C < 1 || c0d < 0 || c0d + C > Csd || c0y < 0 || c0y + C > Csy ||
+      chunks < 1) {
+    set_error("blml_nn_relu_bwd_bias: bad arguments"); return BLML_ERR_ARG;
+  }
+  if (C % 8 || C > 256 || (Csd | c0d) % 4 || (Csy | c0y) % 8 || !nn_aligned16(dY) || !nn_aligned16(Y) || !nn_aligned16(dpre)) {
+    set_error("blml_nn_relu_bwd_bias: channels in multiples of 8 (at most 256), 16-byte aligned slices");
+    return BLML_ERR_UNSUPPORTED;
+  }
+  k_relu_bwd_bias<<<chunks, 256, 0, NST>>>(dY + c0d, Csd, (const __nv_bfloat16*)Y + c0y, Csy, P, C,
+                                           (__nv_bfloat16*)dpre, part);
+  BLML_CHECK_LAUNCH("blml_nn_relu_bwd_bias");
+  k_sum_parts<<<g1(C, kSumOut), 256, 0, NST>>>(part, chunks, C, db);
+  BLML_CHECK_LAUNCH("blml_nn_relu_bwd_bias finish");
+  return BLML_OK;
+}
+
 int blml_nn_sum_splits(const float* in, int splits, int64_t n, float* out, void* stream) {
   if (!in || !out || splits < 1 || n < 1) { set_error("blml_nn_sum_splits: bad arguments"); return BLML_ERR_ARG; }
   k_sum_splits<<<g1(n), 256, 0, NST>>>(in, splits, n, out);
@@ -616,6 +807,12 @@ int blml_nn_pool_fwd(const void* X, int Nb, int H, int W, int Csx, int c0x, int 
 
 int blml_nn_pool_bwd_add(const float* dY, int Nb, int H, int W, int C, float* dX, int Csx, int c0x, void* stream) {
   if (!dY || !dX || (H & 1) || (W & 1) || C < 1) { set_error("blml_nn_pool_bwd_add: bad arguments"); return BLML_ERR_ARG; }
+  if ((C | Csx | c0x) % 4 == 0 && nn_aligned16(dY) && nn_aligned16(dX)) {
+    k_pool_bwd_add4<<<g1((int64_t)Nb * H * W * (C / 4)), 256, 0, NST>>>((const float4*)dY, Nb, H, W, C / 4, (float4*)dX,
+                                                                       Csx / 4, c0x / 4);
+    BLML_CHECK_LAUNCH("blml_nn_pool_bwd_add");
+    return BLML_OK;
+  }
   k_pool_bwd_add<<<g1((int64_t)Nb * H * W * C), 256, 0, NST>>>(dY, Nb, H, W, C, dX, Csx, c0x);
   BLML_CHECK_LAUNCH("blml_nn_pool_bwd_add");
   return BLML_OK;
@@ -631,6 +828,12 @@ int blml_nn_up_fwd(const void* X, int Nb, int h, int w, int C, void* Y, int Csy,
 
 int blml_nn_up_bwd(const float* dY, int Nb, int h, int w, int Csy, int c0y, int C, float* dX, void* stream) {
   if (!dY || !dX || C < 1) { set_error("blml_nn_up_bwd: bad arguments"); return BLML_ERR_ARG; }
+  if ((C | Csy | c0y) % 4 == 0 && nn_aligned16(dY) && nn_aligned16(dX)) {
+    k_up_bwd4<<<g1((int64_t)Nb * h * w * (C / 4)), 256, 0, NST>>>((const float4*)dY, Nb, h, w, Csy / 4, c0y / 4, C / 4,
+                                                                 (float4*)dX);
+    BLML_CHECK_LAUNCH("blml_nn_up_bwd");
+    return BLML_OK;
+  }
   k_up_bwd<<<g1((int64_t)Nb * h * w * C), 256, 0, NST>>>(dY, Nb, h, w, Csy, c0y, C, dX);
   BLML_CHECK_LAUNCH("blml_nn_up_bwd");
   return BLML_OK;
@@ -659,9 +862,10 @@ int blml_nn_head_bwd(const float* dY, const void* X, int64_t P, int Cin, int Cou
     k_head_bwd_data<<<g1(P * Cin), 256, 0, NST>>>(dY, P, Cout, Wt, Cin, dX);
     BLML_CHECK_LAUNCH("blml_nn_head_bwd");
   }
-  k_head_bwd_weight<<<chunks, 256, 0, NST>>>(dY, (const __nv_bfloat16*)X, P, Cin, Cout, part);
+  if (Cin == 32 && nn_aligned16(X)) k_head_bwd_weight32<<<chunks, 256, 0, NST>>>(dY, (const uint4*)X, P, Cout, part);
+  else k_head_bwd_weight<<<chunks, 256, 0, NST>>>(dY, (const __nv_bfloat16*)X, P, Cin, Cout, part);
   BLML_CHECK_LAUNCH("blml_nn_head_bwd");
-  k_sum_splits<<<g1((int64_t)Cout * (Cin + 1)), 256, 0, NST>>>(part, chunks, (int64_t)Cout * (Cin + 1), gw);
+  k_sum_parts<<<g1(Cout * (Cin + 1), kSumOut), 256, 0, NST>>>(part, chunks, Cout * (Cin + 1), gw);
   BLML_CHECK_LAUNCH("blml_nn_head_bwd");
   return BLML_OK;
 }
@@ -672,7 +876,11 @@ int blml_nn_phase_loss(const float* u, const float* t, int64_t HW, int S, double
   if (!u || !t || !stats || !du || !loss || HW < 1 || S < 1 || S > 65535) {
     set_error("blml_nn_phase_loss: bad arguments"); return BLML_ERR_ARG;
   }
-  k_loss_stats<<<S, 256, 0, NST>>>(u, t, HW, stats);
+  if ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(t)) & 7) {
+    set_error("blml_nn_phase_loss: u and t are complex pairs (8-byte aligned)"); return BLML_ERR_ARG;
+  }
+  k_loss_stats<<<S * kLossBlocks, 256, 0, NST>>>(reinterpret_cast<const float2*>(u), reinterpret_cast<const float2*>(t),
+                                               HW, stats);
   BLML_CHECK_LAUNCH("blml_nn_phase_loss");
   k_loss_grad<<<dim3(g1(HW), (unsigned)S), 256, 0, NST>>>(u, t, HW, S, stats, du, loss);
   BLML_CHECK_LAUNCH("blml_nn_phase_loss");
@@ -688,6 +896,29 @@ int blml_nn_adam(float* w, const float* g, float* m, float* v, int64_t n, float 
   k_adam<<<g1(n), 256, 0, NST>>>(w, g, m, v, n, lr, b1, b2, eps, c1, c2, (__nv_bfloat16*)wb, (__nv_bfloat16*)wbt,
                                  rows, cols);
   BLML_CHECK_LAUNCH("blml_nn_adam");
+  return BLML_OK;
+}
+
+int blml_nn_adam_multi(const blml_nn_adam_tensor* tensors, int n, float lr, float b1, float b2, float eps, int step,
+                       void* stream) {
+  if (!tensors || n < 1 || step < 1) { set_error("blml_nn_adam_multi: bad arguments"); return BLML_ERR_ARG; }
+  const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
+  for (int k = 0; k < n; k++) {
+    const blml_nn_adam_tensor& T = tensors[k];
+    if (!T.w || !T.g || !T.m || !T.v || T.n < 1 || (T.wbt && (int64_t)T.rows * T.cols != T.n)) {
+      set_error("blml_nn_adam_multi: tensor %d", k); return BLML_ERR_ARG;
+    }
+  }
+  for (int k0 = 0; k0 < n; k0 += kAdamTensors) {
+    AdamArgs a{};
+    a.n = std::min(kAdamTensors, n - k0);
+    for (int k = 0; k < a.n; k++) {
+      a.t[k] = tensors[k0 + k];
+      a.first[k + 1] = a.first[k] + (int)((a.t[k].n + kAdamPer - 1) / kAdamPer);
+    }
+    k_adam_multi<<<a.first[a.n], 256, 0, NST>>>(a, lr, b1, b2, eps, c1, c2);
+    BLML_CHECK_LAUNCH("blml_nn_adam_multi");
+  }
   return BLML_OK;
 }
 

@@ -364,10 +364,18 @@ int blml_nn_gemm_bf16(const void* A, const void* B, float* C, int M, int N, int 
                       void* stream);
 /* Y slice = act(3 x 3 convolution (pad 1) of the X slice + bias) in BF16, an implicit GEMM on tcgen05 with no im2col
  * matrix: W [Co][9 C] BF16 with columns (ky 3 + kx) C + c, bias FP32 [Co]. With Yup also the nearest x2 upsampled
- * result, a (Nb, 2H, 2W) slice. C = 8 or a multiple of 32, Co a multiple of 16 up to 256, strides and offsets multiples
+ * result, a (Nb, 2H, 2W) slice. C = 8 = Cs or a multiple of 32, Co a multiple of 16 up to 256, strides and offsets multiples
  * of 8 channels, 16-byte aligned pointers. */
 int blml_nn_conv3x3(const void* X, int Nb, int H, int W, int Cs, int c0, int C, const void* Wt, const float* bias,
                     int relu, int Co, void* Y, int Ys, int y0, void* Yup, int Ups, int up0, int* err, void* stream);
+/* its data gradient: dX slice (FP32, stride Xs, offset x0, overwritten) from dPre [P][Co] BF16 and the transposed
+ * weights Wt [9 C][Co] BF16; C and Co multiples of 32 */
+int blml_nn_conv3x3_dgrad(const void* dpre, int Nb, int H, int W, int Co, const void* Wt, int C, float* dX, int Xs,
+                          int x0, int* err, void* stream);
+/* its weight gradient dW [Co][9 C] FP32 from the X slice and dPre [P][Co] BF16, split over the pixels (part: splits x
+ * Co x 9 C floats, summed in order); C = 8 = Cs or a multiple of 32, Co a multiple of 32 up to 256 */
+int blml_nn_conv3x3_wgrad(const void* X, int Nb, int H, int W, int Cs, int c0, int C, const void* dpre, int Co,
+                          int splits, float* part, float* dW, int* err, void* stream);
 /* 3 x 3 (pad 1) im2col of a BF16 slice: col[p][(ky 3 + kx) C + c], or its transpose [9 C][p] */
 int blml_nn_im2col(const void* X, int Nb, int H, int W, int Cs, int c0, int C, void* col, int transposed,
                    void* stream);
@@ -382,6 +390,10 @@ int blml_nn_relu_bwd(const float* dY, int Csd, int c0d, const void* Y, int Csy, 
 /* db[c] = sum_p dY[p, c] (restricted to Y > 0 when relu), fixed-order chunk partials (part: chunks x C floats) */
 int blml_nn_bias_grad(const float* dY, int Csd, int c0d, const void* Y, int Csy, int c0y, int64_t P, int C, int relu,
                       int chunks, float* part, float* db, void* stream);
+/* the ReLU's gradient and the bias gradient in one pass: dPre [P][C] BF16 = dY (Y > 0), db[c] = its FP32 sum over the
+ * pixels (part: chunks x C floats); C a multiple of 8, at most 256 */
+int blml_nn_relu_bwd_bias(const float* dY, int Csd, int c0d, const void* Y, int Csy, int c0y, int64_t P, int C,
+                          void* dpre, int chunks, float* part, float* db, void* stream);
 /* out = sum over splits of in (fixed order) */
 int blml_nn_sum_splits(const float* in, int splits, int64_t n, float* out, void* stream);
 /* 2 x 2 average pooling (forward into a slice; gradient added into a slice) */
@@ -405,6 +417,12 @@ int blml_nn_phase_loss(const float* u, const float* t, int64_t HW, int S, double
    matrix */
 int blml_nn_adam(float* w, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2, float eps,
                  int step, void* wb, void* wbt, int rows, int cols, void* stream);
+/* blml_nn_adam over n tensors in one launch per 32 (host array of descriptions; wb, wbt may be null) */
+typedef struct {
+  float* w; const float* g; float* m; float* v; int64_t n; void* wb; void* wbt; int32_t rows, cols;
+} blml_nn_adam_tensor;
+int blml_nn_adam_multi(const blml_nn_adam_tensor* tensors, int n, float lr, float b1, float b2, float eps, int step,
+                       void* stream);
 int blml_nn_to_bf16(const float* x, int64_t n, void* y, void* yt, int rows, int cols, void* stream);
 
 /* ---- pair accumulation over lattice bins from the row-kernel value tables (blml_local_gpu.rows / cols,
