@@ -474,7 +474,7 @@ int blml_plan_create(int d, const int64_t* shape, const int32_t* nfreq, const do
     }
   }
   if (rc == BLML_OK && engine == BLML_ENGINE_TC) rc = tc_plan_init(p, fwd_all, inv_all);
-  if (rc == BLML_OK && engine == BLML_ENGINE_SIMT) rc = fft_plan_init(p, freqs);
+  if (rc == BLML_OK && engine == BLML_ENGINE_SIMT) rc = fft_plan_init(p, freqs, weights);
   p->route = p->fft ? BLML_ROUTE_FFT : BLML_ROUTE_CONTRACT;
   if (rc != BLML_OK) {
     if (rc == BLML_ERR_CUDA && blml_last_error()[0] == 0) set_error("blml_plan_create: device allocation failed");

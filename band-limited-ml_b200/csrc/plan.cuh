@@ -26,7 +26,7 @@ int64_t tc_workspace(const blml_plan_s* p, int nb);
 int tc_error(blml_plan_s* p);
 
 // the FFT route (fft_matvec.cu): set up when the plan is a 2-D DFT mask on sides 2^a 3^b (else p->fft stays null)
-int fft_plan_init(blml_plan_s* p, const double* freqs);
+int fft_plan_init(blml_plan_s* p, const double* freqs, const double* weights);
 void fft_plan_free(blml_plan_s* p);
 int64_t fft_workspace(const blml_plan_s* p, int nb);
 int fft_matvec(blml_plan_s* p, const void* x, void* y, int nb, int xc, void* ws, cudaStream_t st);

@@ -433,7 +433,7 @@ def segscan_bench(dev, K=4, m=20, reps=20):
     return res
 
 
-def tune_fft(dev, cta_kib=(24, 32, 48, 64, 72), max_cols=(1, 2, 4), reps=20):
+def tune_fft(dev, cta_kib=(24, 32, 48, 64, 72), max_cols=(1, 2, 4, 8, 16), reps=20):
     """The project's autotuner for the FFT route's launch shape: the grouped mat-vec over the 64 sweep lattices
     (complex float64, and real float64 as the start phase runs it) timed with CUDA events for every shared-memory
     budget per CTA and column-stage width; the fastest total is written to the package's fft_tuning.json, which the

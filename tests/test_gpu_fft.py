@@ -116,3 +116,51 @@ def test_kernels_without_a_dft_mask_keep_the_contraction(cuda_device):
         p.route = _lib.ROUTE_FFT
     # a side with a prime factor 5 has no mixed-radix plan here: the contraction route
     assert _plan((80, 64), 0.3, _lib.F64).route == _lib.ROUTE_CONTRACT
+
+
+# sides of one pass (2 .. 8), two and three, odd powers of 3, seven passes (3^7), long and short together; batches on
+# both sides of the one-launch (cluster) rule
+@pytest.mark.parametrize('dt', [np.float64, np.float32])
+@pytest.mark.parametrize('shape,fc,nbs', [((2, 3), 0.9, (1, 5)), ((8, 4), 0.6, (1, 40)), ((54, 81), 0.3, (1, 2)),
+                                          ((64, 64), 0.45, (4, 8, 9, 16, 17)), ((128, 128), 0.45, (4, 5)),
+                                          ((2187, 2), 0.2, (1,)), ((6, 4096), 0.4, (1, 2)), ((486, 48), 0.05, (1, 3))])
+def test_fft_route_sizes(cuda_device, dt, shape, fc, nbs):
+    """FFT route = numpy's FFT of the mask in float64: the same operator whatever the passes, the launch or the batch.
+    Tolerances: the other tests' of the route."""
+    from blml_b200 import _lib
+    code = _lib.F64 if dt == np.float64 else _lib.F32
+    ct, rt = (torch.complex128, torch.float64) if dt == np.float64 else (torch.complex64, torch.float32)
+    p = _plan(shape, fc, code)
+    assert p.route == _lib.ROUTE_FFT
+    k1 = np.fft.fftfreq(shape[0])[:, None]; k2 = np.fft.fftfreq(shape[1])[None, :]
+    mask = (k1 ** 2 + k2 ** 2) <= (fc / 2) ** 2 * (1 + 1e-9) + 1e-12
+    rng = np.random.default_rng(5)
+    st = torch.cuda.current_stream().cuda_stream
+    for nb in nbs:
+        for xc in (True, False):
+            x = rng.standard_normal((nb,) + shape) + (1j * rng.standard_normal((nb,) + shape) if xc else 0)
+            xt = torch.as_tensor(x).to('cuda', ct if xc else rt).contiguous()
+            y = torch.empty_like(xt)
+            p.apply(xt, y, nb, xc, st)
+            ref = np.fft.ifft2(mask * np.fft.fft2(xt.cpu().numpy().astype(complex)))
+            ref = ref if xc else ref.real
+            err = np.abs(y.cpu().numpy() - ref).max()
+            assert err <= (1e-12 if dt == np.float64 else 2e-6) * np.abs(ref).max(), (nb, xc, err)
+
+
+@pytest.mark.parametrize('shape', [(64, 48), (192, 96)])
+def test_fft_route_band_with_a_gap(cuda_device, shape):
+    """dirichlet columns with a fill: harmonics on both sides of an inner gap, found by table instead of arithmetic."""
+    from blml_b200 import operator as op_mod, _lib, make_modes
+    from blml_b200.spec import parse_modes
+    modes = make_modes([0.6, 0.5], ['dirichlet:0.5', 'dirichlet:0.4'], periods=[float(m) for m in shape])
+    sp, _ = parse_modes(modes, 2)
+    p = op_mod.Plan(*op_mod.mode_transform(sp[0], shape, np.ones(2), shape), shape, _lib.F64, _lib.ENGINE_SIMT)
+    assert p.route == _lib.ROUTE_FFT
+    x = torch.randn((3,) + shape, dtype=torch.complex128, device='cuda')
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    st = torch.cuda.current_stream().cuda_stream
+    p.apply(x, y, 3, True, st)
+    p.route = _lib.ROUTE_CONTRACT
+    p.apply(x, z, 3, True, st)
+    assert (y - z).abs().max().item() <= 1e-12 * z.abs().max().item()
