@@ -155,6 +155,8 @@ _SIGS = {
     'blml_fill_modes': (_I, [_I, _I, _L, _I, _I, _I, _D, _P, _P, _P]),
     'blml_cert_weights': (_I, [_I, _I, _L, _I, _P, _P, _P, _P]),
     'blml_rows': (_I, [C.POINTER(Tables), _P, _L, _P, _L, _P, _I, _P, _P, _P]),
+    'blml_rows_workspace': (_L, [_L, _L, _I]),
+    'blml_rows_ws': (_I, [C.POINTER(Tables), _P, _L, _P, _L, _P, _I, _P, _P, _P, _L, _P]),
     'blml_rows_multi': (_I, [C.POINTER(Tables), _P, _L, _P, _L, _P, _I, _P, _P, _P]),
     'blml_cols': (_I, [C.POINTER(Tables), _P, _L, _P, _L, _P, _I, _P]),
     'blml_cols_dep': (_I, [C.POINTER(Tables), _P, _L, _P, _L, _L, _P, _P, _I, _P]),

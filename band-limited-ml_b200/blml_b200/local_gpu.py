@@ -228,8 +228,10 @@ def rows_dev(ZA, ZB, w, tab, grad=False, f32=False):
     s = torch.empty(R, dtype=torch.float64, device=device)
     ds = torch.zeros((R, max(nW, 1)), dtype=torch.float64, device=device)
     st = _struct(tab, t, grad, f32)
-    call('blml_rows', st, ZA.data_ptr(), R, ZB.data_ptr(), M, w.data_ptr(), int(bool(grad)), s.data_ptr(),
-         ds.data_ptr(), torch.cuda.current_stream(device).cuda_stream)
+    # scratch from torch's allocator: a call then makes no device allocation of its own
+    ws = torch.empty(int(_lib.lib().blml_rows_workspace(R, M, nW if grad else 0)), dtype=torch.uint8, device=device)
+    call('blml_rows_ws', st, ZA.data_ptr(), R, ZB.data_ptr(), M, w.data_ptr(), int(bool(grad)), s.data_ptr(),
+         ds.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream(device).cuda_stream)
     return s, ds
 
 

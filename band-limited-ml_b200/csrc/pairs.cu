@@ -7,6 +7,7 @@
 // by a second kernel, so results are deterministic (the reference combines slices with float64 atomics).
 // Before any launch the coordinates are checked against the tables' extents on the device, so a stale table is an
 // error, never an out-of-range read.
+#include <limits.h>
 #include <mutex>
 #include <cuda.h>
 #include "common.cuh"
@@ -181,56 +182,157 @@ __global__ void __launch_bounds__(PR_THREADS) k_rows_multi(ColMeta cm, const REA
   for (int m = 0; m < Mm; m++) part[((int64_t)blockIdx.y * R + r) * Mm + m] = acc[m];
 }
 
-// shared-memory layout of k_rows_offset (the host sizes the launch with the same functions): the table, then the
-// chunk's column coordinates (int32, D per column), then its weights, each part 16-byte aligned
 __host__ __device__ constexpr size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
-template <typename REAL> __host__ __device__ constexpr size_t offset_smem_zb(int64_t Tn) {
-  return align16((size_t)Tn * sizeof(REAL));
-}
-template <typename REAL> __host__ __device__ constexpr size_t offset_smem_w(int64_t Tn, int D) {
-  return offset_smem_zb<REAL>(Tn) + align16((size_t)PR_CHUNK * D * sizeof(int));
-}
-template <typename REAL> __host__ __device__ constexpr size_t offset_smem_bytes(int64_t Tn, int D) {
-  return offset_smem_w<REAL>(Tn, D) + (size_t)PR_CHUNK * sizeof(double);
+
+// Fast rows kernel for product kernels without groups (every unit one column: offset, rank and circular tables).
+// Each table lies in shared memory as one that a linear index reads -- circular columns unfolded to 2 nb - 1 offsets --,
+// so a column's lookup is one add (the row's byte address plus the column's byte offset) and one shared-memory load.
+// Columns are taken in unit order. A thread holds RPT rows; a chunk's columns are staged as packed byte offsets (read as
+// 16-byte broadcasts that the RPT rows share) with the first position at which a column differs from the one before it:
+// the products over the leading positions are kept and only those from there on are formed again, so columns in
+// lexicographic order (unique bins) cost their last positions only. Products in REAL in unit order, sums in float64 over
+// the slice's columns in order.
+// GRAD: with ND >= nW derivative entries, d . prefix . suffix as the general kernel forms them.
+constexpr int kRfMax = MAXD;
+struct RowsFast {
+  int col[kRfMax];                       // the column at each position
+  int kind[kRfMax];                      // 0 offset, 1 circular, 3 rank
+  int base[kRfMax], len[kRfMax], org[kRfMax], mul[kRfMax], nb[kRfMax];   // table; row address org + za mul; unfolded period
+  int64_t zmin[kRfMax];                  // subtracted from both coordinates (offset and circular tables)
+  int so[kRfMax];                        // the table in shared memory (elements)
+  int nW, dpos[MAXW], dbase[MAXW], dlen[MAXW], dso[MAXW];                // derivative entries: position, table
+  int total;                             // shared-memory elements of all tables
+};
+// shared memory: the tables, then per staged column its packed offsets, then its weight
+__host__ __device__ constexpr int rf_words(int D) { return (D + 1 + 3) / 4 * 4; }
+template <typename REAL> __host__ __device__ constexpr size_t rf_smem(int total, int D) {
+  return align16((size_t)total * sizeof(REAL)) + (size_t)PR_CHUNK * (rf_words(D) * sizeof(int) + sizeof(double));
 }
 
-// Fast rows kernel for product kernels whose columns are all offset rows (sinc / slits / raw dirichlet): each
-// thread keeps one pointer per column into the shared-memory table (T_k + base_k + J_k + za_k), so a pair costs
-// D shared-memory gathers, D - 1 multiplies and one float64 FMA; column coordinates (int32) and weights are staged
-// per chunk and read as broadcasts.
-template <typename REAL, int D>
-__global__ void __launch_bounds__(PR_THREADS) k_rows_offset(ColMeta cm, const REAL* Tg, const int64_t* ZA, int64_t R,
-                                                            const int64_t* ZB, const double* w, int64_t slice,
-                                                            int64_t M, double* part) {
-  extern __shared__ unsigned char smem_raw[];
+template <typename REAL, int D, int RPT, int ND>
+__global__ void __launch_bounds__(PR_THREADS) k_rows_fast(const __grid_constant__ RowsFast rf, const REAL* Tg,
+                                                          const REAL* dTg, const int64_t* ZA, int64_t R,
+                                                          const int64_t* ZB, const double* w, int64_t slice, int64_t M,
+                                                          double* part, double* dpart) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int W = rf_words(D), ES = sizeof(REAL);
   REAL* Ts = reinterpret_cast<REAL*>(smem_raw);
-  int* zbs = reinterpret_cast<int*>(smem_raw + offset_smem_zb<REAL>(cm.Tn));
-  double* ws = reinterpret_cast<double*>(smem_raw + offset_smem_w<REAL>(cm.Tn, D));
-  for (int64_t i = threadIdx.x; i < cm.Tn; i += blockDim.x) Ts[i] = Tg[i];
-  const int64_t r = (int64_t)blockIdx.x * PR_THREADS + threadIdx.x;
-  const bool live = r < R;
-  const REAL* ptr[D];
+  int* zs = reinterpret_cast<int*>(smem_raw + align16((size_t)rf.total * sizeof(REAL)));
+  double* ws = reinterpret_cast<double*>(zs + PR_CHUNK * W);
 #pragma unroll
-  for (int k = 0; k < D; k++) ptr[k] = Ts + cm.base[k] + cm.J[k] + (live ? ZA[r * D + k] : 0);
+  for (int k = 0; k < D; k++)
+    for (int i = threadIdx.x; i < rf.len[k]; i += PR_THREADS) {
+      int s = i;
+      if (rf.kind[k] == 1) { s = i - (rf.nb[k] - 1); s = s < 0 ? s + rf.nb[k] : s; s = min(s, rf.nb[k] - s); }
+      Ts[rf.so[k] + i] = Tg[rf.base[k] + s];
+    }
+#pragma unroll
+  for (int q = 0; q < ND; q++)
+    if (q < rf.nW)
+      for (int i = threadIdx.x; i < rf.dlen[q]; i += PR_THREADS) Ts[rf.dso[q] + i] = dTg[rf.dbase[q] + i];
+  const int64_t r0 = (int64_t)blockIdx.x * (PR_THREADS * RPT) + threadIdx.x;
+  int pb[RPT][D], db[ND ? ND : 1];       // byte addresses of the rows' tables (a derivative entry's: its column's, moved)
+#pragma unroll
+  for (int m = 0; m < RPT; m++) {
+    // rows past the end repeat the thread's first one (a thread past it: row R - 1) and are not stored
+    const int64_t r = min(r0 + (int64_t)m * PR_THREADS < R ? r0 + (int64_t)m * PR_THREADS : r0, R - 1);
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      const int za = (int)(ZA[r * D + rf.col[k]] - rf.zmin[k]);
+      pb[m][k] = (rf.so[k] + rf.org[k] + za * rf.mul[k]) * ES;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < ND; q++) {
+    db[q] = 0;
+#pragma unroll
+    for (int k = 0; k < D; k++)
+      if (q < rf.nW && rf.dpos[q] == k) db[q] = pb[0][k] + (rf.dso[q] - rf.so[k]) * ES;
+  }
+  double acc[RPT], dacc[ND ? ND : 1];
+#pragma unroll
+  for (int m = 0; m < RPT; m++) acc[m] = 0.0;
+#pragma unroll
+  for (int q = 0; q < ND; q++) dacc[q] = 0.0;
   const int64_t j0 = (int64_t)blockIdx.y * slice, j1 = min(M, j0 + slice);
-  double acc = 0.0;
   for (int64_t c0 = j0; c0 < j1; c0 += PR_CHUNK) {
     const int n = (int)(j1 - c0 < PR_CHUNK ? j1 - c0 : PR_CHUNK);
     __syncthreads();
-    for (int i = threadIdx.x; i < n * D; i += blockDim.x) zbs[i] = (int)ZB[c0 * D + i];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ws[i] = w[c0 + i];
-    __syncthreads();
-    if (live) {
-#pragma unroll 4
-      for (int jj = 0; jj < n; jj++) {
-        REAL p = ptr[0][-zbs[jj * D]];
+    for (int i = threadIdx.x; i < n; i += PR_THREADS) {
+      const int64_t* z = ZB + (c0 + i) * D;
+      const int64_t* zp = z - D;
+      int lvl = i == 0 ? 0 : D;
 #pragma unroll
-        for (int k = 1; k < D; k++) p *= ptr[k][-zbs[jj * D + k]];
-        acc = fma((double)p, ws[jj], acc);
+      for (int k = D - 1; k >= 0; k--) {
+        const int64_t v = z[rf.col[k]] - rf.zmin[k];
+        zs[i * W + 1 + k] = (rf.kind[k] == 3 ? (int)v : -(int)v) * ES;
+        if (i > 0 && v != zp[rf.col[k]] - rf.zmin[k]) lvl = k;
+      }
+      zs[i * W] = lvl;
+      ws[i] = w[c0 + i];
+    }
+    __syncthreads();
+    REAL pre[RPT][D];
+    for (int jj = 0; jj < n; jj++) {
+      int z[W];
+#pragma unroll
+      for (int q = 0; q < W / 4; q++) {
+        const int4 v = reinterpret_cast<const int4*>(zs + jj * W)[q];
+        z[4 * q] = v.x; z[4 * q + 1] = v.y; z[4 * q + 2] = v.z; z[4 * q + 3] = v.w;
+      }
+      const double wj = ws[jj];
+      const int lvl = z[0];
+      if constexpr (ND == 0) {
+        // positions below lvl keep their products; the last is always formed
+        auto from = [&](int k) {
+#pragma unroll
+          for (int m = 0; m < RPT; m++) {
+            const REAL t = *reinterpret_cast<const REAL*>(smem_raw + (pb[m][k] + z[1 + k]));
+            pre[m][k] = k ? pre[m][k ? k - 1 : 0] * t : t;
+          }
+        };
+        if (D >= 2 && lvl < D - 1) {
+          if (D >= 3 && lvl < D - 2) {
+#pragma unroll
+            for (int k = 0; k < D - 2; k++) from(k);
+          }
+          if (D >= 2) from(D >= 2 ? D - 2 : 0);
+        }
+        from(D - 1);
+#pragma unroll
+        for (int m = 0; m < RPT; m++) acc[m] = fma((double)pre[m][D - 1], wj, acc[m]);
+      } else {
+        REAL t[D], p[D + 1], sf[D + 1];
+#pragma unroll
+        for (int k = 0; k < D; k++) t[k] = *reinterpret_cast<const REAL*>(smem_raw + (pb[0][k] + z[1 + k]));
+        p[0] = REAL(1); sf[D] = REAL(1);
+#pragma unroll
+        for (int k = 0; k < D; k++) p[k + 1] = p[k] * t[k];
+#pragma unroll
+        for (int k = D - 1; k >= 0; k--) sf[k] = sf[k + 1] * t[k];
+        acc[0] += (double)p[D] * wj;
+#pragma unroll
+        for (int q = 0; q < ND; q++)
+          if (q < rf.nW) {
+            const int k = rf.dpos[q];
+            REAL a = p[0], b = sf[1];
+            int zo = z[1];
+#pragma unroll
+            for (int i = 1; i < D; i++)
+              if (k == i) { a = p[i]; b = sf[i + 1]; zo = z[1 + i]; }
+            const REAL dv = *reinterpret_cast<const REAL*>(smem_raw + (db[q] + zo));
+            dacc[q] += (double)(dv * a * b) * wj;
+          }
       }
     }
   }
-  if (live) part[(int64_t)blockIdx.y * R + r] = acc;
+#pragma unroll
+  for (int m = 0; m < RPT; m++)
+    if (r0 + (int64_t)m * PR_THREADS < R) part[(int64_t)blockIdx.y * R + r0 + (int64_t)m * PR_THREADS] = acc[m];
+  if (ND && r0 < R)
+#pragma unroll
+    for (int q = 0; q < ND; q++)
+      if (q < rf.nW) dpart[((int64_t)blockIdx.y * R + r0) * rf.nW + q] = dacc[q];
 }
 
 __global__ void k_sum_slices(const double* part, int nsl, int64_t n, double* out) {
@@ -291,36 +393,82 @@ __global__ void k_coord_range(const int64_t* ZA, int64_t R, const int64_t* ZB, i
   if (threadIdx.x == 0) for (int q = 0; q < 4; q++) out[4 * k + q] = sh[q][0];
 }
 
+// The same ranges with the table metadata, for one read-back: blocks take strided elements with a fixed column per
+// thread (coalesced rows), their ranges go to part[block][4 d], and k_rows_meta joins them behind a copy of the metadata
+// arrays (MetaList's, in order).
+constexpr int kRangeBlocks = 64;
+__global__ void __launch_bounds__(256) k_rows_ranges(const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, int d,
+                                                     long long* part) {
+  __shared__ long long sh[4][256];
+  const int T = 256 / d * d, tid = threadIdx.x;
+  long long v[4] = {LLONG_MAX, LLONG_MIN, LLONG_MAX, LLONG_MIN};
+  if (tid < T) {
+    for (int64_t e = (int64_t)blockIdx.x * T + tid; e < R * d; e += (int64_t)gridDim.x * T) {
+      const long long z = ZA[e]; v[0] = min(v[0], z); v[1] = max(v[1], z);
+    }
+    if (ZB == ZA && M == R) { v[2] = v[0]; v[3] = v[1]; }
+    else
+      for (int64_t e = (int64_t)blockIdx.x * T + tid; e < M * d; e += (int64_t)gridDim.x * T) {
+        const long long z = ZB[e]; v[2] = min(v[2], z); v[3] = max(v[3], z);
+      }
+  }
+  for (int q = 0; q < 4; q++) sh[q][tid] = v[q];
+  __syncthreads();
+  if (tid < 4 * d) {
+    const int k = tid / 4, q = tid - 4 * k;
+    long long x = sh[q][k];
+    for (int i = k + d; i < T; i += d) x = (q & 1) ? max(x, sh[q][i]) : min(x, sh[q][i]);
+    part[(int64_t)blockIdx.x * 4 * d + tid] = x;
+  }
+}
+
+struct MetaList { const int64_t* src[12]; int n[12]; };
+__global__ void __launch_bounds__(256) k_rows_meta(MetaList ml, const long long* part, int d, long long* out) {
+  const int tid = threadIdx.x;
+  if (tid < 4 * d) {                     // out[0 .. 4 d): min / max of ZA, min / max of ZB per column
+    long long x = part[tid];
+    for (int b = 1; b < kRangeBlocks; b++) {
+      const long long y = part[b * 4 * d + tid];
+      x = (tid & 1) ? max(x, y) : min(x, y);
+    }
+    out[tid] = x;
+  }
+  int at = 4 * d;
+  for (int q = 0; q < 12; q++) {
+    if (tid < ml.n[q]) out[at + tid] = ml.src[q][tid];
+    at += ml.n[q];
+  }
+}
+
 }  // namespace blml
 
 using namespace blml;
 
-static int read_meta(const blml_tables* tb, ColMeta& cm, cudaStream_t st) {
+// the metadata arrays of a table set, in the order both read-backs use
+static int meta_list(const blml_tables* tb, MetaList& ml) {
   if (!tb || tb->d < 1 || tb->d > MAXD || tb->U < 1 || tb->U > MAXU || tb->G < 0 || tb->G > MAXG || tb->nW < 0 ||
       tb->nW > MAXW) {
     set_error("pair tables: d <= %d, units <= %d, groups <= %d, derivative entries <= %d", MAXD, MAXU, MAXG, MAXW);
     return BLML_ERR_ARG;
   }
   const int d = tb->d;
+  const int64_t* src[12] = {tb->kinds, tb->base, tb->Jk, tb->mk, tb->nbins, tb->grp, tb->dim_unit, tb->grp_unit,
+                            tb->wunit, tb->wcol, tb->wgrp, tb->dbase};
+  const int n[12] = {d, d, d, d, d, d, d, tb->G, tb->nW, tb->nW, tb->nW, tb->nW};
+  for (int q = 0; q < 12; q++) {
+    if (n[q] && !src[q]) { set_error("pair tables: a metadata array is missing"); return BLML_ERR_ARG; }
+    ml.src[q] = src[q]; ml.n[q] = n[q];
+  }
+  return BLML_OK;
+}
+
+// the metadata (meta_list's arrays one after another) checked into cm
+static int parse_meta(const blml_tables* tb, const int64_t* v, ColMeta& cm) {
+  const int d = tb->d;
   cm.d = d; cm.U = tb->U; cm.G = tb->G; cm.nW = tb->nW; cm.LR = tb->LR;
   cm.Tn = tb->nT; cm.dTn = tb->ndT;
-  auto fetch = [&](const int64_t* src, int n, int64_t* dst) -> int {
-    if (n == 0) return BLML_OK;
-    return cuda_status(cudaMemcpyAsync(dst, src, n * sizeof(int64_t), cudaMemcpyDeviceToHost, st), "pair tables");
-  };
-  int64_t base[MAXD], J[MAXD], mk[MAXD], nb[MAXD], grp[MAXD], du[MAXD], gu[MAXG], wu[MAXW], wc[MAXW], wg[MAXW], db[MAXW];
-  int64_t codes[MAXD];
-  struct { const int64_t* s; int n; int64_t* d; } req[] = {
-      {tb->kinds, d, codes}, {tb->base, d, base}, {tb->Jk, d, J}, {tb->mk, d, mk}, {tb->nbins, d, nb},
-      {tb->grp, d, grp}, {tb->dim_unit, d, du}, {tb->grp_unit, tb->G, gu}, {tb->wunit, tb->nW, wu},
-      {tb->wcol, tb->nW, wc}, {tb->wgrp, tb->nW, wg}, {tb->dbase, tb->nW, db}};
-  for (auto& q : req) {
-    if (q.n && !q.s) { set_error("pair tables: a metadata array is missing"); return BLML_ERR_ARG; }
-    int e = fetch(q.s, q.n, q.d);
-    if (e) return e;
-  }
-  int e = cuda_status(cudaStreamSynchronize(st), "pair tables");
-  if (e) return e;
+  const int64_t *codes = v, *base = v + d, *J = v + 2 * d, *mk = v + 3 * d, *nb = v + 4 * d, *grp = v + 5 * d,
+                *du = v + 6 * d, *gu = v + 7 * d, *wu = gu + tb->G, *wc = wu + tb->nW, *wg = wc + tb->nW, *db = wg + tb->nW;
   for (int k = 0; k < d; k++) {
     cm.code[k] = (int)codes[k]; cm.base[k] = base[k]; cm.J[k] = J[k]; cm.mk[k] = mk[k]; cm.nb[k] = nb[k];
     cm.grp[k] = (int)grp[k]; cm.dim_unit[k] = (int)du[k];
@@ -355,6 +503,23 @@ static int read_meta(const blml_tables* tb, ColMeta& cm, cudaStream_t st) {
   return BLML_OK;
 }
 
+constexpr int kMetaMax = 7 * MAXD + MAXG + 4 * MAXW;
+
+static int read_meta(const blml_tables* tb, ColMeta& cm, cudaStream_t st) {
+  MetaList ml;
+  int e = meta_list(tb, ml);
+  if (e) return e;
+  int64_t v[kMetaMax];
+  int at = 0;
+  for (int q = 0; q < 12; q++) {
+    if (ml.n[q]) e = cuda_status(cudaMemcpyAsync(v + at, ml.src[q], ml.n[q] * sizeof(int64_t), cudaMemcpyDeviceToHost, st), "pair tables");
+    if (e) return e;
+    at += ml.n[q];
+  }
+  e = cuda_status(cudaStreamSynchronize(st), "pair tables");
+  return e ? e : parse_meta(tb, v, cm);
+}
+
 // the per-column coordinate ranges hr[4 k + (0..3)] = min / max of ZA, min / max of ZB against the tables' extents:
 // offsets within +-J (offset rows), ranks within the rank table, folded coordinates within the period (circular /
 // torus), radii within the radial row
@@ -386,7 +551,7 @@ static int extents_ok(const ColMeta& cm, const long long* hr) {
 // the coordinates must lie in the tables' extents: offsets within +-J (offset rows), ranks within the rank table,
 // folded coordinates within the period (circular / torus), radii within the radial row
 static int check_extents(const ColMeta& cm, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M,
-                         cudaStream_t st) {
+                         cudaStream_t st, long long* ranges = nullptr) {
   if (R == 0 || M == 0) return BLML_OK;
   long long* dr = nullptr;
   long long hr[4 * MAXD];
@@ -398,70 +563,165 @@ static int check_extents(const ColMeta& cm, const int64_t* ZA, int64_t R, const 
   cudaFreeAsync(dr, st);
   if (!e) e = cuda_status(cudaStreamSynchronize(st), "pair extents");
   if (e) return e;
+  if (ranges)
+    for (int i = 0; i < 4 * cm.d; i++) ranges[i] = hr[i];
   return extents_ok(cm, hr);
 }
 
-// column slices of a rows launch: so that the grid covers the GPU about four times
-static void rows_slices(int64_t R, int64_t M, int64_t& nsl, int64_t& slice) {
+// column slices of a rows launch: about 16 blocks of 128 rows per SM, at least 256 columns each
+static void rows_slices(int64_t R, int64_t M, int64_t& nsl, int64_t& slice, int64_t most = 65535) {
   const int64_t rblocks = (R + PR_THREADS - 1) / PR_THREADS;
-  nsl = std::max<int64_t>(1, std::min<int64_t>((4 * 148 + rblocks - 1) / rblocks, (M + 1023) / 1024));
-  nsl = std::min<int64_t>(nsl, 65535);
+  nsl = std::max<int64_t>(1, std::min<int64_t>((16 * 148 + rblocks - 1) / rblocks, (M + 255) / 256));
+  nsl = std::min<int64_t>(nsl, most);
   slice = (M + nsl - 1) / nsl;
   nsl = (M + slice - 1) / slice;
 }
 
-// ws: the slice partials (nsl R (1 + nW) doubles) when the caller provides them, else a stream-ordered allocation
-template <typename REAL>
-static int rows_impl(const blml_tables* tb, const ColMeta& cm, const REAL* T, const REAL* RT, const REAL* dT,
-                     const REAL* dR, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, const double* w,
-                     int grad, double* s, double* ds, cudaStream_t st, double* ws = nullptr) {
-  const int64_t rblocks = (R + PR_THREADS - 1) / PR_THREADS;
-  int64_t nsl, slice;
-  rows_slices(R, M, nsl, slice);
-  const int nW = grad ? cm.nW : 0;
-  double* part = ws;
-  const size_t pbytes = (size_t)nsl * R * (1 + nW) * sizeof(double);
-  int e = BLML_OK;
-  if (!part) {
-    e = cuda_status(cudaMallocAsync((void**)&part, std::max<size_t>(pbytes, 8), st), "blml_rows workspace");
-    if (e) return e;
+// the fast kernel's tables; false when a column or derivative entry needs the general kernel (groups, units that are not
+// one column each, tables past shared memory)
+static bool rows_fast(const ColMeta& cm, const long long* hr, int grad, size_t es, RowsFast& rf) {
+  if (cm.G || cm.U != cm.d) return false;
+  int pos_of[MAXD], seen = 0;
+  for (int k = 0; k < cm.d; k++) {
+    if (cm.dim_unit[k] >= cm.d || ((seen >> cm.dim_unit[k]) & 1)) return false;
+    seen |= 1 << cm.dim_unit[k]; pos_of[k] = cm.dim_unit[k];
   }
-  double* dpart = part + (size_t)nsl * R;
+  rf = RowsFast{};
+  int64_t total = 0;
+  for (int k = 0; k < cm.d; k++) {
+    const int p = pos_of[k], code = cm.code[k];
+    if (code != 0 && code != 1 && code != 3) return false;
+    if (code == 1 && cm.nb[k] < 1) return false;
+    const int64_t len = code == 0 ? 2 * cm.J[k] + 1 : code == 1 ? 2 * cm.nb[k] - 1 : cm.mk[k] * cm.mk[k];
+    rf.col[p] = k; rf.kind[p] = code; rf.base[p] = (int)cm.base[k]; rf.nb[p] = (int)cm.nb[k];
+    rf.so[p] = (int)total; rf.len[p] = (int)len;
+    rf.org[p] = code == 0 ? (int)cm.J[k] : code == 1 ? (int)cm.nb[k] - 1 : 0;
+    rf.mul[p] = code == 3 ? (int)cm.mk[k] : 1;
+    rf.zmin[p] = code == 3 ? 0 : hr[4 * k + 2];
+    total += len;
+    if (total * (int64_t)es > 220 * 1024) return false;
+  }
+  if (grad) {
+    rf.nW = cm.nW;
+    for (int q = 0; q < cm.nW; q++) {
+      const int k = cm.wcol[q];
+      if (cm.wgrp[q] >= 0 || k < 0 || cm.wunit[q] != cm.dim_unit[k] || cm.code[k] == 1) return false;
+      rf.dpos[q] = pos_of[k]; rf.dbase[q] = (int)cm.dbase[q]; rf.dso[q] = (int)total; rf.dlen[q] = rf.len[pos_of[k]];
+      total += rf.dlen[q];
+      if (total * (int64_t)es > 220 * 1024) return false;
+    }
+  }
+  rf.total = (int)total;
+  return true;
+}
+
+// the launch of the rows kernel that serves cm: values and, with grad, derivative partials per slice
+template <typename REAL>
+static int rows_launch(const ColMeta& cm, const long long* hr, const REAL* T, const REAL* RT, const REAL* dT,
+                       const REAL* dR, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, const double* w,
+                       int grad, int64_t nsl, int64_t slice, double* part, double* dpart, cudaStream_t st,
+                       const char* who) {
   bool offset_only = cm.G == 0 && !grad;
   for (int k = 0; k < cm.d; k++) offset_only = offset_only && cm.code[k] == 0;
   const size_t tsz = (size_t)cm.Tn * sizeof(REAL);
-  dim3 grid((unsigned)rblocks, (unsigned)nsl);
-  if (offset_only) {
-    const size_t sm = offset_smem_bytes<REAL>(cm.Tn, cm.d);
-    if (sm > 200 * 1024) { if (!ws) cudaFreeAsync(part, st); set_error("blml_rows: tables too large for shared memory"); return BLML_ERR_UNSUPPORTED; }
-#define ROWS_OFF(DD) case DD: \
-      cudaFuncSetAttribute(k_rows_offset<REAL, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-      k_rows_offset<REAL, DD><<<grid, PR_THREADS, sm, st>>>(cm, T, ZA, R, ZB, w, slice, M, part); break;
-    switch (cm.d) { ROWS_OFF(1) ROWS_OFF(2) ROWS_OFF(3) ROWS_OFF(4) ROWS_OFF(5) ROWS_OFF(6) ROWS_OFF(7) ROWS_OFF(8) }
-#undef ROWS_OFF
+  if (offset_only && align16(tsz) + align16((size_t)PR_CHUNK * cm.d * sizeof(int)) + PR_CHUNK * sizeof(double) > 200 * 1024) {
+    set_error("%s: tables too large for shared memory", who); return BLML_ERR_UNSUPPORTED;
+  }
+  if (tsz + (size_t)cm.G * cm.LR * sizeof(REAL) > 200 * 1024) {
+    set_error("%s: tables too large for shared memory", who); return BLML_ERR_UNSUPPORTED;
+  }
+  RowsFast rf;
+  if (rows_fast(cm, hr, grad, sizeof(REAL), rf) && rf_smem<REAL>(rf.total, cm.d) <= 224 * 1024) {
+    const size_t sm = rf_smem<REAL>(rf.total, cm.d);
+    // two rows per thread share a column's offsets and weight while that still leaves 4 blocks per SM
+    const bool two = !grad && (R + 2 * PR_THREADS - 1) / (2 * PR_THREADS) * nsl >= 4 * 148;
+    auto run = [&](auto kern, int rpt) -> int {
+      if (sm > 48 * 1024) {
+        const int e = cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm), who);
+        if (e) return e;
+      }
+      const dim3 grid((unsigned)((R + PR_THREADS * rpt - 1) / (PR_THREADS * rpt)), (unsigned)nsl);
+      kern<<<grid, PR_THREADS, sm, st>>>(rf, T, dT, ZA, R, ZB, w, slice, M, part, dpart);
+      return BLML_OK;
+    };
+#define ROWS_FAST(DD) case DD: \
+      return !grad ? (two ? run(k_rows_fast<REAL, DD, 2, 0>, 2) : run(k_rows_fast<REAL, DD, 1, 0>, 1)) \
+                   : cm.nW <= 4 ? run(k_rows_fast<REAL, DD, 1, 4>, 1) : run(k_rows_fast<REAL, DD, 1, 8>, 1);
+    switch (cm.d) { ROWS_FAST(1) ROWS_FAST(2) ROWS_FAST(3) ROWS_FAST(4) ROWS_FAST(5) ROWS_FAST(6) ROWS_FAST(7) ROWS_FAST(8) }
+#undef ROWS_FAST
+  }
+  const size_t sm = tsz + (size_t)cm.G * cm.LR * sizeof(REAL);
+  const dim3 grid((unsigned)((R + PR_THREADS - 1) / PR_THREADS), (unsigned)nsl);
+  if (grad) {
+    cudaFuncSetAttribute(k_rows_general<REAL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_rows_general<REAL, true><<<grid, PR_THREADS, sm, st>>>(cm, T, RT, dT, dR, ZA, R, ZB, w, 0, slice, M, part, dpart);
   } else {
-    const size_t sm = tsz + (size_t)cm.G * cm.LR * sizeof(REAL);
-    if (sm > 200 * 1024) { if (!ws) cudaFreeAsync(part, st); set_error("blml_rows: tables too large for shared memory"); return BLML_ERR_UNSUPPORTED; }
-    if (grad) {
-      cudaFuncSetAttribute(k_rows_general<REAL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_rows_general<REAL, true><<<grid, PR_THREADS, sm, st>>>(cm, T, RT, dT, dR, ZA, R, ZB, w, 0, slice, M, part, dpart);
-    } else {
-      cudaFuncSetAttribute(k_rows_general<REAL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_rows_general<REAL, false><<<grid, PR_THREADS, sm, st>>>(cm, T, RT, dT, dR, ZA, R, ZB, w, 0, slice, M, part, dpart);
-    }
+    cudaFuncSetAttribute(k_rows_general<REAL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_rows_general<REAL, false><<<grid, PR_THREADS, sm, st>>>(cm, T, RT, dT, dR, ZA, R, ZB, w, 0, slice, M, part, dpart);
   }
-  e = cuda_status(cudaGetLastError(), "blml_rows");
-  if (!e) {
-    count_launches(2);                       // the rows kernel and the slice sum
-    k_sum_slices<<<std::min<int64_t>((R + 255) / 256, 4096), 256, 0, st>>>(part, (int)nsl, R, s);
-    if (grad && nW) {
-      k_sum_slices<<<std::min<int64_t>((R * nW + 255) / 256, 4096), 256, 0, st>>>(dpart, (int)nsl, R * nW, ds);
-      count_launches(1);
-    }
-    e = cuda_status(cudaGetLastError(), "blml_rows finish");
+  return BLML_OK;
+}
+
+// ws: the slice partials (nsl R (1 + nW) doubles)
+template <typename REAL>
+static int rows_impl(const ColMeta& cm, const long long* hr, const REAL* T, const REAL* RT, const REAL* dT,
+                     const REAL* dR, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, const double* w,
+                     int grad, double* s, double* ds, cudaStream_t st, double* part) {
+  int64_t nsl, slice;
+  rows_slices(R, M, nsl, slice);
+  const int nW = grad ? cm.nW : 0;
+  double* dpart = part + (size_t)nsl * R;
+  int e = rows_launch<REAL>(cm, hr, T, RT, dT, dR, ZA, R, ZB, M, w, grad, nsl, slice, part, dpart, st, "blml_rows");
+  if (!e) e = cuda_status(cudaGetLastError(), "blml_rows");
+  if (e) return e;
+  count_launches(2);                         // the rows kernel and the slice sum
+  k_sum_slices<<<std::min<int64_t>((R + 255) / 256, 4096), 256, 0, st>>>(part, (int)nsl, R, s);
+  if (nW) {
+    k_sum_slices<<<std::min<int64_t>((R * nW + 255) / 256, 4096), 256, 0, st>>>(dpart, (int)nsl, R * nW, ds);
+    count_launches(1);
   }
-  if (!ws) cudaFreeAsync(part, st);
-  return e;
+  return cuda_status(cudaGetLastError(), "blml_rows finish");
+}
+
+// device scratch of a rows call: the read-back block, then the slice partials
+constexpr int64_t kPrepBytes = ((kRangeBlocks + 1) * 4 * MAXD + kMetaMax) * (int64_t)sizeof(long long);
+
+static int64_t rows_bytes(int64_t R, int64_t M, int nW) {
+  int64_t nsl, slice;
+  rows_slices(R, M, nsl, slice);
+  return (kPrepBytes + 255) / 256 * 256 + nsl * R * (1 + nW) * (int64_t)sizeof(double);
+}
+
+// metadata and coordinate ranges in one read-back (prep: kPrepBytes of device scratch), both checked
+static int rows_prepare(const blml_tables* tb, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, void* prep,
+                        ColMeta& cm, long long* hr, cudaStream_t st) {
+  MetaList ml;
+  int e = meta_list(tb, ml);
+  if (e) return e;
+  const int d = tb->d;
+  long long* part = reinterpret_cast<long long*>(prep);
+  long long* out = part + (int64_t)kRangeBlocks * 4 * MAXD;
+  k_rows_ranges<<<kRangeBlocks, 256, 0, st>>>(ZA, R, ZB, M, d, part);
+  k_rows_meta<<<1, 256, 0, st>>>(ml, part, d, out);
+  count_launches(2);
+  long long v[4 * MAXD + kMetaMax];
+  int n = 4 * d;
+  for (int q = 0; q < 12; q++) n += ml.n[q];
+  e = cuda_status(cudaMemcpyAsync(v, out, n * sizeof(long long), cudaMemcpyDeviceToHost, st), "pair tables");
+  if (!e) e = cuda_status(cudaStreamSynchronize(st), "pair tables");
+  if (!e) e = parse_meta(tb, reinterpret_cast<const int64_t*>(v + 4 * d), cm);
+  if (e) return e;
+  for (int i = 0; i < 4 * d; i++) hr[i] = v[i];
+  return extents_ok(cm, hr);
+}
+
+static int rows_tables_ok(const blml_tables* tb, const ColMeta& cm, int grad) {
+  if (tb->f32 ? (!tb->T32 || (cm.G && !tb->RT32) || (grad && (!tb->dT32 || !tb->dR32)))
+              : (!tb->T || (cm.G && !tb->RT) || (grad && (!tb->dT || !tb->dR)))) {
+    set_error(tb->f32 ? "blml_rows: float32 tables missing" : "blml_rows: tables missing");
+    return BLML_ERR_ARG;
+  }
+  return BLML_OK;
 }
 
 extern "C" {
@@ -471,6 +731,7 @@ extern "C" {
 struct blml_rows_plan_s {
   blml_tables tb;
   ColMeta cm;
+  long long hr[4 * MAXD];                // the coordinate set's ranges
 };
 
 int blml_rows_plan_create(const blml_tables* tb, const int64_t* Z, int64_t n, void* stream, blml_rows_plan* out) {
@@ -479,7 +740,8 @@ int blml_rows_plan_create(const blml_tables* tb, const int64_t* Z, int64_t n, vo
   blml_rows_plan_s* p = new blml_rows_plan_s();
   p->tb = *tb;
   int e = read_meta(tb, p->cm, st);
-  if (!e && n > 0) e = check_extents(p->cm, Z, n, Z, n, st);          // every pair within Z: min / max per column
+  for (auto& x : p->hr) x = 0;
+  if (!e && n > 0) e = check_extents(p->cm, Z, n, Z, n, st, p->hr);   // every pair within Z: min / max per column
   if (!e && (tb->f32 ? (!tb->T32 || (p->cm.G && !tb->RT32)) : (!tb->T || (p->cm.G && !tb->RT)))) {
     set_error("blml_rows_plan_create: value tables missing"); e = BLML_ERR_ARG;
   }
@@ -507,11 +769,10 @@ int blml_rows_plan_run(blml_rows_plan p, const int64_t* ZA, int64_t R, const int
     return BLML_ERR_WORKSPACE;
   }
   const blml_tables* tb = &p->tb;
+  double* part = reinterpret_cast<double*>(ws);
   if (tb->f32)
-    return rows_impl<float>(tb, p->cm, tb->T32, tb->RT32, nullptr, nullptr, ZA, R, ZB, M, w, 0, s, nullptr, st,
-                            reinterpret_cast<double*>(ws));
-  return rows_impl<double>(tb, p->cm, tb->T, tb->RT, nullptr, nullptr, ZA, R, ZB, M, w, 0, s, nullptr, st,
-                           reinterpret_cast<double*>(ws));
+    return rows_impl<float>(p->cm, p->hr, tb->T32, tb->RT32, nullptr, nullptr, ZA, R, ZB, M, w, 0, s, nullptr, st, part);
+  return rows_impl<double>(p->cm, p->hr, tb->T, tb->RT, nullptr, nullptr, ZA, R, ZB, M, w, 0, s, nullptr, st, part);
 }
 
 int blml_rows_plan_destroy(blml_rows_plan p) {
@@ -519,23 +780,45 @@ int blml_rows_plan_destroy(blml_rows_plan p) {
   return BLML_OK;
 }
 
+int64_t blml_rows_workspace(int64_t R, int64_t M, int nW) {
+  return R < 1 || M < 1 || nW < 0 ? 0 : rows_bytes(R, M, nW);
+}
+
+int blml_rows_ws(const blml_tables* tb, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, const double* w,
+                 int grad, double* s, double* ds, void* ws, int64_t ws_bytes, void* stream) {
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  ColMeta cm;
+  if (R == 0 || M == 0) {                    // nothing to sum: the tables are checked all the same
+    const int e = read_meta(tb, cm, st);
+    if (e || R == 0) return e;
+    return cuda_status(cudaMemsetAsync(s, 0, R * sizeof(double), st), "blml_rows");
+  }
+  if (tb && tb->nW == 0) grad = 0;
+  const int64_t need = rows_bytes(R, M, grad && tb ? tb->nW : 0);
+  if (!ws || ws_bytes < need) {
+    set_error("blml_rows: workspace of %lld bytes, need %lld", (long long)ws_bytes, (long long)need);
+    return BLML_ERR_WORKSPACE;
+  }
+  long long hr[4 * MAXD];
+  int e = rows_prepare(tb, ZA, R, ZB, M, ws, cm, hr, st);
+  if (!e) e = rows_tables_ok(tb, cm, grad);
+  if (e) return e;
+  double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(ws) + (kPrepBytes + 255) / 256 * 256);
+  if (tb->f32) return rows_impl<float>(cm, hr, tb->T32, tb->RT32, tb->dT32, tb->dR32, ZA, R, ZB, M, w, grad, s, ds, st, part);
+  return rows_impl<double>(cm, hr, tb->T, tb->RT, tb->dT, tb->dR, ZA, R, ZB, M, w, grad, s, ds, st, part);
+}
+
 int blml_rows(const blml_tables* tb, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, const double* w,
               int grad, double* s, double* ds, void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  ColMeta cm;
-  int e = read_meta(tb, cm, st);
+  if (R <= 0 || M <= 0 || !tb) return blml_rows_ws(tb, ZA, R, ZB, M, w, grad, s, ds, nullptr, 0, stream);
+  void* ws = nullptr;
+  const int64_t need = rows_bytes(R, M, grad && tb->nW > 0 ? tb->nW : 0);
+  int e = cuda_status(cudaMallocAsync(&ws, need, st), "blml_rows workspace");
   if (e) return e;
-  if (grad && cm.nW == 0) grad = 0;
-  if (R == 0) return BLML_OK;
-  if (M == 0) return cuda_status(cudaMemsetAsync(s, 0, R * sizeof(double), st), "blml_rows");
-  e = check_extents(cm, ZA, R, ZB, M, st);
-  if (e) return e;
-  if (tb->f32) {
-    if (!tb->T32 || (cm.G && !tb->RT32) || (grad && (!tb->dT32 || !tb->dR32))) { set_error("blml_rows: float32 tables missing"); return BLML_ERR_ARG; }
-    return rows_impl<float>(tb, cm, tb->T32, tb->RT32, tb->dT32, tb->dR32, ZA, R, ZB, M, w, grad, s, ds, st);
-  }
-  if (!tb->T || (cm.G && !tb->RT) || (grad && (!tb->dT || !tb->dR))) { set_error("blml_rows: tables missing"); return BLML_ERR_ARG; }
-  return rows_impl<double>(tb, cm, tb->T, tb->RT, tb->dT, tb->dR, ZA, R, ZB, M, w, grad, s, ds, st);
+  e = blml_rows_ws(tb, ZA, R, ZB, M, w, grad, s, ds, ws, need, stream);
+  cudaFreeAsync(ws, st);
+  return e;
 }
 
 }  // extern "C"
@@ -642,33 +925,14 @@ static int rows_scratch(double** out) {
 }
 
 template <typename REAL>
-static int rows_noalloc_launch(const ColMeta& cm, const REAL* T, const REAL* RT, const int64_t* ZA, int64_t R,
-                               const int64_t* ZB, int64_t M, const double* w, double* part, double* s,
+static int rows_noalloc_launch(const ColMeta& cm, const long long* hr, const REAL* T, const REAL* RT, const int64_t* ZA,
+                               int64_t R, const int64_t* ZB, int64_t M, const double* w, double* part, double* s,
                                cudaStream_t st) {
-  const int64_t rblocks = (R + PR_THREADS - 1) / PR_THREADS;
-  int64_t nsl = std::max<int64_t>(1, std::min<int64_t>((4 * 148 + rblocks - 1) / rblocks, (M + 1023) / 1024));
-  nsl = std::min<int64_t>(std::min<int64_t>(nsl, 65535), std::max<int64_t>(1, kRowsNoAllocMaxR / R));
-  const int64_t slice = (M + nsl - 1) / nsl;
-  nsl = (M + slice - 1) / slice;
-  bool offset_only = cm.G == 0;
-  for (int k = 0; k < cm.d; k++) offset_only = offset_only && cm.code[k] == 0;
-  dim3 grid((unsigned)rblocks, (unsigned)nsl);
-  if (offset_only) {
-    const size_t sm = offset_smem_bytes<REAL>(cm.Tn, cm.d);
-    if (sm > 200 * 1024) { set_error("blml_rows_noalloc: tables too large for shared memory"); return BLML_ERR_UNSUPPORTED; }
-#define ROWS_OFF_NA(DD) case DD: \
-      cudaFuncSetAttribute(k_rows_offset<REAL, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-      k_rows_offset<REAL, DD><<<grid, PR_THREADS, sm, st>>>(cm, T, ZA, R, ZB, w, slice, M, part); break;
-    switch (cm.d) { ROWS_OFF_NA(1) ROWS_OFF_NA(2) ROWS_OFF_NA(3) ROWS_OFF_NA(4) ROWS_OFF_NA(5) ROWS_OFF_NA(6) ROWS_OFF_NA(7) ROWS_OFF_NA(8) }
-#undef ROWS_OFF_NA
-  } else {
-    const size_t sm = (size_t)cm.Tn * sizeof(REAL) + (size_t)cm.G * cm.LR * sizeof(REAL);
-    if (sm > 200 * 1024) { set_error("blml_rows_noalloc: tables too large for shared memory"); return BLML_ERR_UNSUPPORTED; }
-    cudaFuncSetAttribute(k_rows_general<REAL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_rows_general<REAL, false><<<grid, PR_THREADS, sm, st>>>(cm, T, RT, nullptr, nullptr, ZA, R, ZB, w, 0, slice, M,
-                                                              part, nullptr);
-  }
-  int e = cuda_status(cudaGetLastError(), "blml_rows_noalloc");
+  int64_t nsl, slice;
+  rows_slices(R, M, nsl, slice, std::max<int64_t>(1, kRowsNoAllocMaxR / R));
+  int e = rows_launch<REAL>(cm, hr, T, RT, nullptr, nullptr, ZA, R, ZB, M, w, 0, nsl, slice, part, nullptr, st,
+                            "blml_rows_noalloc");
+  if (!e) e = cuda_status(cudaGetLastError(), "blml_rows_noalloc");
   if (e) return e;
   k_sum_slices<<<std::min<int64_t>((R + 255) / 256, 4096), 256, 0, st>>>(part, (int)nsl, R, s);
   count_launches(2);
@@ -708,10 +972,10 @@ int blml_rows_noalloc(const blml_tables* tb, const int64_t* ZA, int64_t R, const
   double* part = scratch + kRowsScratchRangeSlots;
   if (tb->f32) {
     if (!tb->T32 || (cm.G && !tb->RT32)) { set_error("blml_rows_noalloc: float32 tables missing"); return BLML_ERR_ARG; }
-    return rows_noalloc_launch<float>(cm, tb->T32, tb->RT32, ZA, R, ZB, M, w, part, s, st);
+    return rows_noalloc_launch<float>(cm, hr, tb->T32, tb->RT32, ZA, R, ZB, M, w, part, s, st);
   }
   if (!tb->T || (cm.G && !tb->RT)) { set_error("blml_rows_noalloc: tables missing"); return BLML_ERR_ARG; }
-  return rows_noalloc_launch<double>(cm, tb->T, tb->RT, ZA, R, ZB, M, w, part, s, st);
+  return rows_noalloc_launch<double>(cm, hr, tb->T, tb->RT, ZA, R, ZB, M, w, part, s, st);
 }
 
 int blml_lattice_coords(const double* Z, int64_t n, int d, const double* h, int64_t* out, void* stream) {

@@ -443,6 +443,11 @@ typedef struct {
 } blml_tables;
 int blml_rows(const blml_tables* tab, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, const double* w,
               int grad, double* s, double* ds, void* stream);
+/* blml_rows with the caller's device scratch (blml_rows_workspace bytes; nW: the derivative entries, 0 without grad), so
+ * that a call allocates nothing: one read-back of the metadata and coordinate ranges, then the sums */
+int64_t blml_rows_workspace(int64_t R, int64_t M, int nW);
+int blml_rows_ws(const blml_tables* tb, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, const double* w,
+                 int grad, double* s, double* ds, void* ws, int64_t ws_bytes, void* stream);
 /* ---- fused rows of several densities (blml_local.py:213-286 rows_multi, FusedFit's joint and marginals; K9 of
  *      blml_local_gpu.py:107-180): s[r * Mm + m] = sum_j W[j * Mm + m] prod_u (bit u of umask[m] ? T_u : 1), the unit
  *      factors of a pair computed once; 1 <= Mm <= 8 densities, values only (no derivative rows) ---- */
