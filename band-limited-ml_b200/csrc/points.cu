@@ -1,12 +1,17 @@
 // The fitted amplitude at arbitrary points (BLMLQuick.sqrt_density / predict, rahuljhu/band-limited-ml
 // blml_trivial.py:3288-3320 with the continuous product kernel of :2573): g(x_i) = sum_b e_b prod_c K_c(x_ic - z_bc)
 // over the fit's B bin centres z_b, the kernel evaluated exactly (not from a lattice table: the query points are off
-// the lattice). One thread per query point; the bins are staged through shared memory in tiles shared by the block,
-// so each bin centre and coefficient is read from HBM once per block. Per pair: d kernel values (sinpi) and d + 1
-// multiplies in float64, summed in a fixed order. A ball unit over a group of D columns (blml_trivial.py:580-591,
-// 135-143) is one radial value per pair: prod fc p(s), s = ||fc (x - z)|| over the group, p(s) = (1/2)^(D/2)
-// J_(D/2)(pi s) / s^(D/2) -- CUDA's jn for whole orders; for half orders the power series below nu + 12 and, above,
-// upward recurrence from the closed forms of J_1/2 and J_3/2 (the standard methods).
+// the lattice). A warp holds 32 query points; the 8 warps of a block share them and take every eighth bin of a staged
+// tile, the blocks of a cluster take slices of the bins, and the sums are joined in a fixed order (shared memory, then
+// distributed shared memory), so a few hundred points still fill the GPU. A ball unit over a group of D columns
+// (blml_trivial.py:580-591, 135-143) is one radial value per pair: prod fc p(s), s = ||fc (x - z)|| over the group,
+// p(s) = (1/2)^(D/2) J_(D/2)(pi s) / s^(D/2) -- CUDA's jn for whole orders; for half orders the power series below
+// nu + 12 and, above, upward recurrence from the closed forms of J_1/2 and J_3/2 (the standard methods).
+// Bound: float64 arithmetic, about 90 instructions per pair of a sinc and a dirichlet column. sin(pi y) is the odd
+// near-minimax polynomial below on the reduced argument, and a pair's factors share one division (numerators and
+// denominators multiplied apart). 20,000 points by 17,000 bins of a sinc and a dirichlet column: 23.0 -> 2.64 ms (the old
+// grid, one thread per point over every bin, was 79 blocks; its sinpi, fmod and three divisions the rest).
+#include <cooperative_groups.h>
 #include "common.cuh"
 
 namespace blml {
@@ -63,45 +68,117 @@ __device__ __noinline__ double ball_profile(double s, int D, double p0) {
   return pow(0.5, 0.5 * D) * J / pow(s, 0.5 * D);
 }
 
-__global__ void __launch_bounds__(kPtThreads) k_point_rows(int64_t m, int d, const double* __restrict__ X,
-                                                          int64_t B, const double* __restrict__ Z,
-                                                          const double* __restrict__ e, blml_point_cols cols,
+// sin(pi r), |r| <= 1/2: r P(r^2), P the degree-8 polynomial of least relative error for sin(pi sqrt s) / sqrt s on
+// [0, 1/4] (Remez exchange in 50-digit arithmetic, coefficients rounded to float64: 4e-17 relative)
+__device__ __forceinline__ double sinpi_core(double r) {
+  const double s = r * r;
+  double p = 7.6947271574417395e-07;
+  p = fma(p, s, -2.1903185407119565e-05);
+  p = fma(p, s, 0.00046629968877016405);
+  p = fma(p, s, -0.0073704304787627463);
+  p = fma(p, s, 0.082145886569892815);
+  p = fma(p, s, -0.59926452931873819);
+  p = fma(p, s, 2.550164039877294);
+  p = fma(p, s, -5.1677127800499694);
+  p = fma(p, s, 3.1415926535897931);
+  return r * p;
+}
+// nearest integer by adding 1.5 2^52 (|y| < 2^51): its parity in the sum's low bit
+constexpr double kRound = 6755399441055744.0, kRoundMax = 2251799813685248.0;
+__device__ __forceinline__ double sinpi_fast(double y) {
+  if (!(fabs(y) < kRoundMax)) return sinpi(y);                    // (also NaN)
+  const double n = y + kRound;
+  const double v = sinpi_core(y - (n - kRound));
+  return __hiloint2double(__double2hiint(v) ^ (__double2loint(n) << 31), __double2loint(v));
+}
+
+// one column's factor as num / den, multiplied into the pair's
+__device__ __forceinline__ void point_factor(const blml_point_col& c, double inv_p, double t, double& num, double& den) {
+  if (c.kind == BLML_PT_DIRICHLET) {
+    const double k = t * inv_p;
+    if (!(fabs(k) < kRoundMax)) { num *= point_unit(c, t); return; }
+    const double u = fma(-((k + kRound) - kRound), c.P, t);       // t folded into [-P / 2, P / 2]
+    if (fabs(u) < 1e-10) { num *= (c.M - c.Mi) / c.P; return; }
+    const double r = u * inv_p;
+    double v = sinpi_fast(c.M * r);
+    if (c.Mi) v -= sinpi_fast(c.Mi * r);
+    num *= v; den *= sinpi_core(r) * c.P;
+    return;
+  }
+  // sinc and slits: sin(pi f t) / (pi t) to rounding f (1 - (pi f t)^2 / 6), so f, below |f t| = 1e-9
+  const double y = c.f * t;
+  const bool slits = c.kind == BLML_PT_SLITS && c.fi > 0;
+  if (fabs(y) < 1e-9) { num *= slits ? c.f - c.fi : c.f; return; }
+  double v = sinpi_fast(y);
+  if (slits) v -= sinpi_fast(c.fi * t);
+  num *= v; den *= M_PI * t;
+}
+
+constexpr int kPtWarps = kPtThreads / 32;
+template <int D>
+__global__ void __launch_bounds__(kPtThreads) k_point_rows(int64_t m, const double* __restrict__ X, int64_t B,
+                                                          int64_t slice, const double* __restrict__ Z,
+                                                          const double* __restrict__ e,
+                                                          const __grid_constant__ blml_point_cols cols,
                                                           double* __restrict__ g) {
-  __shared__ double zs[kPtTile * kPtMaxD];
+  __shared__ double zs[kPtTile * D];
   __shared__ double es[kPtTile];
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double x[kPtMaxD];
-  for (int c = 0; c < d; c++) x[c] = i < m ? X[i * d + c] : 0.0;
+  __shared__ double sums[kPtWarps][32];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, splits = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int64_t i = (int64_t)(blockIdx.x / splits) * 32 + lane;
+  double x[D], inv_p[D];
+#pragma unroll
+  for (int c = 0; c < D; c++) {
+    x[c] = i < m ? X[i * D + c] : 0.0;
+    inv_p[c] = cols.c[c].kind == BLML_PT_DIRICHLET ? 1.0 / cols.c[c].P : 0.0;
+  }
   double acc = 0.0;
-  for (int64_t b0 = 0; b0 < B; b0 += kPtTile) {
-    const int nt = (int)(B - b0 < kPtTile ? B - b0 : kPtTile);
+  const int64_t b_end = min(B, (int64_t)(rank + 1) * slice);
+  for (int64_t b0 = (int64_t)rank * slice; b0 < b_end; b0 += kPtTile) {
+    const int nt = (int)(b_end - b0 < kPtTile ? b_end - b0 : kPtTile);
     __syncthreads();
-    for (int j = threadIdx.x; j < nt * d; j += blockDim.x) zs[j] = Z[b0 * d + j];
-    for (int j = threadIdx.x; j < nt; j += blockDim.x) es[j] = e[b0 + j];
+    for (int j = threadIdx.x; j < nt * D; j += kPtThreads) zs[j] = Z[b0 * D + j];
+    for (int j = threadIdx.x; j < nt; j += kPtThreads) es[j] = e[b0 + j];
     __syncthreads();
-    if (i < m) {
-      for (int j = 0; j < nt; j++) {
-        double p = es[j];
-        for (int c = 0; c < d; c++) {
-          const blml_point_col& cc = cols.c[c];
-          if (cc.kind == BLML_PT_BALL) {
-            if (cc.fi == 0.0) continue;                   // a ball group's value sits on its first column
-            double s2 = 0.0;
-            for (int c2 = 0; c2 < d; c2++)
-              if ((cc.M >> c2) & 1) {
-                const double t = cols.c[c2].f * (x[c2] - zs[j * d + c2]);
-                s2 += t * t;
-              }
-            p *= cc.fi * ball_profile(sqrt(s2), cc.Mi, cc.P);
-          } else {
-            p *= point_unit(cc, x[c] - zs[j * d + c]);
-          }
+    for (int j = warp; j < nt; j += kPtWarps) {
+      double num = es[j], den = 1.0;
+#pragma unroll
+      for (int c = 0; c < D; c++) {
+        const blml_point_col& cc = cols.c[c];
+        if (cc.kind == BLML_PT_BALL) {
+          if (cc.fi == 0.0) continue;                             // a ball group's value sits on its first column
+          double s2 = 0.0;
+#pragma unroll
+          for (int c2 = 0; c2 < D; c2++)
+            if ((cc.M >> c2) & 1) {
+              const double t = cols.c[c2].f * (x[c2] - zs[j * D + c2]);
+              s2 += t * t;
+            }
+          num *= cc.fi * ball_profile(sqrt(s2), cc.Mi, cc.P);
+        } else {
+          point_factor(cc, inv_p[c], x[c] - zs[j * D + c], num, den);
         }
-        acc += p;
       }
+      acc += num / den;
     }
   }
-  if (i < m) g[i] = acc;
+  sums[warp][lane] = acc;
+  __syncthreads();
+  if (warp == 0) {
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < kPtWarps; w++) v += sums[w][lane];
+    sums[0][lane] = v;
+  }
+  cl.sync();
+  if (rank == 0 && warp == 0 && i < m) {
+    double v = 0.0;
+    for (int b = 0; b < splits; b++) v += cl.map_shared_rank(&sums[0][0], b)[lane];
+    g[i] = v;
+  }
+  cl.sync();                                                      // the other blocks' sums stay until they are read
 }
 
 // Point sums of several densities (blml_local.py:555-560, point_rows_multi: FusedFit's joint and marginals at
@@ -209,8 +286,22 @@ int blml_point_rows(int64_t m, int d, const double* X, int64_t B, const double* 
   if (!X || !g || (B > 0 && (!Z || !e))) { set_error("blml_point_rows: null pointer"); return BLML_ERR_ARG; }
   blml_point_cols cc;
   if (check_point_cols(d, cols, cc, "blml_point_rows")) return BLML_ERR_ARG;
-  const int64_t blocks = (m + kPtThreads - 1) / kPtThreads;
-  k_point_rows<<<(unsigned)blocks, kPtThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(m, d, X, B, Z, e, cc, g);
+  // clusters of up to 8 blocks share 32 points' bins until 8 blocks per SM are reached, at least 256 bins each
+  const int64_t groups = (m + 31) / 32;
+  int splits = 1;
+  while (splits < 8 && groups * splits < 8 * 148 && B / (2 * splits) >= kPtTile) splits *= 2;
+  const int64_t slice = (B + splits - 1) / splits;
+  if (groups * splits > 0x7fffffffLL) { set_error("blml_point_rows: too many points"); return BLML_ERR_ARG; }
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3((unsigned)(groups * splits)); lc.blockDim = dim3(kPtThreads);
+  lc.stream = reinterpret_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)splits; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+  lc.attrs = &at; lc.numAttrs = 1;
+#define PT_ROWS(DD) case DD: cudaLaunchKernelEx(&lc, k_point_rows<DD>, m, X, B, slice, Z, e, cc, g); break;
+  switch (d) { PT_ROWS(1) PT_ROWS(2) PT_ROWS(3) PT_ROWS(4) PT_ROWS(5) PT_ROWS(6) PT_ROWS(7) PT_ROWS(8) }
+#undef PT_ROWS
   BLML_CHECK_LAUNCH("blml_point_rows");
   return BLML_OK;
 }
