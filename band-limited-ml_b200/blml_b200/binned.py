@@ -659,24 +659,36 @@ class BLMLBinned:
             raise NotImplementedError("sqrt_density at arbitrary points: sinc / slits / dirichlet / ball units, or pball "
                                       "groups with dirichlet columns in 1-D / 2-D (a pball group times another unit "
                                       "is neither)")
-        freqs, W = mode_transform(sp, self.shape_, self.h_, self.pad_)
-        plan = Plan(freqs, W, self.shape_, _lib.F64, _lib.ENGINE_SIMT)
+        plan, freqs, (f1t, f2t, o_t, h_t) = self._spectrum_plan(k)
         ws = torch.empty(int(_lib.lib().blml_spectrum_workspace(plan._h, 1)), dtype=torch.uint8, device=self.dev_)
         spec = torch.empty(int(np.prod([len(f) for f in freqs])), dtype=torch.complex128, device=self.dev_)
         x = e if e.is_complex() else e.to(torch.complex128)
         call('blml_spectrum', plan._h, x.data_ptr(), spec.data_ptr(), 1, 1, ws.data_ptr(), ws.numel(), self._st)
-        U = (np.asarray(X, float) - self.origin_[None, :]) / self.h_[None, :]
+        Ut = (Xt - o_t) / h_t                             # lattice coordinates
         if self.d_ == 1:
-            f1, f2, U2 = np.zeros(1), np.asarray(freqs[0], float), np.stack([np.zeros(m), U[:, 0]], 1)
-        else:
-            f1, f2, U2 = np.asarray(freqs[0], float), np.asarray(freqs[1], float), U
-        dev = self.dev_
-        f1t, f2t = torch.as_tensor(f1).to(dev), torch.as_tensor(f2).to(dev)
-        Ut = torch.as_tensor(np.ascontiguousarray(U2, np.float64)).to(dev)
-        g = torch.empty(m, dtype=torch.complex128, device=dev)
-        call('blml_planewave_points', len(f1), len(f2), f1t.data_ptr(), f2t.data_ptr(), spec.data_ptr(), m,
+            Ut = torch.cat([torch.zeros_like(Ut), Ut], 1)
+        g = torch.empty(m, dtype=torch.complex128, device=self.dev_)
+        call('blml_planewave_points', f1t.numel(), f2t.numel(), f1t.data_ptr(), f2t.data_ptr(), spec.data_ptr(), m,
              Ut.data_ptr(), g.data_ptr(), self._st)
         return g
+
+    def _spectrum_plan(self, k):
+        """Mode k's float64 contraction plan, its frequencies, and (frequencies per axis, origin, steps) on the device,
+        for sums over its spectrum: the fit's own plan where it is one, else one made for it. Kept by the fit, per kernel,
+        lattice and stream."""
+        held = self.__dict__.setdefault('_spec_plans', {})
+        key = (spec_key(self.specs_[k]), self.shape_, tuple(self.h_), tuple(self.origin_), self._code, self._st)
+        if key not in held:
+            plan, _, (freqs, W) = self.kern_[k]
+            if self._code != _lib.F64 or plan.engine != _lib.ENGINE_SIMT:
+                with torch.cuda.device(self.dev_):
+                    plan = Plan(freqs, W, self.shape_, _lib.F64, _lib.ENGINE_SIMT)
+            f1, f2 = (np.zeros(1), freqs[0]) if self.d_ == 1 else freqs
+            held[key] = plan, freqs, tuple(torch.as_tensor(np.array(a, np.float64)).to(self.dev_)
+                                           for a in (f1, f2, self.origin_, self.h_))
+            while len(held) > 8:
+                held.pop(next(iter(held)))
+        return held[key]
 
     def sqrt_density(self, X, chunk=65536):
         """g_k(x) = (1/n) sum_b e_bk K_k(x - z_b) at arbitrary points X (m, d) (blml_binned.py:451-465): (m,) for
@@ -692,9 +704,21 @@ class BLMLBinned:
         return out[:, 0] if self.K_ == 1 else out
 
     def predict(self, X):
-        """f(x) = sum_k |g_k(x)|^2 at arbitrary points (blml_binned.py:467-469)."""
-        G = self.sqrt_density(X)
-        return np.abs(G) ** 2 if G.ndim == 1 else (np.abs(G) ** 2).sum(1)
+        """f(x) = sum_k |g_k(x)|^2 at arbitrary points (blml_binned.py:467-469), squared and summed on the device."""
+        if type(self).sqrt_density is not BLMLBinned.sqrt_density:
+            G = self.sqrt_density(X)
+            return np.abs(G) ** 2 if G.ndim == 1 else (np.abs(G) ** 2).sum(1)
+        X = np.atleast_2d(np.asarray(X, float))
+        if X.shape[1] != self.d_:
+            X = X.reshape(-1, self.d_)
+        out = np.zeros(len(X))
+        for i in range(0, len(X), 65536):
+            f = 0.0
+            for k in range(self.K_):
+                g = torch.view_as_real(self._mode_at_points(k, X[i:i + 65536]) / self.n_).square()
+                f = f + (g.sum(1) if self.complex_g_ else g[:, 0])
+            out[i:i + 65536] = f.cpu().numpy()
+        return out
 
     def predict_grid(self, r):
         """f on the lattice refined r times per dim (from the origin in steps h / r; the last fine point is the last
