@@ -8,12 +8,279 @@
 // i.e. the new axis moves to the front. After d forward stages the spectrum sits in natural order (q_1 .. q_d),
 // where the weight W is applied in the last forward stage's epilogue; d inverse stages bring the lattice back in
 // natural order. Every stage is one batched GEMM-shaped launch.
+#include <atomic>
+#include <type_traits>
 #include <vector>
 #include <algorithm>
 #include "plan.cuh"
 
 namespace blml {
 
+// One stage of one mat-vec: the rows rho = b R + r of its nb lattices (M apart), T (M x N), W and Y (nb, N, R).
+struct StageDesc {
+  const void* X; const void* T; const void* W; void* Y;
+  int64_t R; int M, N, nb, flags;      // flags: 1 real input, 2 weight epilogue, 4 real output, 8 X not 16-byte aligned
+};
+
+// D += A B on the FP64 tensor cores: A 8 x 4 (row g = lane / 4, column t = lane % 4), B 4 x 8 (row t, column g), D 8 x 8
+// (row g, columns 2 t and 2 t + 1)
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+
+// A float64 stage on them, Y^T[n, rho] = sum_m T[m, n] X[rho, m] with n on the MMA's rows and rho on its columns, so a
+// lane's two results are neighbours in Y. On this GPU the MMA is the chain of fused multiply-adds over its four k in order,
+// and a complex product takes k = (re, im) of two m: re += X.re T.re, - X.im T.im and im += X.re T.im, + X.im T.re, m
+// after m -- the sums of the SIMT tiles bit for bit (a real X takes four m). K is therefore not split; its slices of KS come
+// through a ring of ST shared-memory stages (cp.async), small tiles spread small stages over the SMs.
+// A CTA is WN x WR warps of AN x AR blocks of 8 x 8.
+// Bound: float64 arithmetic on large stages (512^2 x 8 at 1024^2 frequencies: 32 of the 37 TFLOP/s), the chain of M
+// dependent MMAs on small ones (two every 32 cycles). Whole mat-vecs, against SIMT tiles of the same order (both operands
+// read from shared memory for every one or four products, one slice at a time): 200 x 150 x 2 45.4 -> 23.7 us, x 8 84.8 ->
+// 38.1; 128^2 x 64 221 -> 91; 512^2 1,383 -> 474, x 8 5,050 -> 3,180; 51^2 16.4 -> 9.9; 40^3 48.5 -> 25.8; 1,024 points
+// 58.6 -> 25.5.
+__device__ __forceinline__ void stage_copy16(unsigned char* smem, const void* gmem, bool pred) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  const int sz = pred ? 16 : 0;                          // 0: nothing read, zeros written
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem), "r"(sz) : "memory");
+}
+__device__ __forceinline__ void stage_copy8(unsigned char* smem, const void* gmem, bool pred) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  const int sz = pred ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gmem), "r"(sz) : "memory");
+}
+
+// Brings slices of a tile's T (m by n) and X (rho by m) into shared memory, one after the other; what lies outside is
+// zero. A thread's pieces keep their places, so that a slice costs it an addition and a comparison per piece.
+template <int TN, int TR, int KS, int PT, int PX, int PXR, int THREADS>
+struct StageLoad {
+  static constexpr int NT = KS * TN / THREADS, NX = KS * TR / THREADS, DT = THREADS / TN, DX = THREADS / KS;
+  static_assert(NT * THREADS == KS * TN && NX * THREADS == KS * TR && DT * TN == THREADS && DX * KS == THREADS, "whole passes");
+  const unsigned char *tg, *xg;
+  int64_t tstep, xrow;
+  int tm, xm, M, ts0, xs0, xsz;
+  bool tin, split;
+  unsigned xin;
+  __device__ __forceinline__ StageLoad(const StageDesc& D, int64_t r0, int n0) {
+    const int tid = threadIdx.x, nn = tid % TN, mm = tid % KS, rr = tid / KS;
+    M = D.M;
+    tm = tid / TN; tin = n0 + nn < D.N;
+    tg = reinterpret_cast<const unsigned char*>(D.T) + ((int64_t)tm * D.N + n0 + nn) * 16;
+    tstep = (int64_t)D.N * 16;
+    ts0 = tm * PT + nn * 16;
+    xsz = (D.flags & 1) ? 8 : 16; split = D.flags & 8;
+    const int px = (D.flags & 1) ? PXR : PX;
+    xm = mm; xrow = (int64_t)M * xsz;
+    xg = reinterpret_cast<const unsigned char*>(D.X) + (r0 + rr) * xrow + (int64_t)mm * xsz;
+    xs0 = KS * PT + rr * px + mm * xsz;
+    xin = 0;
+#pragma unroll
+    for (int u = 0; u < NX; u++) xin |= (r0 + rr + u * DX < D.R * D.nb ? 1u : 0u) << u;
+  }
+  __device__ __forceinline__ void operator()(const StageDesc& D, unsigned char* st) {
+#pragma unroll
+    for (int u = 0; u < NT; u++) {
+      const bool ok = tin && tm + u * DT < M;
+      stage_copy16(st + ts0 + u * DT * PT, ok ? tg + u * DT * tstep : reinterpret_cast<const unsigned char*>(D.T), ok);
+    }
+    const unsigned char* none = reinterpret_cast<const unsigned char*>(D.T);
+    unsigned char* xs = st + xs0;
+#pragma unroll
+    for (int u = 0; u < NX; u++) {
+      const bool ok = (xin >> u & 1) && xm < M;
+      const unsigned char* src = ok ? xg + u * DX * xrow : none;
+      if (xsz == 8) stage_copy8(xs + u * DX * PXR, src, ok);
+      else if (!split) stage_copy16(xs + u * DX * PX, src, ok);
+      else { stage_copy8(xs + u * DX * PX, src, ok); stage_copy8(xs + u * DX * PX + 8, src + 8 * ok, ok); }
+    }
+    tg += KS * tstep; tm += KS; xg += KS * xsz; xm += KS;
+  }
+};
+
+__device__ __forceinline__ void stage_store(const StageDesc& D, int64_t rho, int n, double re, double im) {
+  const int64_t b = rho / D.R, r = rho - b * D.R;
+  if (D.flags & 2) { const double wv = reinterpret_cast<const double*>(D.W)[(int64_t)n * D.R + r]; re *= wv; im *= wv; }
+  const int64_t o = b * (int64_t)D.N * D.R + (int64_t)n * D.R + r;
+  if (D.flags & 4) reinterpret_cast<double*>(D.Y)[o] = re;
+  else reinterpret_cast<cpx<double>*>(D.Y)[o] = cpx<double>{re, im};
+}
+
+template <int AN, int AR, int WN, int WR, int KS, int ST>
+struct StageTile {
+  static constexpr int TN = 8 * AN * WN, TR = 8 * AR * WR, THREADS = 32 * WN * WR;
+  // rows padded so that a fragment's lanes fall on different banks
+  static constexpr int PT = TN * 16 + 64, PX = KS * 16 + 32, PXR = KS * 8 + 32;
+  static constexpr int STAGE = KS * PT + TR * PX;
+  static constexpr int SMEM = ST * STAGE;
+
+  static __device__ __forceinline__ void run(const StageDesc& D, int64_t r0, int n0, unsigned char* smem) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int wn = warp % WN * AN * 8, wr = warp / WN * AR * 8;
+    const int M = D.M, N = D.N;
+    const int64_t rows = D.R * D.nb;
+    const bool xreal = D.flags & 1, yreal = D.flags & 4;
+    StageLoad<TN, TR, KS, PT, PX, PXR, THREADS> load(D, r0, n0);
+    double cr[AN][AR][2], ci[AN][AR][2];
+#pragma unroll
+    for (int i = 0; i < AN; i++)
+#pragma unroll
+      for (int j = 0; j < AR; j++) { cr[i][j][0] = cr[i][j][1] = 0.0; ci[i][j][0] = ci[i][j][1] = 0.0; }
+    const int nk = (M + KS - 1) / KS;
+    for (int kt = 0; kt < ST - 1; kt++) {
+      if (kt < nk) load(D, smem + kt * STAGE);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    for (int kt = 0; kt < nk; kt++) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");
+      __syncthreads();                                   // slice kt is there, and slice kt - 1 is done with
+      if (kt + ST - 1 < nk) load(D, smem + (kt + ST - 1) % ST * STAGE);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+      const unsigned char* ts = smem + (kt % ST) * STAGE;
+      const unsigned char* xs = ts + KS * PT;
+      // fragments one chunk of steps ahead of the MMAs that use them
+      auto walk = [&](auto real) {
+        constexpr bool XR = decltype(real)::value;
+        constexpr int NS = XR ? KS / 4 : KS / 2, CH = AN * AR == 1 ? 4 : 1, MT = XR ? 4 : 2;
+        const unsigned char* ap = ts + (XR ? t : t >> 1) * PT + (wn + g) * 16;
+        const unsigned char* bp = xs + (wr + g) * (XR ? PXR : PX) + t * 8;
+        const int are_at = XR ? 0 : (t & 1) * 8, aim_at = XR ? 8 : 8 - are_at;
+        const long long flip = !XR && (t & 1) ? (long long)0x8000000000000000ull : 0ll;
+        double fa[2][CH][AN], fi[2][CH][AN], fb[2][CH][AR];
+        auto get = [&](int c) {
+#pragma unroll
+          for (int q = 0; q < CH; q++) {
+            const int s = c * CH + q;
+#pragma unroll
+            for (int i = 0; i < AN; i++) {
+              fa[c & 1][q][i] = *reinterpret_cast<const double*>(ap + s * MT * PT + i * 128 + are_at);
+              fi[c & 1][q][i] = *reinterpret_cast<const double*>(ap + s * MT * PT + i * 128 + aim_at);
+            }
+#pragma unroll
+            for (int j = 0; j < AR; j++)
+              fb[c & 1][q][j] = *reinterpret_cast<const double*>(bp + s * 32 + j * 8 * (XR ? PXR : PX));
+          }
+        };
+        get(0);
+#pragma unroll
+        for (int c = 0; c < NS / CH; c++) {
+          if (c + 1 < NS / CH) get(c + 1);
+#pragma unroll
+          for (int q = 0; q < CH; q++)
+#pragma unroll
+            for (int i = 0; i < AN; i++) {
+              const double a = XR ? fa[c & 1][q][i] : __longlong_as_double(__double_as_longlong(fa[c & 1][q][i]) ^ flip);
+#pragma unroll
+              for (int j = 0; j < AR; j++) {
+                dmma(cr[i][j], a, fb[c & 1][q][j]);
+                if (!yreal) dmma(ci[i][j], fi[c & 1][q][i], fb[c & 1][q][j]);
+              }
+            }
+        }
+      };
+      if (xreal) walk(std::true_type()); else walk(std::false_type());
+    }
+#pragma unroll
+    for (int j = 0; j < AR; j++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int64_t rho = r0 + wr + 8 * j + 2 * t + e;
+        if (rho >= rows) continue;
+#pragma unroll
+        for (int i = 0; i < AN; i++) {
+          const int n = n0 + wn + 8 * i + g;
+          if (n < N) stage_store(D, rho, n, cr[i][j][e], ci[i][j][e]);
+        }
+      }
+  }
+};
+using TileS = StageTile<1, 1, 2, 2, 32, 4>;              // 16 x 16
+using TileD = StageTile<1, 1, 2, 2, 64, 3>;              // 16 x 16, deeper slices: fewer of them, two CTAs per SM
+using TileM = StageTile<2, 2, 2, 2, 16, 4>;              // 32 x 32
+
+// dependent launches: the CTAs may be placed while the stage before drains, and wait here for its results
+__device__ __forceinline__ void stage_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename TL>
+__global__ void __launch_bounds__(TL::THREADS) k_stage(const __grid_constant__ StageDesc D) {
+  extern __shared__ __align__(16) unsigned char stage_smem[];
+  stage_wait();
+  const int64_t n0 = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * TL::TN;
+  if (n0 < D.N) TL::run(D, (int64_t)blockIdx.x * TL::TR, (int)n0, stage_smem);
+}
+
+// the same stage of many mat-vecs: problem blockIdx.z of the subset
+template <typename TL>
+__global__ void __launch_bounds__(TL::THREADS) k_stage_grouped(const StageDesc* __restrict__ descs,
+                                                               const int* __restrict__ subset,
+                                                               const int* __restrict__ live) {
+  extern __shared__ __align__(16) unsigned char stage_smem[];
+  stage_wait();
+  const int gi = subset ? subset[blockIdx.z] : blockIdx.z;
+  if (live && !live[gi]) return;                       // uniform per CTA: a problem that has stopped
+  const StageDesc D = descs[gi];
+  if ((int64_t)blockIdx.x * TL::TR >= D.R * D.nb || (int64_t)blockIdx.y * TL::TN >= D.N) return;   // past its tiles
+  TL::run(D, (int64_t)blockIdx.x * TL::TR, blockIdx.y * TL::TN, stage_smem);
+}
+
+// their shared memory, set once per device (outside any stream capture: at plan creation)
+static int stage_smem_once() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  int e = cuda_status(cudaGetDevice(&dev), "matvec stage");
+  if (e || (dev < 64 && done[dev])) return e;
+  auto set = [&](auto tl) {
+    using TL = decltype(tl);
+    if (!e) e = cuda_status(cudaFuncSetAttribute(k_stage<TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, TL::SMEM), "matvec stage");
+    if (!e) e = cuda_status(cudaFuncSetAttribute(k_stage_grouped<TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, TL::SMEM), "matvec stage");
+  };
+  set(TileS()); set(TileD()); set(TileM());
+  if (!e && dev < 64) done[dev] = true;
+  return e;
+}
+
+// Calls go(tile) with the tile for a launch of `blocks` 8 x 8 blocks of sums of M terms. 16 x 16 tiles up to about 14,000
+// blocks (10,200: 95.5 us against 98.6 with 32 x 32, 8,200: 494 against 533; 65,500: 3,747 against 3,238); the deep
+// slices where two CTAs per SM hold the launch and a sum spans more than one of them (200 x 150 x 2, 500 blocks: 23.7 us
+// against 27.9, x 8, 2,000 blocks: 51.2 against 40.1; M = 96: 16.9 against 14.3). 64 x 64 tiles were slower throughout.
+template <typename F>
+static void stage_tile(double blocks, int64_t M, F go) {
+  if (blocks > 14000) go(TileM());
+  else if (blocks <= 4.0 * 2 * 148 && M > 96) go(TileD());
+  else go(TileS());
+}
+
+template <typename... P, typename... A>
+static void launch_dep(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid; c.blockDim = dim3((unsigned)threads); c.dynamicSmemBytes = smem; c.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at; c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+
+static int64_t tiles_of(int64_t n, int side) { return (n + side - 1) / side; }
+
+static int launch_stage_f64(const StageDesc& D, cudaStream_t st) {
+  const int64_t rows = D.R * D.nb;
+  stage_tile((double)tiles_of(rows, 8) * (double)tiles_of(D.N, 8), D.M, [&](auto tl) {
+    using TL = decltype(tl);
+    const int64_t nt = tiles_of(D.N, TL::TN), ny = std::min<int64_t>(nt, 65535);
+    launch_dep(k_stage<TL>, dim3((unsigned)tiles_of(rows, TL::TR), (unsigned)ny, (unsigned)((nt + ny - 1) / ny)), TL::THREADS,
+               TL::SMEM, st, D);
+  });
+  BLML_CHECK_LAUNCH("matvec stage");
+  return BLML_OK;
+}
+
+// ------------------------------------------------------------------------------- SIMT tiles: float32
+// (widened to the float64 tensor cores they are slower at every size: 200 x 150 x 2 30.2 -> 41.5 us, 512^2 x 8 2,542 ->
+// 4,657)
 constexpr int TR = 64, TN = 64, TK = 16;
 
 // Y[b, n, r] = (sum_m X[b, r, m] T[m, n]) * (W[n R + r] if WEIGHT); X real or complex, Y complex or (YREAL) its real
@@ -137,6 +404,13 @@ __global__ void __launch_bounds__(256) k_contract_small(const void* __restrict__
 template <typename T>
 static int launch_stage(const void* X, bool xreal, const void* Tw, const void* W, void* Y, bool yreal, int64_t R,
                         int M, int N, int nb, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8) {
+    StageDesc D;
+    D.X = X; D.T = Tw; D.W = W; D.Y = Y; D.R = R; D.M = M; D.N = N; D.nb = nb;
+    D.flags = (xreal ? 1 : 0) | (W ? 2 : 0) | (yreal ? 4 : 0) | ((reinterpret_cast<uintptr_t>(X) & 15) ? 8 : 0);
+    return launch_stage_f64(D, st);
+  }
+  else {
   dim3 grid((unsigned)((R + TR - 1) / TR), (unsigned)((N + TN - 1) / TN), (unsigned)nb);
   const cpx<T>* t = reinterpret_cast<const cpx<T>*>(Tw);
   const T* w = reinterpret_cast<const T*>(W);
@@ -159,6 +433,7 @@ static int launch_stage(const void* X, bool xreal, const void* Tw, const void* W
   else k_contract<T, false, false, false><<<grid, 256, 0, st>>>(X, t, w, Y, R, M, N);
   BLML_CHECK_LAUNCH("matvec stage");
   return BLML_OK;
+  }
 }
 
 // the d forward stages alone, the weight in the last one's epilogue: spec = W (v^H x), (nb, H_1 ... H_d) natural order
@@ -213,10 +488,6 @@ static int simt_matvec(blml_plan_s* p, const void* x, void* y, int nb, int xc, v
 // ---------------------------------------------------------------------------------------------- grouped stages
 // One stage of many mat-vecs (different plans, lattice sizes and buffers) in one launch: problem g = blockIdx.z reads
 // its descriptor; rows rho = b R + r of its nb lattices; 32 x 32 output tiles, 2 x 2 outputs per thread.
-struct StageDesc {
-  const void* X; const void* T; const void* W; void* Y;
-  int64_t R; int M, N, nb, flags;      // flags: 1 real input, 2 weight epilogue, 4 real output
-};
 constexpr int GR = 32, GN = 32, GK = 16;
 
 template <typename T>
@@ -396,6 +667,8 @@ struct blml_group_s {
   std::vector<blml::StageDesc*> dev;    // one descriptor array per stage index
   std::vector<dim3> grids, grids_big;   // 32 x 32 and 64 x 64 tile grids per stage
   std::vector<double> tiles_big;        // 64 x 64 tiles of a stage over all problems
+  std::vector<double> blocks8;          // its 8 x 8 blocks (float64)
+  std::vector<int64_t> max_rows, max_n, max_m;   // the largest problem's rows, frequencies and terms per stage
   void* ws;                             // the group's own intermediate buffers
   void* fft;                            // the FFT route's descriptors (every plan a DFT mask), or null
   int route;                            // BLML_ROUTE_CONTRACT or BLML_ROUTE_FFT
@@ -474,6 +747,7 @@ int blml_plan_create(int d, const int64_t* shape, const int32_t* nfreq, const do
     }
   }
   if (rc == BLML_OK && engine == BLML_ENGINE_TC) rc = tc_plan_init(p, fwd_all, inv_all);
+  if (rc == BLML_OK && engine == BLML_ENGINE_SIMT && f64) rc = stage_smem_once();
   if (rc == BLML_OK && engine == BLML_ENGINE_SIMT) rc = fft_plan_init(p, freqs, weights);
   p->route = p->fft ? BLML_ROUTE_FFT : BLML_ROUTE_CONTRACT;
   if (rc != BLML_OK) {
@@ -506,12 +780,11 @@ int blml_group_create(int G, const blml_plan* plans, const int* nbatch, int x_co
       set_error("blml_group_create: every plan of a group has one dimension count and dtype"); return BLML_ERR_ARG;
     }
   // the 64 x 64 stage kernel's dynamic shared memory (set here, outside any stream capture)
-  int e0 = cuda_status(cudaFuncSetAttribute(k_contract_grouped_big<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)big_smem<double>()), "blml_group_create");
-  if (!e0) e0 = cuda_status(cudaFuncSetAttribute(k_contract_grouped_big<float>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)big_smem<float>()),
-                            "blml_group_create");
-  if (e0) return e0;
+  if (dtype == BLML_F32) {
+    const int e0 = cuda_status(cudaFuncSetAttribute(k_contract_grouped_big<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (int)big_smem<float>()), "blml_group_create");
+    if (e0) return e0;
+  }
   const size_t esz = dtype == BLML_F64 ? 16 : 8, rsz = dtype == BLML_F64 ? 8 : 4;
   const size_t xsz = x_complex ? esz : rsz, ysz = x_complex ? esz : rsz;
   std::vector<size_t> wso(G + 1, 0);
@@ -523,8 +796,8 @@ int blml_group_create(int G, const blml_plan* plans, const int* nbatch, int x_co
     delete grp; set_error("blml_group_create: workspace allocation"); return BLML_ERR_CUDA;
   }
   std::vector<std::vector<StageDesc>> host(2 * d, std::vector<StageDesc>(G));
-  std::vector<int64_t> maxr(2 * d, 0), maxn(2 * d, 0);
-  grp->tiles_big.assign(2 * d, 0.0);
+  std::vector<int64_t> maxr(2 * d, 0), maxn(2 * d, 0), maxm(2 * d, 0);
+  grp->tiles_big.assign(2 * d, 0.0); grp->blocks8.assign(2 * d, 0.0);
   for (int g = 0; g < G; g++) {
     const blml_plan_s* p = plans[g];
     std::vector<int64_t> dims(p->shape, p->shape + d);
@@ -541,13 +814,16 @@ int blml_group_create(int G, const blml_plan* plans, const int* nbatch, int x_co
       StageDesc& D = host[s][g];
       D.X = cur; D.T = fwd ? p->tf[a] : p->ti[a]; D.W = (s == d - 1) ? p->W : nullptr; D.Y = outp;
       D.R = R; D.M = (int)M; D.N = (int)N; D.nb = nbatch[g];
-      D.flags = ((s == 0 && !x_complex) ? 1 : 0) | ((s == d - 1) ? 2 : 0) | ((last && !x_complex) ? 4 : 0);
-      maxr[s] = std::max(maxr[s], R * nbatch[g]); maxn[s] = std::max<int64_t>(maxn[s], N);
+      D.flags = ((s == 0 && !x_complex) ? 1 : 0) | ((s == d - 1) ? 2 : 0) | ((last && !x_complex) ? 4 : 0) |
+                ((reinterpret_cast<uintptr_t>(cur) & 15) ? 8 : 0);
+      maxr[s] = std::max(maxr[s], R * nbatch[g]); maxm[s] = std::max(maxm[s], M); maxn[s] = std::max<int64_t>(maxn[s], N);
+      grp->blocks8[s] += (double)tiles_of(R * nbatch[g], 8) * (double)tiles_of(N, 8);
       grp->tiles_big[s] += (double)((R * nbatch[g] + BR - 1) / BR) * (double)((N + BN - 1) / BN);
       dims.pop_back(); dims.insert(dims.begin(), N);
       cur = outp;
     }
   }
+  grp->max_rows = maxr; grp->max_n = maxn; grp->max_m = maxm;
   int e = BLML_OK;
   grp->dev.assign(2 * d, nullptr);
   for (int s = 0; s < 2 * d && !e; s++) {
@@ -582,16 +858,18 @@ int blml_group_matvec_masked(blml_group grp, const int* subset, int n, const int
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (grp->route == BLML_ROUTE_FFT) return fft_group_launch(grp->fft, grp->dtype, subset, n, live, st);
   for (int s = 0; s < grp->nstages; s++) {
-    // 64 x 64 tiles when the launch has enough of them to fill the GPU twice over (the problems of a subset are
-    // taken as average ones), else 32 x 32
-    const bool big = grp->tiles_big[s] * n / grp->G >= 2.0 * 148;
-    dim3 g = big ? grp->grids_big[s] : grp->grids[s]; g.z = (unsigned)n;
-    if (big) {
-      if (grp->dtype == BLML_F64)
-        k_contract_grouped_big<double><<<g, 256, big_smem<double>(), st>>>(grp->dev[s], subset, live);
-      else k_contract_grouped_big<float><<<g, 256, big_smem<float>(), st>>>(grp->dev[s], subset, live);
+    // (the problems of a subset are taken as average ones)
+    if (grp->dtype == BLML_F64) {
+      stage_tile(grp->blocks8[s] * n / grp->G, grp->max_m[s], [&](auto tl) {
+        using TL = decltype(tl);
+        launch_dep(k_stage_grouped<TL>, dim3((unsigned)tiles_of(grp->max_rows[s], TL::TR), (unsigned)tiles_of(grp->max_n[s], TL::TN), (unsigned)n), TL::THREADS, TL::SMEM,
+                   st, grp->dev[s], subset, live);
+      });
     } else {
-      if (grp->dtype == BLML_F64) k_contract_grouped<double><<<g, 256, 0, st>>>(grp->dev[s], subset, live);
+      // 64 x 64 tiles when the launch has enough of them to fill the GPU twice over, else 32 x 32
+      const bool big = grp->tiles_big[s] * n / grp->G >= 2.0 * 148;
+      dim3 g = big ? grp->grids_big[s] : grp->grids[s]; g.z = (unsigned)n;
+      if (big) k_contract_grouped_big<float><<<g, 256, big_smem<float>(), st>>>(grp->dev[s], subset, live);
       else k_contract_grouped<float><<<g, 256, 0, st>>>(grp->dev[s], subset, live);
     }
     BLML_CHECK_LAUNCH("blml_group_matvec");
