@@ -15,6 +15,9 @@ ENGINE_SIMT, ENGINE_TC = 0, 1
 ROUTE_AUTO, ROUTE_CONTRACT, ROUTE_FFT = 0, 1, 2
 
 
+ALLOC_FN = C.CFUNCTYPE(C.c_void_p, C.c_size_t, C.c_void_p)       # blml_alloc_fn
+
+
 class AdamTensor(C.Structure):
     """blml_nn_adam_tensor"""
     _fields_ = [('w', C.c_void_p), ('g', C.c_void_p), ('m', C.c_void_p), ('v', C.c_void_p), ('n', C.c_int64),
@@ -56,6 +59,7 @@ _SIGS = {
     'blml_plan_status': (_I, [_P]),
     'blml_matvec_workspace': (_L, [_P, _I]),
     'blml_matvec': (_I, [_P, _P, _P, _I, _I, _P, _L, _P]),
+    'blml_group_create_with': (_I, [_I, _P, _P, _I, _P, _P, _P, _P, ALLOC_FN, _P, _P, C.POINTER(_P)]),
     'blml_group_create': (_I, [_I, _P, _P, _I, _P, _P, _P, _P, C.POINTER(_P)]),
     'blml_group_matvec': (_I, [_P, _P]),
     'blml_group_destroy': (_I, [_P]),
@@ -110,6 +114,8 @@ _SIGS = {
     'blml_nn_adam': (_I, [_P, _P, _P, _P, _L, C.c_float, C.c_float, C.c_float, C.c_float, _I, _P, _P, _I, _I, _P]),
     'blml_nn_to_bf16': (_I, [_P, _L, _P, _P, _I, _I, _P]),
     'blml_lbfgs_batch_create': (_I, [_I, _I, _P, _P, _I, _D, _D, _L, _P, _P, _P, _P, _P, C.POINTER(_P)]),
+    'blml_lbfgs_batch_create_with': (_I, [_I, _I, _P, _P, _I, _D, _D, _L, _P, _P, _P, _P, _P, _I, ALLOC_FN, _P, _P,
+                                          C.POINTER(_P)]),
     'blml_lbfgs_batch_set_caps': (_I, [_P, _P]),
     'blml_lbfgs_batch_set_history': (_I, [_P, _I]),
     'blml_seg_dots2_h32': (_I, [_I, _P, _P, _I, _P, _P, _P, _P, _P, _P, _P]),
@@ -122,6 +128,8 @@ _SIGS = {
     'blml_lbfgs_batch_stats': (_I, [_P, _P]),
     'blml_lbfgs_batch_destroy': (_I, [_P]),
     'blml_start_batch_create': (_I, [_I, _P, _P, _I, _D, _L, _L, _P, _P, _P, _P, _P, C.POINTER(_P)]),
+    'blml_start_batch_create_with': (_I, [_I, _P, _P, _I, _D, _L, _L, _P, _P, _P, _P, _P, ALLOC_FN, _P, _P,
+                                          C.POINTER(_P)]),
     'blml_start_batch_run': (_I, [_P, _P]),
     'blml_start_batch_result': (_I, [_P, _P, _P]),
     'blml_start_batch_stats': (_I, [_P, _P]),
@@ -208,6 +216,25 @@ def check(rc, what):
 
 def call(name, *args):
     check(getattr(lib(), name)(*args), name)
+
+
+class Lender:
+    """Device memory lent to the library (blml_alloc_fn) from torch's allocator, on the device's current stream. Keep it
+    until the objects created with it are destroyed."""
+
+    def __init__(self, device):
+        import torch
+        self.tensors = []
+
+        def alloc(nbytes, ctx):
+            try:
+                t = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+            except Exception:                      # none left: the library reports it (nothing may unwind through it)
+                return None
+            self.tensors.append(t)
+            return t.data_ptr()
+
+        self.fn = ALLOC_FN(alloc)
 
 
 def ptrs(arrs):

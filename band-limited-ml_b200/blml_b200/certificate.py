@@ -9,6 +9,7 @@ import torch
 
 from . import _lib
 from ._lib import call, ptrs, dbl
+from .noise import seeded_normals
 
 
 def lanczos_max(plan, dh, red, stream, tol=1e-6, seed=0, max_basis=96, max_restarts=20):
@@ -149,7 +150,7 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
     every = Subset(np.arange(F))
     nb = max_basis
     V = torch.empty((nb + 1, B), dtype=torch.float64, device=dev)
-    V[0].copy_(torch.as_tensor(np.random.default_rng(seed).standard_normal(B)))
+    seeded_normals(seed, B, dev, out=V[0])
     nrm = dots(every, [(V[0], V[0])])[:, 0]
     lin(every, V[0], (1.0 / np.sqrt(np.maximum(nrm, 1e-300)))[:, None], [V[0]])
     theta = np.zeros(F); done = np.zeros(F, bool); prev = np.full(F, np.nan); theta2 = np.full(F, np.nan)

@@ -27,6 +27,7 @@ from . import _lib
 from ._lib import call, ptrs
 from .spec import parse_modes, spec_key
 from .operator import pad_rule, mode_transform, kernel_at_zero, Plan
+from .noise import seeded_normals
 
 NT = 40
 _PLANS = OrderedDict()          # (kernel spec, lattice, dtype, device) -> (Plan, K(0))
@@ -58,11 +59,19 @@ class _Group:
         nb = np.ones(G, np.int32) if nbatch is None else np.ascontiguousarray(nbatch, np.int32)
         xo = np.ascontiguousarray(x_off, np.int64); yo = np.ascontiguousarray(y_off, np.int64)
         h = C.c_void_p()
-        call('blml_group_create', G, C.cast(arr, C.c_void_p), nb.ctypes.data_as(C.c_void_p), int(x_complex),
-             x.data_ptr(), xo.ctypes.data_as(C.c_void_p), y.data_ptr(), yo.ctypes.data_as(C.c_void_p), C.byref(h))
+        self._mem = _lib.Lender(x.device)
+        self._st = torch.cuda.current_stream(x.device).cuda_stream
+        call('blml_group_create_with', G, C.cast(arr, C.c_void_p), nb.ctypes.data_as(C.c_void_p), int(x_complex),
+             x.data_ptr(), xo.ctypes.data_as(C.c_void_p), y.data_ptr(), yo.ctypes.data_as(C.c_void_p), self._mem.fn, None,
+             self._st, C.byref(h))
         self._h = h; self._keep = (plans, x, y)
 
     def __call__(self, stream):
+        if (stream or 0) != self._st:                       # lent memory on another stream than its own
+            other = torch.cuda.ExternalStream(stream or 0, device=self._keep[1].device)
+            other.wait_stream(torch.cuda.ExternalStream(self._st, device=other.device))
+            for t in self._mem.tensors:
+                t.record_stream(other)
         call('blml_group_matvec', self._h, stream)
 
     @property
@@ -153,7 +162,8 @@ class BLMLBinnedBatch:
         self.Btot = int(boff[-1])
         self.w64 = w64
         self.w = w64.to(self.rt)
-        self.c64 = w64 * torch.as_tensor(np.repeat(self.n, self.B)).to(dev)
+        nB = torch.as_tensor(np.stack([self.n, self.B.astype(float)])).to(dev)
+        self.c64 = w64 * torch.repeat_interleave(nB[0], nB[1].long(), output_size=self.Btot)
         self.c = self.c64.to(self.rt)
         self.sg64 = torch.ones(self.Btot, dtype=torch.float64, device=dev); self.sg = self.sg64.to(self.rt)
         nb = _lib.lib().blml_seg_blocks()
@@ -333,11 +343,12 @@ class BLMLBinnedBatch:
         segs = (_Seg * F)(*self.segs_all)
         plans = (C.c_void_p * F)(*[p._h.value for p in self.p64])
         h = C.c_void_p()
+        mem = _lib.Lender(self.device)                      # until the runner is destroyed
         n = np.ascontiguousarray(self.n, np.float64); s0 = np.ascontiguousarray(self.s, np.float64)
-        call('blml_start_batch_create', F, C.cast(segs, C.c_void_p), C.cast(plans, C.c_void_p), int(self.anderson),
+        call('blml_start_batch_create_with', F, C.cast(segs, C.c_void_p), C.cast(plans, C.c_void_p), int(self.anderson),
              float(self.tol), -1 if self.max_sweeps is None else int(self.max_sweeps), int(self.stall),
              n.ctypes.data_as(C.c_void_p), s0.ctypes.data_as(C.c_void_p), self.c64.data_ptr(), self.sg64.data_ptr(),
-             E.data_ptr(), C.byref(h))
+             E.data_ptr(), mem.fn, None, self.st, C.byref(h))
         try:
             call('blml_start_batch_run', h, self.st)
             sweeps = np.zeros(F, np.int64)
@@ -358,18 +369,17 @@ class BLMLBinnedBatch:
         segs = (_Seg * F)(*self.segs_all)
         plans = (C.c_void_p * F)(*[p._h.value for p in self.pfit])
         h = C.c_void_p()
+        mem = _lib.Lender(self.device)                      # until the runner is destroyed
         n = np.ascontiguousarray(self.n, np.float64)
         ftol = self.ll_tol if self.ll_tol is not None else 1e-11
-        call('blml_lbfgs_batch_create', self.code, F, C.cast(segs, C.c_void_p), C.cast(plans, C.c_void_p),
+        call('blml_lbfgs_batch_create_with', self.code, F, C.cast(segs, C.c_void_p), C.cast(plans, C.c_void_p),
              self.lbfgs_m, float(self.tol), float(ftol), -1 if self.max_sweeps is None else int(self.max_sweeps),
              n.ctypes.data_as(C.c_void_p), self.w.data_ptr(), self.c.data_ptr(), E.data_ptr(), U.data_ptr(),
-             C.byref(h))
+             int(getattr(self, '_history_f32', False)), mem.fn, None, self.st, C.byref(h))
         try:
             if getattr(self, '_caps', None) is not None:
                 caps = np.ascontiguousarray(self._caps, np.int64)
                 call('blml_lbfgs_batch_set_caps', h, caps.ctypes.data_as(C.c_void_p))
-            if getattr(self, '_history_f32', False):
-                call('blml_lbfgs_batch_set_history', h, 1)
             call('blml_lbfgs_batch_run', h, self.st)
             it = np.zeros(F, np.int64); stop = np.zeros(F, np.int32); L = np.zeros(F); res = np.zeros(F)
             call('blml_lbfgs_batch_result', h, it.ctypes.data_as(C.c_void_p), stop.ctypes.data_as(C.c_void_p),
@@ -424,9 +434,11 @@ class BLMLBinnedBatch:
             er_fit = er.to(self.rt)
             call('blml_seg_real_to_complex', code, F, self.segs_t.data_ptr(), self.segs_t.data_ptr(),
                  er_fit.data_ptr(), E.data_ptr(), self.st)
-            z = np.concatenate([np.random.default_rng(self.seed).standard_normal(shape).ravel()
-                                for shape in self.shapes])
-            zt = torch.as_tensor(z, dtype=torch.float64).to(dev)
+            if isinstance(self.seed, (int, np.integer)):    # every fit draws from the seed afresh: the same values' prefix
+                z = seeded_normals(self.seed, int(self.B.max()), dev)
+                zt = torch.cat([z[:int(b)] for b in self.B])
+            else:
+                zt = torch.cat([seeded_normals(self.seed, int(b), dev) for b in self.B])
             call('blml_seg_phases', code, F, self.segs_t.data_ptr(), float(self.phase_noise), zt.data_ptr(),
                  E.data_ptr(), self.st)
         ev[1].record()

@@ -683,16 +683,24 @@ struct Runner {
   std::vector<blml_seg> segs_all;
   std::vector<int> ids;                 // current compact set (fit ids)
   blml_seg *d_segs_c = nullptr, *d_segs_eff = nullptr;
-  int *d_fid = nullptr, *d_live = nullptr, *h_live = nullptr;
+  int *d_fid = nullptr, *d_live = nullptr;
+  std::vector<int> h_live;
   cudaStream_t st = nullptr;
   cudaEvent_t ev = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   long long nodes = 0, steps = 0, replays = 0, rebuilds = 0;
-  std::vector<void*> allocs;
+  std::vector<void*> allocs;            // the library's own allocations
+  blml_alloc_fn lend = nullptr;         // or the caller's memory, first used behind what the caller's stream holds
+  void* lend_ctx = nullptr;
+  cudaStream_t lend_st = nullptr;
 
   void* dalloc(size_t bytes) {
     void* p = nullptr;
+    if (lend) {
+      p = lend(std::max<size_t>(bytes, 16), lend_ctx);
+      return p && begin(lend_st) == BLML_OK ? p : nullptr;
+    }
     if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) return nullptr;
     allocs.push_back(p);
     return p;
@@ -700,14 +708,14 @@ struct Runner {
   int base_init(int F_, const blml_seg* segs) {
     F = F_;
     segs_all.assign(segs, segs + F);
+    h_live.resize(F);
+    RC(cuda_status(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "batch runner stream"));
+    RC(cuda_status(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "batch runner event"));
     d_segs_c = (blml_seg*)dalloc(F * sizeof(blml_seg));
     d_segs_eff = (blml_seg*)dalloc(F * sizeof(blml_seg));
     d_fid = (int*)dalloc(F * sizeof(int));
     d_live = (int*)dalloc(F * sizeof(int));
     if (!d_segs_c || !d_segs_eff || !d_fid || !d_live) { set_error("batch runner: device allocation"); return BLML_ERR_CUDA; }
-    if (cudaMallocHost(&h_live, F * sizeof(int)) != cudaSuccess) { set_error("batch runner: pinned allocation"); return BLML_ERR_CUDA; }
-    RC(cuda_status(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "batch runner stream"));
-    RC(cuda_status(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "batch runner event"));
     return BLML_OK;
   }
   void drop_graph() {
@@ -720,10 +728,9 @@ struct Runner {
     if (st) cudaStreamSynchronize(st);
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
-    if (h_live) cudaFreeHost(h_live);
     if (ev) cudaEventDestroy(ev);
     if (st) cudaStreamDestroy(st);
-    h_live = nullptr; ev = nullptr; st = nullptr;
+    ev = nullptr; st = nullptr;
   }
   // the compact set: fits `sel`, all live, largest first (launches over fits dispatch their blocks in compact order,
   // so the longest-running fits start first and the small ones fill in behind them)
@@ -740,7 +747,7 @@ struct Runner {
   }
   // the live mask of every fit -> the fits still iterating
   int read_live(std::vector<int>& on) {
-    RC(cuda_status(cudaMemcpyAsync(h_live, d_live, F * sizeof(int), cudaMemcpyDeviceToHost, st), "live mask"));
+    RC(cuda_status(cudaMemcpyAsync(h_live.data(), d_live, F * sizeof(int), cudaMemcpyDeviceToHost, st), "live mask"));
     RC(cuda_status(cudaStreamSynchronize(st), "live mask"));
     on.clear();
     for (int f = 0; f < F; f++)
@@ -1070,19 +1077,19 @@ struct blml_start_batch_s : Runner {
   }
 };
 
-// one grouped mat-vec over every fit's K modes (the K lattices of fit f from off[f], one plan per fit)
-static int make_group(int F, const blml_plan* plans, const blml_seg* segs, int xc, const void* x, void* y,
-                      const std::vector<int64_t>& off, blml_group* out) {
+// one grouped mat-vec over every fit's K modes (the K lattices of fit f from off[f], one plan per fit); the runner's
+// groups run one after another on its stream and share the buffers of `first`
+static int make_group(Runner* r, int F, const blml_plan* plans, const blml_seg* segs, int xc, const void* x, void* y,
+                      const std::vector<int64_t>& off, blml_group first, blml_group* out) {
   std::vector<int> nb(F);
   for (int f = 0; f < F; f++) nb[f] = segs[f].K;
-  return blml_group_create(F, plans, nb.data(), xc, x, off.data(), y, off.data(), out);
+  return group_create(F, plans, nb.data(), xc, x, off.data(), y, off.data(), r->lend, r->lend_ctx, r->lend_st,
+                      first ? group_ws(first) : nullptr, true, out);
 }
 
-extern "C" {
-
-int blml_lbfgs_batch_create(int dtype, int F, const blml_seg* segs, const blml_plan* plans, int m, double tol,
-                            double ll_tol, int64_t max_iters, const double* n, const void* w, const void* c, void* E,
-                            void* U, blml_lbfgs_batch* out) {
+static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan* plans, int m, double tol,
+                        double ll_tol, int64_t max_iters, const double* n, const void* w, const void* c, void* E,
+                        void* U, int h32, blml_alloc_fn lend, void* ctx, void* stream, blml_lbfgs_batch* out) {
   if ((dtype != BLML_F64 && dtype != BLML_F32) || F < 1 || F > 65535 || !segs || !plans || !n || !w || !c || !E ||
       !U || !out || m < 1 || m > LB_MMAX) {
     set_error("blml_lbfgs_batch_create: dtype, 1 <= F <= 65535 fits, 1 <= m <= 20 and every pointer");
@@ -1101,21 +1108,23 @@ int blml_lbfgs_batch_create(int dtype, int F, const blml_seg* segs, const blml_p
   blml_lbfgs_batch_s* r = new blml_lbfgs_batch_s();
   r->m = m; r->dtype = dtype; r->tol = tol; r->ftol = ll_tol; r->cap = max_iters < 0 ? LLONG_MAX : max_iters;
   r->E = E; r->U = U; r->w = w; r->c = c;
+  r->h32 = h32 && dtype == BLML_F64;     // (float32 state: the history is float32 already)
+  r->lend = lend; r->lend_ctx = ctx; r->lend_st = reinterpret_cast<cudaStream_t>(stream);
   int rc = r->base_init(F, segs);
-  const size_t esz = dtype == BLML_F64 ? 16 : 8;
+  const size_t esz = dtype == BLML_F64 ? 16 : 8, hsz = r->h32 ? 8 : esz;
   char* vec = rc ? nullptr : (char*)r->dalloc(6 * tot * esz);
-  char* hv = rc ? nullptr : (char*)r->dalloc(2 * (size_t)m * tot * esz);
+  char* hv = rc ? nullptr : (char*)r->dalloc(2 * (size_t)m * tot * hsz);
   if (!rc && (!vec || !hv)) { set_error("blml_lbfgs_batch_create: vector allocation"); rc = BLML_ERR_CUDA; }
   if (!rc) {
     r->tot = tot; r->hvec = hv;
     void** v6[6] = {&r->g, &r->gn, &r->q, &r->Sq, &r->V, &r->SV};
     for (int i = 0; i < 6; i++) *v6[i] = vec + (size_t)i * tot * esz;
     for (int i = 0; i < m; i++) {
-      r->Sh[i] = hv + (size_t)i * tot * esz;
-      r->Yh[i] = hv + ((size_t)m + i) * tot * esz;
+      r->Sh[i] = hv + (size_t)i * tot * hsz;
+      r->Yh[i] = hv + ((size_t)m + i) * tot * hsz;
     }
     cudaMemsetAsync(vec, 0, 6 * tot * esz, r->st);
-    cudaMemsetAsync(hv, 0, 2 * (size_t)m * tot * esz, r->st);
+    cudaMemsetAsync(hv, 0, 2 * (size_t)m * tot * hsz, r->st);
     // >= Fa * seg_blocks_for(Fa) for every Fa <= F, and 48 pw >= 43 (SEG_SPLIT_BLOCKS + Fa) for the split scan
     const size_t pw = (size_t)SEG_PART_WIDTH(F);
     const int nq = 48;                    // the widest reduction: blml_seg_dots' 48 accumulators
@@ -1149,12 +1158,29 @@ int blml_lbfgs_batch_create(int dtype, int F, const blml_seg* segs, const blml_p
       if (!rc) rc = cuda_status(cudaStreamSynchronize(r->st), "lbfgs create");
     }
   }
-  if (!rc) rc = make_group(F, plans, segs, 1, E, U, off, &r->gEU);
-  if (!rc) rc = make_group(F, plans, segs, 1, r->q, r->Sq, off, &r->gq);
-  if (!rc) rc = make_group(F, plans, segs, 1, r->V, r->SV, off, &r->gV);
+  if (!rc) rc = make_group(r, F, plans, segs, 1, E, U, off, nullptr, &r->gEU);
+  if (!rc) rc = make_group(r, F, plans, segs, 1, r->q, r->Sq, off, r->gEU, &r->gq);
+  if (!rc) rc = make_group(r, F, plans, segs, 1, r->V, r->SV, off, r->gEU, &r->gV);
+  if (!rc && lend) rc = r->begin(stream);           // the descriptors' copies
   if (rc) { r->release(); delete r; return rc; }
   *out = r;
   return BLML_OK;
+}
+
+extern "C" {
+
+int blml_lbfgs_batch_create(int dtype, int F, const blml_seg* segs, const blml_plan* plans, int m, double tol,
+                            double ll_tol, int64_t max_iters, const double* n, const void* w, const void* c, void* E,
+                            void* U, blml_lbfgs_batch* out) {
+  return lbfgs_create(dtype, F, segs, plans, m, tol, ll_tol, max_iters, n, w, c, E, U, 0, nullptr, nullptr, nullptr, out);
+}
+
+int blml_lbfgs_batch_create_with(int dtype, int F, const blml_seg* segs, const blml_plan* plans, int m, double tol,
+                                 double ll_tol, int64_t max_iters, const double* n, const void* w, const void* c,
+                                 void* E, void* U, int history_f32, blml_alloc_fn alloc, void* ctx, void* stream,
+                                 blml_lbfgs_batch* out) {
+  if (!alloc) { set_error("blml_lbfgs_batch_create_with: null allocator"); return BLML_ERR_ARG; }
+  return lbfgs_create(dtype, F, segs, plans, m, tol, ll_tol, max_iters, n, w, c, E, U, history_f32, alloc, ctx, stream, out);
 }
 
 int blml_lbfgs_batch_set_history(blml_lbfgs_batch r, int f32) {
@@ -1164,12 +1190,15 @@ int blml_lbfgs_batch_set_history(blml_lbfgs_batch r, int f32) {
   // a complex64 history in place of the complex128 one (half its size); the old allocation is released
   const size_t bytes = 2 * (size_t)r->m * r->tot * 8;
   void* hv = nullptr;
-  if (cudaMalloc(&hv, bytes) != cudaSuccess) { set_error("blml_lbfgs_batch_set_history: allocation"); return BLML_ERR_CUDA; }
+  if (r->lend) hv = r->dalloc(bytes);               // the lent one stays the caller's until the runner is destroyed
+  else if (cudaMalloc(&hv, bytes) != cudaSuccess) hv = nullptr;
+  if (!hv) { set_error("blml_lbfgs_batch_set_history: allocation"); return BLML_ERR_CUDA; }
   int rc = cuda_status(cudaStreamSynchronize(r->st), "blml_lbfgs_batch_set_history");
   if (!rc) rc = cuda_status(cudaMemsetAsync(hv, 0, bytes, r->st), "blml_lbfgs_batch_set_history");
-  if (rc) { cudaFree(hv); return rc; }
-  for (auto& p : r->allocs)
-    if (p == r->hvec) { cudaFree(p); p = hv; break; }
+  if (rc) { if (!r->lend) cudaFree(hv); return rc; }
+  if (!r->lend)
+    for (auto& p : r->allocs)
+      if (p == r->hvec) { cudaFree(p); p = hv; break; }
   r->hvec = hv;
   for (int i = 0; i < r->m; i++) {
     r->Sh[i] = (char*)hv + (size_t)i * r->tot * 8;
@@ -1232,9 +1261,11 @@ int blml_lbfgs_batch_destroy(blml_lbfgs_batch r) {
   return BLML_OK;
 }
 
-int blml_start_batch_create(int F, const blml_seg* segs, const blml_plan* plans, int mA, double tol,
-                            int64_t max_sweeps, int64_t stall, const double* n, const double* s0, const double* c,
-                            const double* sg, double* E, blml_start_batch* out) {
+}  // extern "C"
+
+static int start_create(int F, const blml_seg* segs, const blml_plan* plans, int mA, double tol, int64_t max_sweeps,
+                        int64_t stall, const double* n, const double* s0, const double* c, const double* sg, double* E,
+                        blml_alloc_fn lend, void* ctx, void* stream, blml_start_batch* out) {
   if (F < 1 || F > 65535 || !segs || !plans || !n || !s0 || !c || !sg || !E || !out || mA < 0 || mA > AA_MMAX) {
     set_error("blml_start_batch_create: 1 <= F <= 65535 fits, 0 <= anderson <= 8 and every pointer");
     return BLML_ERR_ARG;
@@ -1251,6 +1282,7 @@ int blml_start_batch_create(int F, const blml_seg* segs, const blml_plan* plans,
   r->mA = mA; r->tol = tol; r->cap = max_sweeps < 0 ? LLONG_MAX : max_sweeps; r->stall = stall;
   r->E = E; r->c = c; r->sg = sg;
   r->s0_host.assign(s0, s0 + F);
+  r->lend = lend; r->lend_ctx = ctx; r->lend_st = reinterpret_cast<cudaStream_t>(stream);
   int rc = r->base_init(F, segs);
   double* vec = rc ? nullptr : (double*)r->dalloc((10 + 2 * (size_t)mA) * tot * sizeof(double));
   if (!rc && !vec) { set_error("blml_start_batch_create: vector allocation"); rc = BLML_ERR_CUDA; }
@@ -1289,12 +1321,29 @@ int blml_start_batch_create(int F, const blml_seg* segs, const blml_plan* plans,
       if (!rc) rc = cuda_status(cudaStreamSynchronize(r->st), "start create");
     }
   }
-  if (!rc) rc = make_group(F, plans, segs, 0, E, r->U, off, &r->gEU);
-  if (!rc) rc = make_group(F, plans, segs, 0, r->EJ, r->UJ, off, &r->gJ);
-  if (!rc) rc = make_group(F, plans, segs, 0, r->EA, r->UA, off, &r->gA);
+  if (!rc) rc = make_group(r, F, plans, segs, 0, E, r->U, off, nullptr, &r->gEU);
+  if (!rc) rc = make_group(r, F, plans, segs, 0, r->EJ, r->UJ, off, r->gEU, &r->gJ);
+  if (!rc) rc = make_group(r, F, plans, segs, 0, r->EA, r->UA, off, r->gEU, &r->gA);
+  if (!rc && lend) rc = r->begin(stream);
   if (rc) { r->release(); delete r; return rc; }
   *out = r;
   return BLML_OK;
+}
+
+extern "C" {
+
+int blml_start_batch_create(int F, const blml_seg* segs, const blml_plan* plans, int mA, double tol,
+                            int64_t max_sweeps, int64_t stall, const double* n, const double* s0, const double* c,
+                            const double* sg, double* E, blml_start_batch* out) {
+  return start_create(F, segs, plans, mA, tol, max_sweeps, stall, n, s0, c, sg, E, nullptr, nullptr, nullptr, out);
+}
+
+int blml_start_batch_create_with(int F, const blml_seg* segs, const blml_plan* plans, int mA, double tol,
+                                 int64_t max_sweeps, int64_t stall, const double* n, const double* s0, const double* c,
+                                 const double* sg, double* E, blml_alloc_fn alloc, void* ctx, void* stream,
+                                 blml_start_batch* out) {
+  if (!alloc) { set_error("blml_start_batch_create_with: null allocator"); return BLML_ERR_ARG; }
+  return start_create(F, segs, plans, mA, tol, max_sweeps, stall, n, s0, c, sg, E, alloc, ctx, stream, out);
 }
 
 int blml_start_batch_run(blml_start_batch r, void* stream) {

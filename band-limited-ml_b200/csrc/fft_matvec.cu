@@ -792,8 +792,11 @@ static int launch_fft_one(const FftDesc& D, size_t smA, size_t smB, cudaStream_t
   return BLML_OK;
 }
 
+static size_t desc_bytes(int G) { return ((size_t)G * sizeof(FftDesc) + 255) & ~(size_t)255; }
+size_t fft_group_bytes(int G) { return desc_bytes(G) + sizeof(FftSched); }
+
 int fft_group_init(void** out, int G, const blml_plan* plans, const int* nbatch, int xc, const void* const* x,
-                   void* const* y, void* const* z) {
+                   void* const* y, void* const* z, void* dev, std::vector<char>& up) {
   *out = nullptr;
   for (int g = 0; g < G; g++)
     if (!plans[g]->fft) return BLML_OK;
@@ -817,21 +820,16 @@ int fft_group_init(void** out, int G, const blml_plan* plans, const int* nbatch,
   const int nmax = std::min(G, kSchedMax);
   fg->boundA.assign(nmax + 1, 0); fg->boundB.assign(nmax + 1, 0);
   for (int i = 0; i < nmax; i++) { fg->boundA[i + 1] = fg->boundA[i] + cA[i]; fg->boundB[i + 1] = fg->boundB[i] + cB[i]; }
-  int e = fft_smem_once();
-  if (!e && cudaMalloc(&fg->dev, G * sizeof(FftDesc)) != cudaSuccess) { set_error("FFT route: allocation"); e = BLML_ERR_CUDA; }
-  if (!e && cudaMalloc(&fg->sch, sizeof(FftSched)) != cudaSuccess) { set_error("FFT route: allocation"); e = BLML_ERR_CUDA; }
-  if (!e) e = cuda_status(cudaMemcpy(fg->dev, h.data(), G * sizeof(FftDesc), cudaMemcpyHostToDevice), "FFT route");
-  if (e) { fft_group_free(fg); return e; }
+  const int e = fft_smem_once();
+  if (e) { delete fg; return e; }
+  fg->dev = reinterpret_cast<FftDesc*>(dev);
+  fg->sch = reinterpret_cast<FftSched*>(reinterpret_cast<char*>(dev) + desc_bytes(G));
+  up.assign(reinterpret_cast<const char*>(h.data()), reinterpret_cast<const char*>(h.data() + G));
   *out = fg;
   return BLML_OK;
 }
 
-void fft_group_free(void* fgv) {
-  FftGroup* fg = reinterpret_cast<FftGroup*>(fgv);
-  if (!fg) return;
-  cudaFree(fg->dev); cudaFree(fg->sch);
-  delete fg;
-}
+void fft_group_free(void* fgv) { delete reinterpret_cast<FftGroup*>(fgv); }
 
 // problems of the launch in chunks of kSchedMax (one schedule buffer: the chunks run one after another on st)
 int fft_group_launch(void* fgv, int dtype, const int* subset, int n, const int* live, cudaStream_t st) {

@@ -664,17 +664,117 @@ __global__ void __launch_bounds__(256, 2) k_contract_grouped_big(const StageDesc
 // a set of mat-vecs applied together: per stage a device array of descriptors and the grid that covers them
 struct blml_group_s {
   int G, d_max, dtype, nstages;
-  std::vector<blml::StageDesc*> dev;    // one descriptor array per stage index
+  std::vector<blml::StageDesc*> dev;    // one descriptor array per stage index (empty: the FFT route alone)
   std::vector<dim3> grids, grids_big;   // 32 x 32 and 64 x 64 tile grids per stage
   std::vector<double> tiles_big;        // 64 x 64 tiles of a stage over all problems
   std::vector<double> blocks8;          // its 8 x 8 blocks (float64)
   std::vector<int64_t> max_rows, max_n, max_m;   // the largest problem's rows, frequencies and terms per stage
-  void* ws;                             // the group's own intermediate buffers
+  void* ws;                             // the intermediate buffers
+  std::vector<void*> own;               // the library's allocations (none in lent memory)
   void* fft;                            // the FFT route's descriptors (every plan a DFT mask), or null
   int route;                            // BLML_ROUTE_CONTRACT or BLML_ROUTE_FFT
 };
 
 using namespace blml;
+
+namespace blml {
+void* group_ws(blml_group g) { return g->ws; }
+
+int group_create(int G, const blml_plan* plans, const int* nbatch, int x_complex, const void* x_base,
+                 const int64_t* x_off, void* y_base, const int64_t* y_off, blml_alloc_fn alloc, void* ctx,
+                 cudaStream_t st, void* ws, bool fft_only, blml_group* out) {
+  if (G < 1 || G > 65535 || !plans || !nbatch || !x_off || !y_off || !out) {
+    set_error("blml_group_create: bad arguments"); return BLML_ERR_ARG;
+  }
+  const int d = plans[0]->d, dtype = plans[0]->dtype;
+  for (int g = 0; g < G; g++)
+    if (!plans[g] || plans[g]->d != d || plans[g]->dtype != dtype || nbatch[g] < 1) {
+      set_error("blml_group_create: every plan of a group has one dimension count and dtype"); return BLML_ERR_ARG;
+    }
+  // the stage kernels' dynamic shared memory (set here, outside any stream capture)
+  if (dtype == BLML_F32) {
+    const int e0 = cuda_status(cudaFuncSetAttribute(k_contract_grouped_big<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (int)big_smem<float>()), "blml_group_create");
+    if (e0) return e0;
+  } else if (const int e0 = stage_smem_once()) {
+    return e0;
+  }
+  const size_t esz = dtype == BLML_F64 ? 16 : 8, rsz = dtype == BLML_F64 ? 8 : 4;
+  const size_t xsz = x_complex ? esz : rsz, ysz = x_complex ? esz : rsz;
+  bool all_fft = true;
+  for (int g = 0; g < G; g++) all_fft &= plans[g]->fft != nullptr;
+  const bool contract = !(all_fft && fft_only);
+  std::vector<size_t> wso(G + 1, 0);
+  for (int g = 0; g < G; g++) wso[g + 1] = wso[g] + (contract ? 2 : 1) * (size_t)nbatch[g] * plans[g]->max_elems * esz;
+  const size_t stage_b = ((size_t)G * sizeof(StageDesc) + 255) & ~(size_t)255, desc_b = contract ? 2 * d * stage_b : 0;
+  blml_group_s* grp = new blml_group_s();
+  grp->G = G; grp->d_max = d; grp->dtype = dtype; grp->nstages = 2 * d; grp->ws = nullptr;
+  grp->fft = nullptr; grp->route = BLML_ROUTE_CONTRACT;
+  auto take = [&](size_t bytes) -> void* {
+    void* p = nullptr;
+    if (alloc) return alloc(std::max<size_t>(bytes, 16), ctx);
+    if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) return nullptr;
+    grp->own.push_back(p);
+    return p;
+  };
+  grp->ws = ws ? ws : take(wso[G]);
+  char* desc = (char*)take(desc_b + (all_fft ? fft_group_bytes(G) : 0));
+  if (!grp->ws || !desc) { blml_group_destroy(grp); set_error("blml_group_create: workspace allocation"); return BLML_ERR_CUDA; }
+  std::vector<std::vector<StageDesc>> host(contract ? 2 * d : 0, std::vector<StageDesc>(G));
+  std::vector<int64_t> maxr(2 * d, 0), maxn(2 * d, 0), maxm(2 * d, 0);
+  grp->tiles_big.assign(2 * d, 0.0); grp->blocks8.assign(2 * d, 0.0);
+  for (int g = 0; g < G && contract; g++) {
+    const blml_plan_s* p = plans[g];
+    std::vector<int64_t> dims(p->shape, p->shape + d);
+    char* buf[2] = {reinterpret_cast<char*>(grp->ws) + wso[g],
+                    reinterpret_cast<char*>(grp->ws) + wso[g] + (size_t)nbatch[g] * p->max_elems * esz};
+    const void* cur = reinterpret_cast<const char*>(x_base) + x_off[g] * xsz;
+    for (int s = 0; s < 2 * d; s++) {
+      const bool fwd = s < d, last = s == 2 * d - 1;
+      const int a = d - 1 - (s % d);
+      const int64_t M = dims.back();
+      int64_t tot = 1; for (auto v : dims) tot *= v;
+      const int64_t R = tot / M, N = fwd ? p->nfreq[a] : p->shape[a];
+      void* outp = last ? reinterpret_cast<char*>(y_base) + y_off[g] * ysz : buf[s & 1];
+      StageDesc& D = host[s][g];
+      D.X = cur; D.T = fwd ? p->tf[a] : p->ti[a]; D.W = (s == d - 1) ? p->W : nullptr; D.Y = outp;
+      D.R = R; D.M = (int)M; D.N = (int)N; D.nb = nbatch[g];
+      D.flags = ((s == 0 && !x_complex) ? 1 : 0) | ((s == d - 1) ? 2 : 0) | ((last && !x_complex) ? 4 : 0) |
+                ((reinterpret_cast<uintptr_t>(cur) & 15) ? 8 : 0);
+      maxr[s] = std::max(maxr[s], R * nbatch[g]); maxm[s] = std::max(maxm[s], M); maxn[s] = std::max<int64_t>(maxn[s], N);
+      grp->blocks8[s] += (double)tiles_of(R * nbatch[g], 8) * (double)tiles_of(N, 8);
+      grp->tiles_big[s] += (double)((R * nbatch[g] + BR - 1) / BR) * (double)((N + BN - 1) / BN);
+      dims.pop_back(); dims.insert(dims.begin(), N);
+      cur = outp;
+    }
+  }
+  grp->max_rows = maxr; grp->max_n = maxn; grp->max_m = maxm;
+  int e = BLML_OK;
+  std::vector<char> up(desc_b);                 // the descriptors, in one copy
+  for (int s = 0; s < 2 * d && contract; s++) {
+    grp->dev.push_back(reinterpret_cast<StageDesc*>(desc + s * stage_b));
+    std::copy_n(reinterpret_cast<const char*>(host[s].data()), G * sizeof(StageDesc), up.data() + s * stage_b);
+    grp->grids.push_back(dim3((unsigned)((maxr[s] + GR - 1) / GR), (unsigned)((maxn[s] + GN - 1) / GN), (unsigned)G));
+    grp->grids_big.push_back(dim3((unsigned)((maxr[s] + BR - 1) / BR), (unsigned)((maxn[s] + BN - 1) / BN), (unsigned)G));
+  }
+  if (all_fft) {      // the FFT route: problem g keeps its spectrum in the first of its two intermediate buffers
+    std::vector<const void*> xs(G); std::vector<void*> ys(G), zs(G);
+    for (int g = 0; g < G; g++) {
+      xs[g] = reinterpret_cast<const char*>(x_base) + x_off[g] * xsz;
+      ys[g] = reinterpret_cast<char*>(y_base) + y_off[g] * ysz;
+      zs[g] = reinterpret_cast<char*>(grp->ws) + wso[g];
+    }
+    std::vector<char> fd;
+    e = fft_group_init(&grp->fft, G, plans, nbatch, x_complex, xs.data(), ys.data(), zs.data(), desc + desc_b, fd);
+    if (!e) { grp->route = BLML_ROUTE_FFT; up.insert(up.end(), fd.begin(), fd.end()); }
+  }
+  if (!e) e = alloc ? cuda_status(cudaMemcpyAsync(desc, up.data(), up.size(), cudaMemcpyHostToDevice, st), "blml_group_create")
+                    : cuda_status(cudaMemcpy(desc, up.data(), up.size(), cudaMemcpyHostToDevice), "blml_group_create");
+  if (e) { blml_group_destroy(grp); return e; }
+  *out = grp;
+  return BLML_OK;
+}
+}  // namespace blml
 
 extern "C" {
 
@@ -771,80 +871,15 @@ int blml_plan_destroy(blml_plan p) {
 
 int blml_group_create(int G, const blml_plan* plans, const int* nbatch, int x_complex, const void* x_base,
                       const int64_t* x_off, void* y_base, const int64_t* y_off, blml_group* out) {
-  if (G < 1 || G > 65535 || !plans || !nbatch || !x_off || !y_off || !out) {
-    set_error("blml_group_create: bad arguments"); return BLML_ERR_ARG;
-  }
-  const int d = plans[0]->d, dtype = plans[0]->dtype;
-  for (int g = 0; g < G; g++)
-    if (!plans[g] || plans[g]->d != d || plans[g]->dtype != dtype || nbatch[g] < 1) {
-      set_error("blml_group_create: every plan of a group has one dimension count and dtype"); return BLML_ERR_ARG;
-    }
-  // the 64 x 64 stage kernel's dynamic shared memory (set here, outside any stream capture)
-  if (dtype == BLML_F32) {
-    const int e0 = cuda_status(cudaFuncSetAttribute(k_contract_grouped_big<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    (int)big_smem<float>()), "blml_group_create");
-    if (e0) return e0;
-  }
-  const size_t esz = dtype == BLML_F64 ? 16 : 8, rsz = dtype == BLML_F64 ? 8 : 4;
-  const size_t xsz = x_complex ? esz : rsz, ysz = x_complex ? esz : rsz;
-  std::vector<size_t> wso(G + 1, 0);
-  for (int g = 0; g < G; g++) wso[g + 1] = wso[g] + 2 * (size_t)nbatch[g] * plans[g]->max_elems * esz;
-  blml_group_s* grp = new blml_group_s();
-  grp->G = G; grp->d_max = d; grp->dtype = dtype; grp->nstages = 2 * d; grp->ws = nullptr;
-  grp->fft = nullptr; grp->route = BLML_ROUTE_CONTRACT;
-  if (cudaMalloc(&grp->ws, std::max<size_t>(wso[G], 16)) != cudaSuccess) {
-    delete grp; set_error("blml_group_create: workspace allocation"); return BLML_ERR_CUDA;
-  }
-  std::vector<std::vector<StageDesc>> host(2 * d, std::vector<StageDesc>(G));
-  std::vector<int64_t> maxr(2 * d, 0), maxn(2 * d, 0), maxm(2 * d, 0);
-  grp->tiles_big.assign(2 * d, 0.0); grp->blocks8.assign(2 * d, 0.0);
-  for (int g = 0; g < G; g++) {
-    const blml_plan_s* p = plans[g];
-    std::vector<int64_t> dims(p->shape, p->shape + d);
-    char* buf[2] = {reinterpret_cast<char*>(grp->ws) + wso[g],
-                    reinterpret_cast<char*>(grp->ws) + wso[g] + (size_t)nbatch[g] * p->max_elems * esz};
-    const void* cur = reinterpret_cast<const char*>(x_base) + x_off[g] * xsz;
-    for (int s = 0; s < 2 * d; s++) {
-      const bool fwd = s < d, last = s == 2 * d - 1;
-      const int a = d - 1 - (s % d);
-      const int64_t M = dims.back();
-      int64_t tot = 1; for (auto v : dims) tot *= v;
-      const int64_t R = tot / M, N = fwd ? p->nfreq[a] : p->shape[a];
-      void* outp = last ? reinterpret_cast<char*>(y_base) + y_off[g] * ysz : buf[s & 1];
-      StageDesc& D = host[s][g];
-      D.X = cur; D.T = fwd ? p->tf[a] : p->ti[a]; D.W = (s == d - 1) ? p->W : nullptr; D.Y = outp;
-      D.R = R; D.M = (int)M; D.N = (int)N; D.nb = nbatch[g];
-      D.flags = ((s == 0 && !x_complex) ? 1 : 0) | ((s == d - 1) ? 2 : 0) | ((last && !x_complex) ? 4 : 0) |
-                ((reinterpret_cast<uintptr_t>(cur) & 15) ? 8 : 0);
-      maxr[s] = std::max(maxr[s], R * nbatch[g]); maxm[s] = std::max(maxm[s], M); maxn[s] = std::max<int64_t>(maxn[s], N);
-      grp->blocks8[s] += (double)tiles_of(R * nbatch[g], 8) * (double)tiles_of(N, 8);
-      grp->tiles_big[s] += (double)((R * nbatch[g] + BR - 1) / BR) * (double)((N + BN - 1) / BN);
-      dims.pop_back(); dims.insert(dims.begin(), N);
-      cur = outp;
-    }
-  }
-  grp->max_rows = maxr; grp->max_n = maxn; grp->max_m = maxm;
-  int e = BLML_OK;
-  grp->dev.assign(2 * d, nullptr);
-  for (int s = 0; s < 2 * d && !e; s++) {
-    if (cudaMalloc(&grp->dev[s], G * sizeof(StageDesc)) != cudaSuccess) { set_error("blml_group_create: allocation"); e = BLML_ERR_CUDA; break; }
-    e = cuda_status(cudaMemcpy(grp->dev[s], host[s].data(), G * sizeof(StageDesc), cudaMemcpyHostToDevice), "blml_group_create");
-    grp->grids.push_back(dim3((unsigned)((maxr[s] + GR - 1) / GR), (unsigned)((maxn[s] + GN - 1) / GN), (unsigned)G));
-    grp->grids_big.push_back(dim3((unsigned)((maxr[s] + BR - 1) / BR), (unsigned)((maxn[s] + BN - 1) / BN), (unsigned)G));
-  }
-  if (!e) {      // the FFT route: problem g keeps its spectrum in the first of its two intermediate buffers
-    std::vector<const void*> xs(G); std::vector<void*> ys(G), zs(G);
-    for (int g = 0; g < G; g++) {
-      xs[g] = reinterpret_cast<const char*>(x_base) + x_off[g] * xsz;
-      ys[g] = reinterpret_cast<char*>(y_base) + y_off[g] * ysz;
-      zs[g] = reinterpret_cast<char*>(grp->ws) + wso[g];
-    }
-    e = fft_group_init(&grp->fft, G, plans, nbatch, x_complex, xs.data(), ys.data(), zs.data());
-    if (!e && grp->fft) grp->route = BLML_ROUTE_FFT;
-  }
-  if (e) { blml_group_destroy(grp); return e; }
-  *out = grp;
-  return BLML_OK;
+  return group_create(G, plans, nbatch, x_complex, x_base, x_off, y_base, y_off, nullptr, nullptr, nullptr, nullptr, false, out);
+}
+
+int blml_group_create_with(int G, const blml_plan* plans, const int* nbatch, int x_complex, const void* x_base,
+                           const int64_t* x_off, void* y_base, const int64_t* y_off, blml_alloc_fn alloc, void* ctx,
+                           void* stream, blml_group* out) {
+  if (!alloc) { set_error("blml_group_create_with: null allocator"); return BLML_ERR_ARG; }
+  return group_create(G, plans, nbatch, x_complex, x_base, x_off, y_base, y_off, alloc, ctx,
+                      reinterpret_cast<cudaStream_t>(stream), nullptr, false, out);
 }
 
 int blml_group_matvec(blml_group grp, void* stream) {
@@ -879,9 +914,8 @@ int blml_group_matvec_masked(blml_group grp, const int* subset, int n, const int
 
 int blml_group_destroy(blml_group grp) {
   if (!grp) return BLML_OK;
-  for (auto p : grp->dev) cudaFree(p);
-  cudaFree(grp->ws);
-  fft_group_free(grp->fft);
+  for (auto p : grp->own) cudaFree(p);
+  if (grp->fft) fft_group_free(grp->fft);
   delete grp;
   return BLML_OK;
 }
@@ -936,6 +970,9 @@ int blml_group_set_route(blml_group grp, int route) {
     set_error("blml_group_set_route: a plan of this group has no FFT route"); return BLML_ERR_UNSUPPORTED;
   }
   if (route != BLML_ROUTE_FFT && route != BLML_ROUTE_CONTRACT) { set_error("blml_group_set_route: route"); return BLML_ERR_ARG; }
+  if (route == BLML_ROUTE_CONTRACT && grp->dev.empty()) {
+    set_error("blml_group_set_route: this group has the FFT route alone"); return BLML_ERR_UNSUPPORTED;
+  }
   grp->route = route;
   return BLML_OK;
 }

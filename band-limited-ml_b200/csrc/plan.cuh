@@ -31,9 +31,18 @@ void fft_plan_free(blml_plan_s* p);
 int64_t fft_workspace(const blml_plan_s* p, int nb);
 int fft_matvec(blml_plan_s* p, const void* x, void* y, int nb, int xc, void* ws, cudaStream_t st);
 // a group's descriptors: problem g reads x[g], writes y[g] and keeps its spectrum in z[g] (its workspace); *out stays
-// null when a plan has no FFT route
+// null when a plan has no FFT route. dev: fft_group_bytes(G) bytes of device memory (kept); its first bytes are to be
+// filled from `up`
+size_t fft_group_bytes(int G);
 int fft_group_init(void** out, int G, const blml_plan* plans, const int* nbatch, int xc, const void* const* x,
-                   void* const* y, void* const* z);
+                   void* const* y, void* const* z, void* dev, std::vector<char>& up);
 void fft_group_free(void* fg);
+// blml_group_create in the caller's memory (alloc null: the library's own); ws: intermediate buffers shared with a group
+// of the same problems whose launches do not overlap this one's (null: its own); fft_only: no contraction descriptors
+// when every plan has the FFT route
+int group_create(int G, const blml_plan* plans, const int* nbatch, int x_complex, const void* x_base,
+                 const int64_t* x_off, void* y_base, const int64_t* y_off, blml_alloc_fn alloc, void* ctx,
+                 cudaStream_t st, void* ws, bool fft_only, blml_group* out);
+void* group_ws(blml_group g);
 int fft_group_launch(void* fg, int dtype, const int* subset, int n, const int* live, cudaStream_t st);
 }  // namespace blml

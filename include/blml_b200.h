@@ -12,6 +12,7 @@
  */
 #ifndef BLML_B200_H
 #define BLML_B200_H
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -67,6 +68,14 @@ int blml_plan_route(blml_plan plan);
 typedef struct blml_group_s* blml_group;
 int blml_group_create(int G, const blml_plan* plans, const int* nbatch, int x_complex, const void* x_base,
                       const int64_t* x_off, void* y_base, const int64_t* y_off, blml_group* group);
+/* Device memory that the caller lends: `bytes` bytes of the current device, aligned to 256 (null: none). The memory
+ * is first used behind the work that `stream` held when the function was called; the caller takes it back once the
+ * object is destroyed and, for a group, its launches are done (a runner's destroy waits for its own). The function and
+ * ctx stay valid until then. It must not unwind into the library. */
+typedef void* (*blml_alloc_fn)(size_t bytes, void* ctx);
+int blml_group_create_with(int G, const blml_plan* plans, const int* nbatch, int x_complex, const void* x_base,
+                           const int64_t* x_off, void* y_base, const int64_t* y_off, blml_alloc_fn alloc, void* ctx,
+                           void* stream, blml_group* group);
 int blml_group_matvec(blml_group group, void* stream);
 /* the same for the n problems g = subset[i] (device int array; null: problems 0 .. n-1), skipping those with
    live[g] == 0 (device int array over all G problems, or null), both read when the kernels run, so a captured CUDA
@@ -310,6 +319,11 @@ typedef struct blml_lbfgs_batch_s* blml_lbfgs_batch;
 int blml_lbfgs_batch_create(int dtype, int F, const blml_seg* segs, const blml_plan* plans, int m, double tol,
                             double ll_tol, int64_t max_iters, const double* n, const void* w, const void* c, void* E,
                             void* U, blml_lbfgs_batch* runner);
+/* the same in lent memory (blml_alloc_fn); history_f32: blml_lbfgs_batch_set_history from the start */
+int blml_lbfgs_batch_create_with(int dtype, int F, const blml_seg* segs, const blml_plan* plans, int m, double tol,
+                                 double ll_tol, int64_t max_iters, const double* n, const void* w, const void* c,
+                                 void* E, void* U, int history_f32, blml_alloc_fn alloc, void* ctx, void* stream,
+                                 blml_lbfgs_batch* runner);
 /* per-fit iteration caps (F host values, < 0: none) in place of max_iters, before blml_lbfgs_batch_run: rounds of a
    certified fit cap the fits still growing their rank and let the final ones run to tol */
 int blml_lbfgs_batch_set_caps(blml_lbfgs_batch runner, const int64_t* caps);
@@ -348,6 +362,11 @@ typedef struct blml_start_batch_s* blml_start_batch;
 int blml_start_batch_create(int F, const blml_seg* segs, const blml_plan* plans, int anderson, double tol,
                             int64_t max_sweeps, int64_t stall, const double* n, const double* s0, const double* c,
                             const double* sg, double* E, blml_start_batch* runner);
+/* the same in lent memory (blml_alloc_fn) */
+int blml_start_batch_create_with(int F, const blml_seg* segs, const blml_plan* plans, int anderson, double tol,
+                                 int64_t max_sweeps, int64_t stall, const double* n, const double* s0, const double* c,
+                                 const double* sg, double* E, blml_alloc_fn alloc, void* ctx, void* stream,
+                                 blml_start_batch* runner);
 int blml_start_batch_run(blml_start_batch runner, void* stream);
 int blml_start_batch_result(blml_start_batch runner, int64_t* sweeps, double* res);
 int blml_start_batch_stats(blml_start_batch runner, int64_t* out4);
