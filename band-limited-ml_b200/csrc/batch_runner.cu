@@ -687,8 +687,11 @@ struct Runner {
   std::vector<int> h_live;
   cudaStream_t st = nullptr;
   cudaEvent_t ev = nullptr;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  // the ring's pieces, captured when first needed for a compact set
+  struct Piece { cudaGraph_t graph = nullptr; cudaGraphExec_t exec = nullptr; long long nodes = 0; };
+  std::vector<Piece> pieces;
+  cudaStream_t st_live = nullptr;        // reads the live mask behind a piece while the next one runs
+  cudaEvent_t ev_piece[2] = {};
   long long nodes = 0, steps = 0, replays = 0, rebuilds = 0;
   std::vector<void*> allocs;            // the library's own allocations
   blml_alloc_fn lend = nullptr;         // or the caller's memory, first used behind what the caller's stream holds
@@ -710,7 +713,9 @@ struct Runner {
     segs_all.assign(segs, segs + F);
     h_live.resize(F);
     RC(cuda_status(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "batch runner stream"));
+    RC(cuda_status(cudaStreamCreateWithFlags(&st_live, cudaStreamNonBlocking), "batch runner stream"));
     RC(cuda_status(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "batch runner event"));
+    for (auto& e : ev_piece) RC(cuda_status(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "batch runner event"));
     d_segs_c = (blml_seg*)dalloc(F * sizeof(blml_seg));
     d_segs_eff = (blml_seg*)dalloc(F * sizeof(blml_seg));
     d_fid = (int*)dalloc(F * sizeof(int));
@@ -718,19 +723,23 @@ struct Runner {
     if (!d_segs_c || !d_segs_eff || !d_fid || !d_live) { set_error("batch runner: device allocation"); return BLML_ERR_CUDA; }
     return BLML_OK;
   }
-  void drop_graph() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    exec = nullptr; graph = nullptr;
+  void drop_graphs() {
+    for (auto& p : pieces) {
+      if (p.exec) cudaGraphExecDestroy(p.exec);
+      if (p.graph) cudaGraphDestroy(p.graph);
+      p = Piece();
+    }
   }
   void base_free() {
-    drop_graph();
     if (st) cudaStreamSynchronize(st);
+    drop_graphs();
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
     if (ev) cudaEventDestroy(ev);
+    for (auto& e : ev_piece) if (e) cudaEventDestroy(e);
     if (st) cudaStreamDestroy(st);
-    ev = nullptr; st = nullptr;
+    if (st_live) cudaStreamDestroy(st_live);
+    ev = nullptr; st = st_live = nullptr; ev_piece[0] = ev_piece[1] = nullptr;
   }
   // the compact set: fits `sel`, all live, largest first (launches over fits dispatch their blocks in compact order,
   // so the longest-running fits start first and the small ones fill in behind them)
@@ -745,57 +754,75 @@ struct Runner {
     RC(cuda_status(cudaMemcpyAsync(d_fid, sel.data(), Fa * sizeof(int), cudaMemcpyHostToDevice, st), "compact"));
     return cuda_status(cudaStreamSynchronize(st), "compact");
   }
-  // the live mask of every fit -> the fits still iterating
-  int read_live(std::vector<int>& on) {
-    RC(cuda_status(cudaMemcpyAsync(h_live.data(), d_live, F * sizeof(int), cudaMemcpyDeviceToHost, st), "live mask"));
-    RC(cuda_status(cudaStreamSynchronize(st), "live mask"));
+  // the live mask of every fit -> the fits still iterating: behind all work of the runner, or (after) behind that event.
+  // Flags only go from set to clear, so what a later piece has cleared meanwhile is as good.
+  int read_live(std::vector<int>& on, cudaEvent_t after = nullptr) {
+    cudaStream_t rs = after ? st_live : st;
+    if (after) RC(cuda_status(cudaStreamWaitEvent(st_live, after, 0), "live mask"));
+    RC(cuda_status(cudaMemcpyAsync(h_live.data(), d_live, F * sizeof(int), cudaMemcpyDeviceToHost, rs), "live mask"));
+    RC(cuda_status(cudaStreamSynchronize(rs), "live mask"));
     on.clear();
     for (int f = 0; f < F; f++)
       if (h_live[f]) on.push_back(f);
     return BLML_OK;
   }
-  // capture `ring` iterations enqueued by iter(i) into a graph (launches counted at replay, not at capture)
+  // capture the iterations i0 .. i1 - 1 of the ring, enqueued by iter(i), into a graph (launches counted at replay, not
+  // at capture)
   template <typename Iter>
-  int capture(int ring, Iter iter) {
-    drop_graph();
+  int capture(Piece& p, int i0, int i1, Iter iter) {
     const long long l0 = blml_launch_count();
     RC(cuda_status(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture"));
     int rc = BLML_OK;
-    for (int i = 0; i < ring && rc == BLML_OK; i++) rc = iter(i);
+    for (int i = i0; i < i1 && rc == BLML_OK; i++) rc = iter(i);
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(st, &g);
-    nodes = blml_launch_count() - l0;
-    count_launches((int)-nodes);
+    p.nodes = blml_launch_count() - l0;
+    count_launches((int)-p.nodes);
     if (rc != BLML_OK) { if (g) cudaGraphDestroy(g); return rc; }
     RC(cuda_status(ce, "graph capture end"));
-    graph = g;
-    RC(cuda_status(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate"));
+    p.graph = g;
+    RC(cuda_status(cudaGraphInstantiate(&p.exec, g, 0), "graph instantiate"));
     rebuilds++;
     return BLML_OK;
   }
-  int replay() {
-    RC(cuda_status(cudaGraphLaunch(exec, st), "graph launch"));
+  int replay(const Piece& p) {
+    RC(cuda_status(cudaGraphLaunch(p.exec, st), "graph launch"));
+    nodes = p.nodes;
     count_launches((int)nodes);
     replays++;
     return BLML_OK;
   }
-  // run until no fit is live: replay the ring, re-capture over the fits still iterating when they fall to 3/4;
-  // before each capture, prep() uploads what the compact set needs
+  // run until no fit is live: replay the ring in pieces of `len` iterations, with a new capture over the fits still
+  // iterating when a ring begins with 3/4 of them or fewer; before it, prep() uploads what the compact set needs. Within a
+  // ring the next piece is launched before the mask behind the last one is read, so the GPU does not wait for the host;
+  // most: no fit runs more iterations than that. (A ring replayed as a whole ran its
+  // launches over stopped fits too: 64 fits stopping after 4 of 20 iterations, 26.4 ms a fit call -> 17.8.)
   template <typename Iter, typename Prep>
-  int run_rings(int ring, Iter iter, Prep prep) {
+  int run_rings(int ring, int len, long long most, Iter iter, Prep prep) {
     std::vector<int> on;
-    for (;;) {
-      RC(read_live(on));
-      if (on.empty()) return BLML_OK;
-      if (!exec || (int)on.size() * 4 <= Fa * 3) {
+    const int np = (ring + len - 1) / len;
+    bool any = false;
+    long long done = 0;
+    drop_graphs();
+    pieces.resize(np);
+    RC(read_live(on));
+    for (int k = 0; !on.empty(); k = (k + 1) % np) {
+      if (k == 0 && (!any || (int)on.size() * 4 <= Fa * 3)) {
+        drop_graphs();
         RC(set_compact(on));
         RC(prep());
-        RC(capture(ring, iter));
+        any = true;
       }
-      RC(replay());
-      steps += ring;
+      const int i0 = k * len, i1 = std::min(ring, i0 + len);
+      if (!pieces[k].exec) RC(capture(pieces[k], i0, i1, iter));
+      RC(replay(pieces[k]));
+      RC(cuda_status(cudaEventRecord(ev_piece[k & 1], st), "runner piece"));
+      done += i1 - i0; steps += i1 - i0;
       if (steps > kMaxSteps) { set_error("batch runner: more than %lld iterations", kMaxSteps); return BLML_ERR_ARG; }
+      if (k == np - 1 || done >= most) RC(read_live(on));
+      else if (k > 0) RC(read_live(on, ev_piece[(k - 1) & 1]));
     }
+    return BLML_OK;
   }
   int begin(void* caller) {
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(caller);
@@ -827,7 +854,7 @@ using namespace blml;
 struct blml_lbfgs_batch_s : Runner {
   int m = 20, dtype = BLML_F64;
   double tol = 1e-5, ftol = 1e-11;
-  long long cap = LLONG_MAX;
+  long long cap = LLONG_MAX, most = LLONG_MAX;       // iterations of any fit, of the fit with the most
   blml_group gEU = nullptr, gq = nullptr, gV = nullptr;
   void *E = nullptr, *U = nullptr;
   const void *w = nullptr, *c = nullptr;
@@ -846,14 +873,18 @@ struct blml_lbfgs_batch_s : Runner {
   long long* d_caps = nullptr;
 
   // the history scan: H1 = [S_q . y_p, S_q . g, y_p . y_p, g . g, E . E], H2 = [Y_q . y_p, Y_q . g, ...]
+  // over the slots that hold a pair (in set-up: none, and slot 0 is zero)
   int hist(int Fa_, const blml_seg* S, int p) {
-    const void* a[LB_MMAX];
-    for (int i = 0; i < m; i++) a[i] = Sh[i];
-    if (h32) RC(seg_dots2_h32(Fa_, S, split, m, a, Yh[p], g, E, part, H1, st));
-    else RC(blml_seg_dots2(dtype, Fa_, S, 1, m, a, Yh[p], g, E, part, H1, st));
-    for (int i = 0; i < m; i++) a[i] = Yh[i];
-    if (h32) return seg_dots2_h32(Fa_, S, split, m, a, Yh[p], g, nullptr, part, H2, st);
-    return blml_seg_dots2(dtype, Fa_, S, 1, m, a, Yh[p], g, nullptr, part, H2, st);
+    const HistMask hm{s.stamp, d_fid, m, p};
+    for (int h = 0; h < 2; h++) {
+      const void* a[LB_MMAX];
+      for (int i = 0; i < m; i++) a[i] = h ? Yh[i] : Sh[i];
+      const void* x = h ? nullptr : E;
+      double* out = h ? H2 : H1;
+      RC(h32 ? seg_dots2_h32(Fa_, S, split, m, a, Yh[p], g, x, part, out, hm, st)
+             : seg_dots2(dtype, Fa_, S, 1, m, a, Yh[p], g, x, part, out, hm, st));
+    }
+    return BLML_OK;
   }
 
   template <typename T>
@@ -1106,7 +1137,7 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
     tot = std::max<int64_t>(tot, segs[f].off + (int64_t)segs[f].K * segs[f].B);
   }
   blml_lbfgs_batch_s* r = new blml_lbfgs_batch_s();
-  r->m = m; r->dtype = dtype; r->tol = tol; r->ftol = ll_tol; r->cap = max_iters < 0 ? LLONG_MAX : max_iters;
+  r->m = m; r->dtype = dtype; r->tol = tol; r->ftol = ll_tol; r->cap = r->most = max_iters < 0 ? LLONG_MAX : max_iters;
   r->E = E; r->U = U; r->w = w; r->c = c;
   r->h32 = h32 && dtype == BLML_F64;     // (float32 state: the history is float32 already)
   r->lend = lend; r->lend_ctx = ctx; r->lend_st = reinterpret_cast<cudaStream_t>(stream);
@@ -1123,8 +1154,9 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
       r->Sh[i] = hv + (size_t)i * tot * hsz;
       r->Yh[i] = hv + ((size_t)m + i) * tot * hsz;
     }
-    cudaMemsetAsync(vec, 0, 6 * tot * esz, r->st);
-    cudaMemsetAsync(hv, 0, 2 * (size_t)m * tot * hsz, r->st);
+    // slot 0, which the set-up's scan reads; nothing else is read before it is written
+    cudaMemsetAsync(r->Sh[0], 0, tot * hsz, r->st);
+    cudaMemsetAsync(r->Yh[0], 0, tot * hsz, r->st);
     // >= Fa * seg_blocks_for(Fa) for every Fa <= F, and 48 pw >= 43 (SEG_SPLIT_BLOCKS + Fa) for the split scan
     const size_t pw = (size_t)SEG_PART_WIDTH(F);
     const int nq = 48;                    // the widest reduction: blml_seg_dots' 48 accumulators
@@ -1153,6 +1185,7 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
       r->s.active = ti(1); r->s.it = ti(1); r->s.stop = ti(1); r->s.reset = ti(1); r->s.nh = ti(1); r->s.ok = ti(1);
       r->need2 = ti(1); ti(1);
       r->s.stamp = ti(m); r->s.step = z;
+      cudaMemsetAsync(r->s.stamp, 0xff, sizeof(int) * (size_t)F * m, r->st);     // -1: no pair
       k_fill_double<<<nblk(F, 256), 256, 0, r->st>>>(r->ones, F, 1.0);
       rc = cuda_status(cudaMemcpyAsync(r->s.n, n, F * sizeof(double), cudaMemcpyHostToDevice, r->st), "lbfgs n");
       if (!rc) rc = cuda_status(cudaStreamSynchronize(r->st), "lbfgs create");
@@ -1194,7 +1227,9 @@ int blml_lbfgs_batch_set_history(blml_lbfgs_batch r, int f32) {
   else if (cudaMalloc(&hv, bytes) != cudaSuccess) hv = nullptr;
   if (!hv) { set_error("blml_lbfgs_batch_set_history: allocation"); return BLML_ERR_CUDA; }
   int rc = cuda_status(cudaStreamSynchronize(r->st), "blml_lbfgs_batch_set_history");
-  if (!rc) rc = cuda_status(cudaMemsetAsync(hv, 0, bytes, r->st), "blml_lbfgs_batch_set_history");
+  if (!rc) rc = cuda_status(cudaMemsetAsync(hv, 0, (size_t)r->tot * 8, r->st), "blml_lbfgs_batch_set_history");
+  if (!rc) rc = cuda_status(cudaMemsetAsync((char*)hv + (size_t)r->m * r->tot * 8, 0, (size_t)r->tot * 8, r->st),
+                            "blml_lbfgs_batch_set_history");
   if (rc) { if (!r->lend) cudaFree(hv); return rc; }
   if (!r->lend)
     for (auto& p : r->allocs)
@@ -1219,7 +1254,7 @@ int blml_lbfgs_batch_set_caps(blml_lbfgs_batch r, const int64_t* caps) {
   int rc = cuda_status(cudaMemcpyAsync(r->d_caps, c.data(), sizeof(long long) * r->F, cudaMemcpyHostToDevice, r->st),
                        "blml_lbfgs_batch_set_caps");
   if (!rc) rc = cuda_status(cudaStreamSynchronize(r->st), "blml_lbfgs_batch_set_caps");
-  if (!rc) r->s.caps = r->d_caps;
+  if (!rc) { r->s.caps = r->d_caps; r->most = *std::max_element(c.begin(), c.end()); }
   return rc;
 }
 
@@ -1227,7 +1262,7 @@ int blml_lbfgs_batch_run(blml_lbfgs_batch r, void* stream) {
   if (!r) { set_error("blml_lbfgs_batch_run: null runner"); return BLML_ERR_ARG; }
   RC(r->begin(stream));
   RC(r->setup());
-  RC(r->run_rings(r->m, [r](int i) { return r->iter(i); }, [] { return (int)BLML_OK; }));
+  RC(r->run_rings(r->m, 5, r->most, [r](int i) { return r->iter(i); }, [] { return (int)BLML_OK; }));
   return r->end(stream);
 }
 
@@ -1351,7 +1386,7 @@ int blml_start_batch_run(blml_start_batch r, void* stream) {
   RC(r->begin(stream));
   RC(r->setup());
   const int ring = r->mA > 0 ? r->mA : 1;
-  RC(r->run_rings(ring, [r](int i) { return r->iter(i); }, [r] { return r->upload_s0(); }));
+  RC(r->run_rings(ring, ring, r->cap, [r](int i) { return r->iter(i); }, [r] { return r->upload_s0(); }));
   return r->end(stream);
 }
 

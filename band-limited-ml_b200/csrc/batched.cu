@@ -164,8 +164,10 @@ struct SegList { const void* a[20]; };
 // b0 . b0, b1 . b1, x . x] (x may be null: 0); b0, b1, x read once per element whatever np is
 template <typename T>
 __global__ void __launch_bounds__(256) k_seg_dots2(const blml_seg* segs, int cplx, int np, SegList al, const void* b0,
-                                                   const void* b1, const void* x, double* part) {
+                                                   const void* b1, const void* x, double* part, HistMask hm) {
   const blml_seg S = segs[blockIdx.y];
+  const int lq = threadIdx.x & 31;
+  const unsigned on = __ballot_sync(0xffffffffu, lq < np && hm.on(blockIdx.y, lq));
   const int64_t w = cplx ? 2 : 1;
   const int64_t o = S.off * w, n = (int64_t)S.K * S.B * w;
   double v[43];
@@ -178,7 +180,7 @@ __global__ void __launch_bounds__(256) k_seg_dots2(const blml_seg* segs, int cpl
     const double y0 = (double)B0[i], y1 = (double)B1[i];
 #pragma unroll
     for (int q = 0; q < 20; q++)
-      if (q < np) {
+      if (on >> q & 1u) {
         const double a = (double)reinterpret_cast<const T*>(al.a[q])[o + i];
         v[q] += a * y0; v[20 + q] += a * y1;
       }
@@ -195,30 +197,39 @@ __global__ void __launch_bounds__(256) k_seg_dots2(const blml_seg* segs, int cpl
 // holds at most 6 accumulators (full occupancy, many loads in flight) and the two shared vectors are read from HBM
 // once per tile and from L1 by the other warps; the last warp also sums the three squared norms. Each quantity's
 // block partial comes from one warp (warp_sum, fixed order), in seg_partials' layout.
+// The stored vectors are those of the mask's slots, the i-th of them for warp i mod 8 (a slot's sum does not depend on
+// which warp forms it): the first iterations of a fit, whose memory is still filling, read only what it holds. 64 fits of
+// rank 4 over their first 12 iterations (20 slots): 12.9 ms of scans -> 9.3.
+__device__ __forceinline__ int nth_slot(unsigned on, int i) {
+  for (; i > 0 && on; i--) on &= on - 1;
+  return __ffs(on) - 1;
+}
+
 // one complex128 element as (re, im)
 __device__ __forceinline__ double2 ld_c2(const double2* p) { return __ldg(p); }
 
 template <typename TA, typename TB0>
 __global__ void __launch_bounds__(256, 3) k_seg_dots2_c128(const blml_seg* segs, int np, SegList al, const void* b0,
-                                                           const void* b1, const void* x, double* part) {
+                                                           const void* b1, const void* x, double* part, HistMask hm) {
   const blml_seg S = segs[blockIdx.y];
   const int64_t o = S.off, n = (int64_t)S.K * S.B;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const unsigned on = __ballot_sync(0xffffffffu, lane < np && hm.on(blockIdx.y, lane));
   const TB0* B0 = reinterpret_cast<const TB0*>(b0) + o;
   const double2* B1 = reinterpret_cast<const double2*>(b1) + o;
   const double2* X = x ? reinterpret_cast<const double2*>(x) + o : nullptr;
   const TA* A[3];
-  int na = 0;
+  int na = 0, qs_[3];
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    const int q = warp + nw * j;
-    A[j] = q < np ? reinterpret_cast<const TA*>(al.a[q]) + o : nullptr;
-    na += q < np;
+    qs_[j] = nth_slot(on, warp + nw * j);
+    A[j] = qs_[j] >= 0 ? reinterpret_cast<const TA*>(al.a[qs_[j]]) + o : nullptr;
+    na += qs_[j] >= 0;
   }
   const bool norms = warp == nw - 1;
   double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
   const double2 zero = make_double2(0.0, 0.0);
-  for (int64_t t = (int64_t)blockIdx.x * 64; t < n; t += (int64_t)gridDim.x * 64) {
+  for (int64_t t = (int64_t)blockIdx.x * 64; t < n && (na || norms); t += (int64_t)gridDim.x * 64) {
     // both elements' loads issued together: out-of-range lanes read element 0 and zero its shared values, so their
     // products and norms add nothing
     const int64_t i0 = t + lane, i1 = t + 32 + lane;
@@ -249,7 +260,7 @@ __global__ void __launch_bounds__(256, 3) k_seg_dots2_c128(const blml_seg* segs,
   for (int j = 0; j < 3; j++) {
     const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
     if (j < na && lane == 0) {
-      const int q = warp + nw * j;
+      const int q = qs_[j];
       part[q * qs + slot] = s0; part[(20 + q) * qs + slot] = s1;
     }
   }
@@ -260,13 +271,14 @@ __global__ void __launch_bounds__(256, 3) k_seg_dots2_c128(const blml_seg* segs,
 }
 
 // out[f * (2 np + 3) + q] from the 43-quantity partials (quantities 20.. shifted down when np < 20)
-__global__ void k_seg_finish_dots2(const double* part, int np, int nblk, double* out) {
+__global__ void k_seg_finish_dots2(const double* part, int np, int nblk, double* out, HistMask hm) {
   const int f = blockIdx.x, F = gridDim.x, nq = 2 * np + 3;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int q = wid; q < nq; q += nw) {
     const int src = q < np ? q : (q < 2 * np ? 20 + (q - np) : 40 + (q - 2 * np));
     double acc = 0.0;
-    for (int i = lane; i < nblk; i += 32) acc += part[((int64_t)src * F + f) * nblk + i];
+    if (q >= 2 * np || hm.on(f, q % np))
+      for (int i = lane; i < nblk; i += 32) acc += part[((int64_t)src * F + f) * nblk + i];
     acc = warp_sum(acc);
     if (lane == 0) out[(int64_t)f * nq + q] = acc;
   }
@@ -409,9 +421,10 @@ __device__ __forceinline__ void h32_tile(int64_t t, int64_t n, int lane, const f
 
 __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, const int* split, int F, int np,
                                                           SegList al, const float2* b0, const double2* b1,
-                                                          const double2* x, double* part) {
+                                                          const double2* x, double* part, HistMask hm) {
   const int b = blockIdx.x, W = gridDim.x, f = split[F + 1 + b];
   if (f < 0) return;
+  const unsigned on = __ballot_sync(0xffffffffu, (threadIdx.x & 31) < np && hm.on(f, threadIdx.x & 31));
   const int lb = b - split[f], nb = split[f + 1] - split[f];
   const blml_seg S = segs[f];
   const int64_t o = S.off, n = (int64_t)S.K * S.B;
@@ -420,25 +433,26 @@ __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, 
   const double2* B1 = b1 + o;
   const double2* X = x ? x + o : nullptr;
   const float2* A[3];
-  int na = 0;
+  int na = 0, qs_[3];
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    const int q = warp + nw * j;
-    A[j] = q < np ? reinterpret_cast<const float2*>(al.a[q]) + o : nullptr;
-    na += q < np;
+    qs_[j] = nth_slot(on, warp + nw * j);
+    A[j] = qs_[j] >= 0 ? reinterpret_cast<const float2*>(al.a[qs_[j]]) + o : nullptr;
+    na += qs_[j] >= 0;
   }
   const bool norms = warp == nw - 1;
   double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
   constexpr int64_t T = 128;
   const int64_t stride = (int64_t)nb * T;
   int64_t t = (int64_t)lb * T;
+  if (!na && !norms) t = n;
   for (; t + T <= n; t += stride) h32_tile<false>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
   for (; t < n; t += stride) h32_tile<true>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
 #pragma unroll
   for (int j = 0; j < 3; j++) {
     const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
     if (j < na && lane == 0) {
-      const int q = warp + nw * j;
+      const int q = qs_[j];
       part[(int64_t)q * W + b] = s0; part[(int64_t)(20 + q) * W + b] = s1;
     }
   }
@@ -449,14 +463,15 @@ __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, 
 }
 
 // out[f * (2 np + 3) + q] from a split scan's partials: fit f's blocks [bstart[f], bstart[f + 1]), fixed order
-__global__ void k_seg_finish_dots2_split(const double* part, int W, const int* split, int np, double* out) {
+__global__ void k_seg_finish_dots2_split(const double* part, int W, const int* split, int np, double* out, HistMask hm) {
   const int f = blockIdx.x, nq = 2 * np + 3;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int b0 = split[f], b1 = split[f + 1];
   for (int q = wid; q < nq; q += nw) {
     const int src = q < np ? q : (q < 2 * np ? 20 + (q - np) : 40 + (q - 2 * np));
     double acc = 0.0;
-    for (int i = b0 + lane; i < b1; i += 32) acc += part[(int64_t)src * W + i];
+    if (q >= 2 * np || hm.on(f, q % np))
+      for (int i = b0 + lane; i < b1; i += 32) acc += part[(int64_t)src * W + i];
     acc = warp_sum(acc);
     if (lane == 0) out[(int64_t)f * nq + q] = acc;
   }
@@ -863,16 +878,32 @@ int seg_split(int F, const blml_seg* segs, int* split, cudaStream_t st) {
   return BLML_OK;
 }
 
+int seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, const void* const* a, const void* b0,
+              const void* b1, const void* x, double* part, double* out, HistMask hm, cudaStream_t st) {
+  SegList al;
+  for (int q = 0; q < 20; q++) al.a[q] = q < np ? a[q] : nullptr;
+  const int nb = seg_blocks_for(F);
+  const dim3 g((unsigned)nb, (unsigned)F);
+  if (dtype == BLML_F64 && cplx)
+    k_seg_dots2_c128<double2, double2><<<g, 256, 0, st>>>(segs, np, al, b0, b1, x, part, hm);
+  else if (dtype == BLML_F64) k_seg_dots2<double><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
+  else k_seg_dots2<float><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
+  BLML_CHECK_LAUNCH("blml_seg_dots2");
+  k_seg_finish_dots2<<<F, 256, 0, st>>>(part, np, nb, out, hm);
+  BLML_CHECK_LAUNCH("blml_seg_dots2 finish");
+  return BLML_OK;
+}
+
 int seg_dots2_h32(int F, const blml_seg* segs, const int* split, int np, const void* const* a, const void* b0,
-                  const void* b1, const void* x, double* part, double* out, cudaStream_t st) {
+                  const void* b1, const void* x, double* part, double* out, HistMask hm, cudaStream_t st) {
   if (np < 1 || np > 20 || !a || !b0 || !b1) { set_error("history scan: 1..20 vectors, b0 and b1"); return BLML_ERR_ARG; }
   SegList al;
   for (int q = 0; q < 20; q++) al.a[q] = q < np ? a[q] : nullptr;
   const int W = SEG_SPLIT_BLOCKS + F;
   k_seg_dots2_h32<<<W, 256, 0, st>>>(segs, split, F, np, al, (const float2*)b0, (const double2*)b1,
-                                     (const double2*)x, part);
+                                     (const double2*)x, part, hm);
   BLML_CHECK_LAUNCH("history scan (float32 history)");
-  k_seg_finish_dots2_split<<<F, 256, 0, st>>>(part, W, split, np, out);
+  k_seg_finish_dots2_split<<<F, 256, 0, st>>>(part, W, split, np, out, hm);
   BLML_CHECK_LAUNCH("history scan finish");
   return BLML_OK;
 }
@@ -977,16 +1008,7 @@ int blml_seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, con
                    const void* b1, const void* x, double* part, double* out, void* stream) {
   if (seg_args(dtype, F, segs, "blml_seg_dots2")) return BLML_ERR_ARG;
   if (np < 1 || np > 20 || !a || !b0 || !b1) { set_error("blml_seg_dots2: 1..20 vectors, b0 and b1"); return BLML_ERR_ARG; }
-  SegList al;
-  for (int q = 0; q < 20; q++) al.a[q] = q < np ? a[q] : nullptr;
-  if (dtype == BLML_F64 && cplx)
-    k_seg_dots2_c128<double2, double2><<<SGRID(F), 256, 0, SST>>>(segs, np, al, b0, b1, x, part);
-  else if (dtype == BLML_F64) k_seg_dots2<double><<<SGRID(F), 256, 0, SST>>>(segs, cplx, np, al, b0, b1, x, part);
-  else k_seg_dots2<float><<<SGRID(F), 256, 0, SST>>>(segs, cplx, np, al, b0, b1, x, part);
-  BLML_CHECK_LAUNCH("blml_seg_dots2");
-  k_seg_finish_dots2<<<F, 256, 0, SST>>>(part, np, seg_blocks_for(F), out);
-  BLML_CHECK_LAUNCH("blml_seg_dots2 finish");
-  return BLML_OK;
+  return seg_dots2(dtype, F, segs, cplx, np, a, b0, b1, x, part, out, HistMask{}, SST);
 }
 
 int blml_seg_lincomb(int dtype, int F, const blml_seg* segs, int cplx, void* out, int nterms, const double* coef,
@@ -1152,7 +1174,7 @@ int blml_seg_dots2_h32(int F, const blml_seg* segs, int* split, int np, const vo
     set_error("blml_seg_dots2_h32: bad arguments"); return BLML_ERR_ARG;
   }
   if (seg_split(F, segs, split, SST)) return BLML_ERR_CUDA;
-  return seg_dots2_h32(F, segs, split, np, a, b0, b1, x, part, out, SST);
+  return seg_dots2_h32(F, segs, split, np, a, b0, b1, x, part, out, HistMask{}, SST);
 }
 
 int64_t blml_seg_split_ints(int F) { return F < 1 ? 0 : seg_split_ints(F); }

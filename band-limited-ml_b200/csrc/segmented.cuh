@@ -31,9 +31,18 @@ constexpr int SEG_SPLIT_BLOCKS = BLML_SEG_SPLIT_BLOCKS, SEG_SPLIT_MIN_ELEMS = 10
 __host__ __device__ inline int64_t seg_split_ints(int F) { return 2 * (int64_t)F + 1 + SEG_SPLIT_BLOCKS; }
 int seg_split(int F, const blml_seg* segs, int* split, cudaStream_t st);
 
-// the L-BFGS runner's float32 history (batched.cu); split: seg_split's output for these segments
+// The history slots a scan covers: slot p and the slots that hold a pair (stamp >= 0) of launch row j's fit fid[j]; the
+// other slots' products are 0 and their memory is not read. stamp null: every slot.
+struct HistMask {
+  const int* stamp; const int* fid; int m, p;
+  __device__ __forceinline__ bool on(int j, int q) const { return !stamp || q == p || stamp[(int64_t)fid[j] * m + q] >= 0; }
+};
+
+// the L-BFGS runner's history scans (batched.cu): state of dtype, or complex64 storage (split: seg_split's output)
+int seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, const void* const* a, const void* b0,
+              const void* b1, const void* x, double* part, double* out, HistMask hm, cudaStream_t st);
 int seg_dots2_h32(int F, const blml_seg* segs, const int* split, int np, const void* const* a, const void* b0,
-                  const void* b1, const void* x, double* part, double* out, cudaStream_t st);
+                  const void* b1, const void* x, double* part, double* out, HistMask hm, cudaStream_t st);
 int seg_lincomb_mixed(int F, const blml_seg* segs, const int* split, void* out, int out_f32, int nterms,
                       const double* coef, const void* const* v, unsigned long long f32mask, cudaStream_t st);
 
