@@ -100,14 +100,25 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
     tmp = torch.empty(B, dtype=torch.float64, device=dev)
     sv = torch.empty(B, dtype=torch.float64, device=dev)
 
+    # bins per block of a step: at least 512, at most 256 blocks a fit
+    chunk = max(512, -(-int(batch.B.max()) // (256 * 256)) * 256)
+
     class Subset:
-        """The fits a launch covers: their segment list (offsets into the full vectors) and grouped mat-vec."""
+        """The fits a launch covers: their segment list (offsets into the full vectors), grouped mat-vec and blocks."""
 
         def __init__(self, idx):
             self.idx = np.asarray(idx, np.int64)
             segs = (_Seg * len(self.idx))(*[_Seg(int(batch.boff[f]), int(batch.boff[f]), int(batch.B[f]), 1, 0)
                                             for f in self.idx])
-            self.segs_t = torch.frombuffer(bytearray(segs), dtype=torch.uint8).to(dev)
+            nc = -(-np.asarray(batch.B)[self.idx] // chunk)
+            row = np.repeat(np.arange(len(self.idx)), nc)
+            tab = np.stack([row, np.arange(len(row)) - np.repeat(np.cumsum(nc) - nc, nc)], 1).astype(np.int32)
+            self.nblocks = len(tab)
+            ints = np.concatenate([np.frombuffer(bytes(segs), np.int32), self.idx.astype(np.int32),
+                                   np.zeros(len(self.idx), np.int32)])      # 10 ints a row: tab stays 8-byte aligned
+            self.segs_t = torch.from_numpy(np.concatenate([ints, tab.ravel()])).to(dev)
+            at = self.segs_t.data_ptr()
+            self.fid, self.cnt, self.tab = at + len(bytes(segs)), at + len(bytes(segs)) + 4 * len(self.idx), at + 4 * len(ints)
             off = np.asarray(batch.boff[:-1])[self.idx]
             self.grp = _Group([batch.p64[f] for f in self.idx], tmp, off, sv, off, False)
 
@@ -142,11 +153,6 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
         call('blml_seg_lincomb', code, len(S.idx), S.segs_t.data_ptr(), 0, out.data_ptr(), len(vecs),
              ring_d[k].data_ptr(), ptrs(vecs), st)
 
-    def op(S, x, out):                               # out = dh * S (dh * x) on S's fits
-        call('blml_mul_bins', code, 1, B, 0, x.data_ptr(), dh.data_ptr(), tmp.data_ptr(), st)
-        S.grp(st)
-        call('blml_mul_bins', code, 1, B, 0, sv.data_ptr(), dh.data_ptr(), out.data_ptr(), st)
-
     every = Subset(np.arange(F))
     nb = max_basis
     V = torch.empty((nb + 1, B), dtype=torch.float64, device=dev)
@@ -160,20 +166,19 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
     vec2 = torch.zeros(B, dtype=torch.float64, device=dev) if (vectors and second) else None
     R2 = torch.empty(B, dtype=torch.float64, device=dev) if vec2 is not None else None
     R = torch.empty(B, dtype=torch.float64, device=dev)
-    # the steps themselves make no host round trip: the reorthogonalisation's coefficients and alpha / beta come from
-    # the inner products on the device (blml_lanczos_coef / _beta); the host reads alpha and beta at the checks
-    coef_d = torch.empty(F * 48 + 64, dtype=torch.float64, device=dev)
-    bcoef_d = torch.empty(F + 64, dtype=torch.float64, device=dev)
-    alpha_d = torch.zeros((nb, F), dtype=torch.float64, device=dev)
-    beta_d = torch.zeros((nb, F), dtype=torch.float64, device=dev)
+    # the steps themselves make no host round trip (blml_lanczos_step); the host reads alpha and beta at the checks, while
+    # the next step already runs
+    coef_d = torch.empty(64 * F, dtype=torch.float64, device=dev)
+    scale_d = torch.empty(F, dtype=torch.float64, device=dev)
+    ab_d = torch.zeros((nb, 2, F), dtype=torch.float64, device=dev)
+    ab_h = torch.empty((nb, 2, F), dtype=torch.float64, pin_memory=True)
+    part = torch.empty(64 * every.nblocks, dtype=torch.float64, device=dev)
+    read = torch.cuda.Event()
 
-    def dots_dev(S, pairs):                          # inner products into batch.out (rows of S), no read
-        call('blml_seg_dots', code, len(S.idx), S.segs_t.data_ptr(), 0, len(pairs), ptrs([p[0] for p in pairs]),
-             ptrs([p[1] for p in pairs]), batch.part.data_ptr(), batch.out.data_ptr(), st)
-
-    def lin_dev(S, out, cptr, vecs):
-        call('blml_seg_lincomb', code, len(S.idx), S.segs_t.data_ptr(), 0, out.data_ptr(), len(vecs), cptr,
-             ptrs(vecs), st)
+    def step(S, j):
+        call('blml_lanczos_step', len(S.idx), S.segs_t.data_ptr(), S.fid, S.nblocks, S.tab, chunk, S.grp.on(st), V.data_ptr(),
+             B, j, dh.data_ptr(), tmp.data_ptr(), sv.data_ptr(), wv.data_ptr(), part.data_ptr(), S.cnt, coef_d.data_ptr(),
+             ab_d[j, 0].data_ptr(), ab_d[j, 1].data_ptr(), scale_d.data_ptr(), st)
 
     steps = 0
     for rnd in range(max_restarts + 1):
@@ -181,63 +186,61 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
         conv = np.zeros(F, bool); yr = [None] * F; yr2 = [None] * F
         S = every if not done.any() else Subset(np.where(~done)[0])
         j_end = nb
-        fetched = 0                                   # steps whose alpha / beta the host holds
+        fetched = 0                                   # steps whose alpha / beta the host holds or has asked for
+        waiting = None                                # the step whose check is still to be made
+
+        def check(j):
+            """Every open fit's tridiagonal problem after step j; True when all have converged."""
+            t0 = time.perf_counter()
+            read.synchronize()
+            clock['wait_s'] += time.perf_counter() - t0
+            t0 = time.perf_counter()
+            ab = ab_h.numpy()
+            of = np.where(~(done | conv))[0]
+            alphas[of, :j + 1] = ab[:j + 1, 0, of].T
+            betas[of, :j + 1] = ab[:j + 1, 1, of].T
+            beta = betas[:, j]
+            # the largest eigenpair of each T_f (j + 1 square), all at once
+            T = np.zeros((len(of), j + 1, j + 1))
+            ii = np.arange(j + 1)
+            T[:, ii, ii] = alphas[of, :j + 1]
+            T[:, ii[:-1], ii[1:]] = betas[of, :j]
+            T[:, ii[1:], ii[:-1]] = betas[of, :j]
+            ev_all, evec_all = np.linalg.eigh(T)
+            for t_, f in enumerate(of):
+                th = float(ev_all[t_, -1]); y = evec_all[t_, :, -1].copy()
+                theta[f] = th; yr[f] = y
+                if j > 0:
+                    yr2[f] = evec_all[t_, :, -2].copy(); theta2[f] = float(ev_all[t_, -2])
+                if (abs(beta[f] * y[-1]) <= tol * max(abs(th), 1e-300) or beta[f] <= 1e-14 * max(abs(th), 1e-300)
+                        or th > above[f] or abs(th - prev[f]) <= 1e-8 * abs(th)):
+                    conv[f] = True
+                prev[f] = th
+            clock['host_s'] += time.perf_counter() - t0
+            return bool(np.all(done | conv))
+
         for j in range(nb):
-            op(S, V[j], wv)
+            step(S, j)
             steps += 1
-            n = len(S.idx)
-            for ps in range(2):                       # full reorthogonalisation against the basis, twice
-                for c0 in range(0, j + 1, 47):
-                    idx = list(range(c0, min(j + 1, c0 + 47)))
-                    dots_dev(S, [(V[i], wv) for i in idx])
-                    acol = j - c0 if (ps == 0 and c0 <= j < c0 + 47) else -1
-                    call('blml_lanczos_coef', n, len(idx), batch.out.data_ptr(), coef_d.data_ptr(),
-                         alpha_d[j].data_ptr() if acol >= 0 else None, acol, st)
-                    lin_dev(S, wv, coef_d.data_ptr(), [wv] + [V[i] for i in idx])
-            dots_dev(S, [(wv, wv)])
-            call('blml_lanczos_beta', n, batch.out.data_ptr(), beta_d[j].data_ptr(), bcoef_d.data_ptr(), st)
-            open_ = np.zeros(F, bool); open_[S.idx] = True
-            open_ &= ~(done | conv)
-            check = j == nb - 1 or (j >= 5 and j % 3 == 2)
-            if check:
-                t0 = time.perf_counter()
-                a_h = alpha_d[fetched:j + 1, :n].cpu().numpy()
-                b_h = beta_d[fetched:j + 1, :n].cpu().numpy()
-                clock['wait_s'] += time.perf_counter() - t0
-                alphas[S.idx, fetched:j + 1] = a_h.T
-                betas[S.idx, fetched:j + 1] = b_h.T
-                fetched = j + 1
-                beta = betas[:, j]
-                t0 = time.perf_counter()
-                of = np.where(open_)[0]
-                # every open fit's tridiagonal problem at once: the largest eigenpair of T_f (j + 1 square)
-                T = np.zeros((len(of), j + 1, j + 1))
-                ii = np.arange(j + 1)
-                T[:, ii, ii] = alphas[of, :j + 1]
-                T[:, ii[:-1], ii[1:]] = betas[of, :j]
-                T[:, ii[1:], ii[:-1]] = betas[of, :j]
-                ev_all, evec_all = np.linalg.eigh(T)
-                for t_, f in enumerate(of):
-                    th = float(ev_all[t_, -1]); y = evec_all[t_, :, -1].copy()
-                    theta[f] = th; yr[f] = y
-                    if j > 0:
-                        yr2[f] = evec_all[t_, :, -2].copy(); theta2[f] = float(ev_all[t_, -2])
-                    if (abs(beta[f] * y[-1]) <= tol * max(abs(th), 1e-300) or beta[f] <= 1e-14 * max(abs(th), 1e-300)
-                            or th > above[f] or abs(th - prev[f]) <= 1e-8 * abs(th)):
-                        conv[f] = True
-                    prev[f] = th
-                clock['host_s'] += time.perf_counter() - t0
-                if np.all(done | conv):
-                    j_end = j + 1
+            if waiting is not None:
+                pj, waiting = waiting, None
+                if check(pj):                         # (this step was one too many: its vectors go unused)
+                    j_end = pj + 1
                     break
-            lin_dev(S, V[j + 1], bcoef_d.data_ptr(), [wv])
-            still = np.where(~(done | conv))[0]
-            if check and j + 1 < nb and len(still) <= 0.75 * len(S.idx):
-                # the steps go on over the open fits only; the converged ones keep V[0..j], all their Ritz vectors use
-                S = Subset(still)
+                still = np.where(~(done | conv))[0]
+                if j + 1 < nb and len(still) <= 0.75 * len(S.idx):
+                    # the steps go on over the open fits only; the converged ones keep V[0..pj], all their Ritz vectors use
+                    S = Subset(still)
+            if j == nb - 1 or (j >= 5 and j % 3 == 2):
+                ab_h[fetched:j + 1].copy_(ab_d[fetched:j + 1], non_blocking=True)
+                read.record(torch.cuda.current_stream(dev))
+                fetched = j + 1
+                waiting = j
+                if j == nb - 1:
+                    check(j)
         # the Ritz vector of every fit still open at the start of this round: R = sum_i y_i V[i]
         act = ~done
-        SA = Subset(np.where(act)[0])
+        SA = every if act.all() else Subset(np.where(act)[0])
         R.zero_()
         for c0 in range(0, j_end, 47):
             idx = list(range(c0, min(j_end, c0 + 47)))

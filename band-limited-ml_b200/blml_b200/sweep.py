@@ -66,13 +66,17 @@ class _Group:
              self._st, C.byref(h))
         self._h = h; self._keep = (plans, x, y)
 
-    def __call__(self, stream):
+    def on(self, stream):
+        """The handle, its lent memory ready for a launch on `stream`."""
         if (stream or 0) != self._st:                       # lent memory on another stream than its own
             other = torch.cuda.ExternalStream(stream or 0, device=self._keep[1].device)
             other.wait_stream(torch.cuda.ExternalStream(self._st, device=other.device))
             for t in self._mem.tensors:
                 t.record_stream(other)
-        call('blml_group_matvec', self._h, stream)
+        return self._h
+
+    def __call__(self, stream):
+        call('blml_group_matvec', self.on(stream), stream)
 
     @property
     def route(self):

@@ -303,6 +303,15 @@ int blml_seg_append_mode(int dtype, int F, const blml_seg* old_segs, const blml_
    1 / beta (0 when beta is 0) for the next basis vector. */
 int blml_lanczos_coef(int n, int np, const double* dots, double* coef, double* alpha, int alpha_col, void* stream);
 int blml_lanczos_beta(int n, const double* dots, double* beta, double* coef, void* stream);
+/* One whole step over the F fits of a launch (float64, real): x = V[j] (j > 0: V[j] = scale w first), w = dh S (dh x) by
+ * `group` (from tmp to sv), w orthogonalised twice against V[0 .. j] (rows ldv apart), alpha = V[j] . w of the first
+ * pass, beta = |w|, scale = 1 / beta (0 for 0). segs (boff, B): the launch's fits; fid[r]: the fit of row r, which alpha,
+ * beta, scale and coef are indexed by. Blocks: tab holds (row, chunk) per block, each row's ceil(B / chunk) chunks in
+ * order; part: 64 nblocks doubles, coef: 64 per fit, counters: F ints, zero at the first call. */
+int blml_lanczos_step(int F, const blml_seg* segs, const int* fid, int nblocks, const int* tab, int chunk,
+                      blml_group group, double* V, int64_t ldv, int j, const double* dh, double* tmp, const double* sv,
+                      double* w, double* part, int* counters, double* coef, double* alpha, double* beta, double* scale,
+                      void* stream);
 
 /* ---- batched solver phases with device-side control: the per-fit decisions of every
  *      iteration run as kernels, a ring of iterations is one CUDA graph replayed until every fit has stopped, the
