@@ -59,6 +59,9 @@ _SIGS = {
     'blml_plan_status': (_I, [_P]),
     'blml_matvec_workspace': (_L, [_P, _I]),
     'blml_matvec': (_I, [_P, _P, _P, _I, _I, _P, _L, _P]),
+    'blml_matvecs_workspace': (_L, [_I, _P, _P]),
+    'blml_matvecs': (_I, [_I, _P, _P, _P, _P, _I, _P, _L, _P]),
+    'blml_stream_wait': (_I, [_P]),
     'blml_group_create_with': (_I, [_I, _P, _P, _I, _P, _P, _P, _P, ALLOC_FN, _P, _P, C.POINTER(_P)]),
     'blml_group_create': (_I, [_I, _P, _P, _I, _P, _P, _P, _P, C.POINTER(_P)]),
     'blml_group_matvec': (_I, [_P, _P]),
@@ -217,6 +220,13 @@ def check(rc, what):
 
 def call(name, *args):
     check(getattr(lib(), name)(*args), name)
+
+
+def current_stream(device):
+    """The handle of torch's current stream on a CUDA device (no Stream object: it is asked for before every launch)."""
+    import torch
+    i = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
 
 class Lender:

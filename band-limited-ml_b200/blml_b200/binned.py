@@ -11,6 +11,8 @@ the history instead of 2m sequential dots); line-search trials update U = S E li
 is formed only at the accepted point; bin-wise arithmetic is float64 internally for both storage types. Arrays
 (density_, e_hat_, Se_) are NumPy on the host, read back from the device on first access; the device copies are
 density_t_, e_hat_t_, Se_t_ (torch)."""
+import ctypes
+
 import numpy as np
 import torch
 
@@ -18,6 +20,7 @@ from . import _lib
 from ._lib import call, ptrs, dbl
 from .spec import parse_modes, spec_key, units_of
 from .operator import pad_rule, mode_transform, mode_transform_dlog, kernel_at_zero, Plan
+from .noise import seeded_normals
 
 
 from collections import OrderedDict
@@ -33,18 +36,33 @@ def _device(dev):
 
 
 class _Red:
-    """Reduction workspace (block partials) and the device results of one fit."""
+    """Reduction workspace (block partials) and the results of one fit's reductions, in pinned host memory that the
+    finishing kernels write to: a read is a wait for the stream, with no copy. Several reductions at places of their own
+    share one wait."""
+    SIZE = 256
 
     def __init__(self, device):
         nb = _lib.lib().blml_reduce_blocks()
+        self.device = device
         self.part = torch.empty(64 * nb, dtype=torch.float64, device=device)
-        self.out = torch.empty(64, dtype=torch.float64, device=device)
-        self.host = torch.empty(64, dtype=torch.float64, pin_memory=True)
+        self.out = torch.empty(self.SIZE, dtype=torch.float64, pin_memory=True)
+        self._np = self.out.numpy()
+        self._at = self.out.data_ptr()
+
+    def at(self, i):
+        """The address of result i."""
+        return self._at + 8 * i
+
+    def wait(self):
+        call('blml_stream_wait', _lib.current_stream(self.device))
+
+    def got(self, i, n):
+        """Results i .. i + n - 1, after a wait."""
+        return self._np[i:i + n].tolist()
 
     def read(self, nq):
-        self.host[:nq].copy_(self.out[:nq], non_blocking=True)
-        torch.cuda.current_stream(self.out.device).synchronize()
-        return self.host[:nq].tolist()
+        self.wait()
+        return self.got(0, nq)
 
 
 def point_cols(sp, d):
@@ -169,31 +187,41 @@ class BLMLBinned:
     # ---------------------------------------------------------------- device helpers
     @property
     def _st(self):
-        return torch.cuda.current_stream(self.dev_).cuda_stream
+        return _lib.current_stream(self.dev_)
 
     def _Sall(self, E, out=None):
         """S_k E_k for every mode (modes sharing a plan in one batched call)."""
         out = torch.empty_like(E) if out is None else out
-        K = E.shape[0]; k = 0
+        K = E.shape[0]; runs = []; k = 0
         while k < K:
             j = k + 1
             while j < K and self.kern_[j][0] is self.kern_[k][0]:
                 j += 1
-            self.kern_[k][0].apply(E[k:j], out[k:j], j - k, E.is_complex(), self._st)
+            runs.append((self.kern_[k][0], j - k))
             k = j
+        if len(runs) == 1:
+            runs[0][0].apply(E, out, K, E.is_complex(), self._st)
+            return out
+        plans = (ctypes.c_void_p * len(runs))(*[p._h.value for p, _ in runs])
+        nb = (ctypes.c_int * len(runs))(*[n for _, n in runs])
+        need = int(_lib.lib().blml_matvecs_workspace(len(runs), plans, nb))
+        ws = torch.empty(max(need, 1), dtype=torch.uint8, device=E.device)
+        call('blml_matvecs', len(runs), plans, nb, E.data_ptr(), out.data_ptr(), int(E.is_complex()), ws.data_ptr(), need,
+             self._st)
         return out
 
     def _nreal(self, x):
         return x.numel() * (2 if x.is_complex() else 1)
 
+    def _q_dots(self, pairs, at):
+        """Re <a, b> for a list of (a, b) tensor pairs, float64, one pass; results from place `at` after a wait."""
+        if pairs:
+            call('blml_dots', self._code, self._nreal(pairs[0][0]), len(pairs), ptrs([p[0] for p in pairs]),
+                 ptrs([p[1] for p in pairs]), self._red.part.data_ptr(), self._red.at(at), self._st)
+
     def _dots(self, pairs):
-        """Re <a, b> for a list of (a, b) tensor pairs, float64, one pass."""
-        if not pairs:
-            return []
-        n = self._nreal(pairs[0][0])
-        call('blml_dots', self._code, n, len(pairs), ptrs([p[0] for p in pairs]), ptrs([p[1] for p in pairs]),
-             self._red.part.data_ptr(), self._red.out.data_ptr(), self._st)
-        return self._red.read(len(pairs))
+        self._q_dots(pairs, 0)
+        return self._red.read(len(pairs)) if pairs else []
 
     def _lin(self, terms, out=None):
         """out = sum c_i v_i over (c_i, v_i) terms."""
@@ -208,12 +236,13 @@ class BLMLBinned:
         return x
 
     # ---------------------------------------------------------------- merit, update, residual
-    def _merit(self, E, U):
-        """Larger is better. psd: scale-free log-likelihood / n; real rank 1: -Phi / n (blml_binned.py:171-182)."""
+    def _q_merit(self, E, U, at):
         call('blml_merit_terms', self._code, E.shape[0], self.B_, int(E.is_complex()), int(self.psd_), E.data_ptr(),
-             U.data_ptr(), self.c_t_.data_ptr(), self.sg_t_.data_ptr(), self._red.part.data_ptr(),
-             self._red.out.data_ptr(), self._st)
-        a, b, bad = self._red.read(3)
+             U.data_ptr(), self.c_t_.data_ptr(), self.sg_t_.data_ptr(), self._red.part.data_ptr(), self._red.at(at),
+             self._st)
+
+    def _got_merit(self, at):
+        a, b, bad = self._red.got(at, 3)
         n = self.n_
         if self.psd_:
             if not b > 0:
@@ -222,6 +251,12 @@ class BLMLBinned:
         if bad > 0:
             return -np.inf
         return -(0.5 * a - b) / n
+
+    def _merit(self, E, U):
+        """Larger is better. psd: scale-free log-likelihood / n; real rank 1: -Phi / n (blml_binned.py:171-182)."""
+        self._q_merit(E, U, 0)
+        self._red.wait()
+        return self._got_merit(0)
 
     def _update(self, E, U):
         out = torch.empty_like(E)
@@ -239,11 +274,18 @@ class BLMLBinned:
         sc = float(self.n_ / np.sqrt(Q)) if Q > 0 else 1.0
         return self._scale_(E, sc), self._scale_(U, sc)
 
-    def _resid(self, E, U, scale=1.0):
+    def _q_resid(self, E, U, scale, at):
         call('blml_resid', self._code, E.shape[0], self.B_, int(E.is_complex()), E.data_ptr(), U.data_ptr(),
-             self.c_t_.data_ptr(), float(scale), self._red.part.data_ptr(), self._red.out.data_ptr(), self._st)
-        mx, nnan = self._red.read(2)
+             self.c_t_.data_ptr(), float(scale), self._red.part.data_ptr(), self._red.at(at), self._st)
+
+    def _got_resid(self, at):
+        mx, nnan = self._red.got(at, 2)
         return float('nan') if nnan > 0 else mx
+
+    def _resid(self, E, U, scale=1.0):
+        self._q_resid(E, U, scale, 0)
+        self._red.wait()
+        return self._got_resid(0)
 
     # ---------------------------------------------------------------- CD solver
     def _solve(self, E, max_sweeps):
@@ -295,8 +337,11 @@ class BLMLBinned:
                         EJ, UJ, mJ = self._grad_steps(E, U, cur); n_grad += 1
             E, U = EJ, UJ
             self._rescale(E, U)
+            self._q_resid(E, U, 1.0, 4)
             cur = mJ if self.psd_ else self._merit(E, U); mhist.append(cur)
-            res = self._resid(E, U); hist.append(res)
+            if self.psd_:
+                self._red.wait()
+            res = self._got_resid(4); hist.append(res)
             if res < 0.9 * best_res or cur > best_m + 1e-13 * abs(best_m):
                 best_res, best_it, best_m = min(res, best_res), it, max(cur, best_m)
             if self.verbose and it % 100 == 0:
@@ -309,12 +354,15 @@ class BLMLBinned:
         self.rho_history_, self.n_anderson_, self.n_damped_, self.n_gradient_ = hist, n_and, n_damp, n_grad
         return E, U
 
-    def _grad_weights(self, U, vscale=1.0):
-        """V = vscale w / F U on occupied bins and sum_occ w log F."""
+    def _q_grad_weights(self, U, at, vscale=1.0):
+        """V = vscale w / F U on occupied bins; sum_occ w log F at place `at` after a wait."""
         V = torch.empty_like(U)
         call('blml_lgrad_weights', self._code, U.shape[0], self.B_, int(U.is_complex()), U.data_ptr(),
-             self.w_t_.data_ptr(), float(vscale), V.data_ptr(), self._red.part.data_ptr(), self._red.out.data_ptr(),
-             self._st)
+             self.w_t_.data_ptr(), float(vscale), V.data_ptr(), self._red.part.data_ptr(), self._red.at(at), self._st)
+        return V
+
+    def _grad_weights(self, U, vscale=1.0):
+        V = self._q_grad_weights(U, 0, vscale)
         return V, self._red.read(1)[0]
 
     def _grad_finish(self, SV, U, nq):
@@ -367,7 +415,12 @@ class BLMLBinned:
         L, g, Q = self._lgrad(E, U)
         Sh, Yh = [], []; SY = np.zeros((0, 0)); YY = np.zeros((0, 0))
         it = 0
-        res = self._resid(E, U, self.n_ / np.sqrt(Q) if Q > 0 else 1.0); hist = [res]; mhist = [L / n]
+        self._q_resid(E, U, self.n_ / np.sqrt(Q) if Q > 0 else 1.0, 0)
+        if g is not None:
+            self._q_dots([(g, g), (E, E)], 2)
+        self._red.wait()
+        res = self._got_resid(0); hist = [res]; mhist = [L / n]
+        a_ = b_ = np.zeros(0); gg, ee = self._red.got(2, 2)        # S^T g, Y^T g, g . g, e . e of the current point
         cap = np.inf if max_iter is None else max_iter; self.stop_reason_ = 'tol'; reset = False
         ftol, fwin = (self.ll_tol if self.ll_tol is not None else 1e-11), 10
         while res >= self.tol and it < cap:
@@ -375,8 +428,6 @@ class BLMLBinned:
                 self.stop_reason_ = 'll_tol'; break
             it += 1
             m = len(Sh)
-            vals = self._dots([(s, g) for s in Sh] + [(y, g) for y in Yh] + [(g, g), (E, E)])
-            a_, b_ = np.array(vals[:m]), np.array(vals[m:2 * m]); gg, ee = vals[2 * m], vals[2 * m + 1]
             first = 1e-3 * np.sqrt(ee / max(gg, 1e-300))
             if m:
                 gam = SY[-1, -1] / YY[-1, -1]
@@ -411,23 +462,37 @@ class BLMLBinned:
             # the accepted point's U exactly: U + t S q equals S(E + t q) only up to rounding, and a drifting U lets
             # the ascent move e along the near-null directions of S (which change Q = <E, U> through the drift alone)
             self._Sall(En, out=Un)
-            Qn = self._Q(En, Un)
-            V, Lwn = self._grad_weights(Un)
+            self._q_dots([(En, Un)], 0)
+            V = self._q_grad_weights(Un, 1)
+            SV = self._Sall(V)
+            self._red.wait()
+            Qn, Lwn = self._red.got(0, 2)
             Ln = Lwn - n * np.log(Qn) if Qn > 0 else -np.inf
-            gn = self._grad_finish(self._Sall(V), Un, n / Qn)
+            gn = self._grad_finish(SV, Un, n / Qn)
             s_ = self._lin([(t, q)]); y_ = self._lin([(1.0, g), (-1.0, gn)])
-            vals = self._dots([(s_, y_), (s_, s_), (y_, y_)] + [(s, y_) for s in Sh] + [(y, y_) for y in Yh])
+            # the new pair's products, the residual and the next direction's products (with the new pair's, in case it
+            # enters) share one wait
+            m = len(Sh)
+            Sn, Yn = Sh + [s_], Yh + [y_]
+            self._q_dots([(s_, y_), (s_, s_), (y_, y_)] + [(s, y_) for s in Sh] + [(y, y_) for y in Yh], 0)
+            self._q_resid(En, Un, self.n_ / np.sqrt(Qn), 64)
+            self._q_dots([(s, gn) for s in Sn] + [(y, gn) for y in Yn] + [(gn, gn), (En, En)], 66)
+            self._red.wait()
+            vals = self._red.got(0, 3 + 2 * m)
+            nxt = self._red.got(66, 2 * m + 4)
+            a_, b_ = np.array(nxt[:m + 1]), np.array(nxt[m + 1:2 * m + 2]); gg, ee = nxt[2 * m + 2:]
             sy, ss, yy = vals[:3]
             if sy > 1e-12 * np.sqrt(ss * yy):
-                m = len(Sh)
                 SYn = np.zeros((m + 1, m + 1)); SYn[:m, :m] = SY; SYn[:m, m] = vals[3:3 + m]; SYn[m, m] = sy
                 YYn = np.zeros((m + 1, m + 1)); YYn[:m, :m] = YY; YYn[:m, m] = YYn[m, :m] = vals[3 + m:3 + 2 * m]
                 YYn[m, m] = yy
-                Sh.append(s_); Yh.append(y_); SY, YY = SYn, YYn
+                Sh, Yh, SY, YY = Sn, Yn, SYn, YYn
                 if len(Sh) > m_:
-                    Sh.pop(0); Yh.pop(0); SY = SY[1:, 1:]; YY = YY[1:, 1:]
+                    Sh.pop(0); Yh.pop(0); SY = SY[1:, 1:]; YY = YY[1:, 1:]; a_, b_ = a_[1:], b_[1:]
+            else:
+                a_, b_ = a_[:m], b_[:m]
             E, U, L, g, Q = En, Un, Ln, gn, Qn
-            res = self._resid(E, U, self.n_ / np.sqrt(Q)); hist.append(res); mhist.append(L / n)
+            res = self._got_resid(64); hist.append(res); mhist.append(L / n)
             if self.verbose and it % 100 == 0:
                 print(f'  lbfgs {it}: max|rho|={res:.2e} L/n={L / n:.9f}', flush=True)
         if res >= self.tol and self.stop_reason_ == 'tol':
@@ -536,17 +601,10 @@ class BLMLBinned:
     def _fill_modes(self, E, kk, phases=True):
         """The reference's seeded start noise (blml_binned.py:429-436): the normals are drawn on the host with the same
         generator and order, then applied on the device."""
-        rng = np.random.default_rng(self.seed); sh = self.shape_
-        draws = []
-        if self.complex_g_ and phases:
-            draws.append(rng.standard_normal(sh).ravel())
-        for _ in range(kk, self.K_):
-            draws.append(rng.standard_normal(sh).ravel())
-            if self.complex_g_:
-                draws.append(rng.standard_normal(sh).ravel())
+        draws = int(self.complex_g_ and phases) + (self.K_ - kk) * (2 if self.complex_g_ else 1)     # one after another
         if not draws:
             return E
-        z = torch.as_tensor(np.concatenate(draws), dtype=torch.float64).to(self.dev_)
+        z = seeded_normals(self.seed, draws * self.B_, self.dev_)
         call('blml_fill_modes', self._code, self.K_, self.B_, int(E.is_complex()), int(kk), int(phases),
              float(self.phase_noise), z.data_ptr(), E.data_ptr(), self._st)
         return E

@@ -517,6 +517,11 @@ __device__ __forceinline__ int sched_find(const int* off, int n, int x, int& loc
   return lo;
 }
 
+// a few plans' lattices in one launch, their descriptors by value (the modes of one fit with kernels of their own: two
+// of 256 x 256 complex: 6 launches -> 3, 28 -> 19 us of kernels)
+constexpr int kFew = 4;
+struct FftFew { FftDesc d[kFew]; int n, offA[kFew + 1], offB[kFew + 1]; };
+
 // 4 CTAs per SM over many problems (the sweep's lattices 78 -> 73 us), 3 and more registers for one plan's lattices
 // (384 x 384 x 8: 36.1 -> 34.0 us)
 #define FFT_STAGE(NAME, BODY, OFF)                                                                                \
@@ -542,6 +547,14 @@ __device__ __forceinline__ int sched_find(const int* off, int n, int x, int& loc
     extern __shared__ __align__(16) unsigned char fft_smem[];                                                    \
     stage_wait();                                                                                                \
     BODY<T>(D, blockIdx.x, fft_smem);                                                                            \
+  }                                                                                                              \
+  template <typename T>                                                                                          \
+  __global__ void __launch_bounds__(kFT, 3) NAME##_few(const __grid_constant__ FftFew P) {                          \
+    extern __shared__ __align__(16) unsigned char fft_smem[];                                                    \
+    int i = 0;                                                                                                   \
+    while (i < P.n - 1 && (int)blockIdx.x >= P.OFF[i + 1]) i++;                                                  \
+    stage_wait();                                                                                                \
+    BODY<T>(P.d[i], (int)blockIdx.x - P.OFF[i], fft_smem);                                                       \
   }
 
 FFT_STAGE(k_fft_rows_fwd, rows_fwd_body, offA)
@@ -735,6 +748,7 @@ static int set_fft_smem() {
   if (!e) e = cuda_status(cudaFuncSetAttribute(k_fft_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmem), "FFT route");
   if (!e) e = cuda_status(cudaFuncSetAttribute(k_fft_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "FFT route");
   set((const void*)k_fft_rows_fwd_one<T>); set((const void*)k_fft_cols_one<T>); set((const void*)k_fft_rows_inv_one<T>);
+  set((const void*)k_fft_rows_fwd_few<T>); set((const void*)k_fft_cols_few<T>); set((const void*)k_fft_rows_inv_few<T>);
   return e;
 }
 
@@ -879,6 +893,10 @@ static int cluster_launch(const FftCluster& C, int nb, int cs, size_t smem, cuda
   return BLML_OK;
 }
 
+static bool cluster_rule(const blml_plan_s* p, int nb, int cs) {
+  return nb * cs <= 64 && p->shape[0] * p->shape[1] <= 1024LL * cs;
+}
+
 int fft_matvec(blml_plan_s* p, const void* x, void* y, int nb, int xc, void* ws, cudaStream_t st) {
   const size_t esz = p->dtype == BLML_F64 ? 16 : 8;
   const FftDesc D = make_desc(p, x, y, ws, nb, xc, (long long)nb * p->shape[0], (long long)nb * p->nfreq[1]);
@@ -886,7 +904,7 @@ int fft_matvec(blml_plan_s* p, const void* x, void* y, int nb, int xc, void* ws,
   // CTAs together (more than the GPU's clusters of that size would run in two waves). Float64, one lattice (three
   // launches -> one): 64 x 64 12.9 -> 8.7 us, 128 x 128 12.7 -> 11.0; at 256 x 256 sixteen CTAs are too few (15.1 -> 20.5).
   for (int cs = 16; cs >= 4; cs >>= 1) {
-    if (nb * cs > 64 || p->shape[0] * p->shape[1] > 1024LL * cs) continue;
+    if (!cluster_rule(p, nb, cs)) continue;
     FftCluster C;
     size_t smem = 0;
     if (cluster_args(D, cs, esz, C, smem))
@@ -894,6 +912,42 @@ int fft_matvec(blml_plan_s* p, const void* x, void* y, int nb, int xc, void* ws,
   }
   const size_t smA = rows_smem(D.ax2, D.rows, esz), smB = cols_smem(D.ax1, D.cols, esz);
   return p->dtype == BLML_F64 ? launch_fft_one<double>(D, smA, smB, st) : launch_fft_one<float>(D, smA, smB, st);
+}
+
+template <typename T>
+static int launch_fft_few(const FftFew& P, size_t smA, size_t smB, cudaStream_t st) {
+  launch_dep(k_fft_rows_fwd_few<T>, P.offA[P.n], smA, st, P);
+  BLML_CHECK_LAUNCH("FFT route: rows");
+  launch_dep(k_fft_cols_few<T>, P.offB[P.n], smB, st, P);
+  BLML_CHECK_LAUNCH("FFT route: columns");
+  launch_dep(k_fft_rows_inv_few<T>, P.offA[P.n], smA, st, P);
+  BLML_CHECK_LAUNCH("FFT route: inverse rows");
+  return BLML_OK;
+}
+
+// whether n problems go in one launch chain: a few, and none small enough for one of its own
+bool fft_few(int n, const blml_plan* plans, const int* nb) {
+  if (n < 2 || n > kFew) return false;
+  for (int i = 0; i < n; i++)
+    if (cluster_rule(plans[i], nb[i], 16)) return false;
+  return true;
+}
+
+int fft_matvec_few(int n, const blml_plan* plans, const int* nb, const void* const* x, void* const* y, void* const* z,
+                   int xc, cudaStream_t st) {
+  const bool f64 = plans[0]->dtype == BLML_F64;
+  const size_t esz = f64 ? 16 : 8;
+  long long rows = 0, cols = 0;
+  for (int i = 0; i < n; i++) { rows += (long long)nb[i] * plans[i]->shape[0]; cols += (long long)nb[i] * plans[i]->nfreq[1]; }
+  FftFew P{};
+  size_t smA = 0, smB = 0;
+  P.n = n;
+  for (int i = 0; i < n; i++) {
+    P.d[i] = make_desc(plans[i], x[i], y[i], z[i], nb[i], xc, rows, cols);
+    P.offA[i + 1] = P.offA[i] + P.d[i].ctasA; P.offB[i + 1] = P.offB[i] + P.d[i].ctasB;
+    smA = std::max(smA, rows_smem(P.d[i].ax2, P.d[i].rows, esz)); smB = std::max(smB, cols_smem(P.d[i].ax1, P.d[i].cols, esz));
+  }
+  return f64 ? launch_fft_few<double>(P, smA, smB, st) : launch_fft_few<float>(P, smA, smB, st);
 }
 
 }  // namespace blml

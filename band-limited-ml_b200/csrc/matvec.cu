@@ -949,6 +949,61 @@ int blml_matvec(blml_plan p, const void* x, void* y, int nb, int xc, void* ws, i
                               : simt_matvec<float>(p, x, y, nb, xc, ws, st);
 }
 
+// whether the plans' FFT routes go in one launch chain
+static bool few_ffts(int n, const blml_plan* plans, const int* nb) {
+  for (int i = 0; i < n; i++)
+    if (plans[i]->engine == BLML_ENGINE_TC || plans[i]->route != BLML_ROUTE_FFT) return false;
+  return fft_few(n, plans, nb);
+}
+
+static int matvecs_args(int n, const blml_plan* plans, const int* nb) {
+  bool ok = n >= 1 && plans && nb;
+  for (int i = 0; i < n && ok; i++) ok = plans[i] && nb[i] >= 1 && plans[i]->dtype == plans[0]->dtype;
+  if (!ok) { set_error("blml_matvecs: plans of one dtype, nb >= 1 each"); return BLML_ERR_ARG; }
+  return BLML_OK;
+}
+
+int64_t blml_matvecs_workspace(int n, const blml_plan* plans, const int* nb) {
+  if (matvecs_args(n, plans, nb)) return -1;
+  const bool few = few_ffts(n, plans, nb);
+  int64_t sum = 0, most = 0;
+  for (int i = 0; i < n; i++) {
+    const int64_t w = (blml_matvec_workspace(plans[i], nb[i]) + 255) & ~(int64_t)255;
+    sum += w; most = std::max(most, w);
+  }
+  return few ? sum : most;
+}
+
+int blml_matvecs(int n, const blml_plan* plans, const int* nb, const void* x, void* y, int xc, void* ws, int64_t wsb,
+                 void* stream) {
+  const int e = matvecs_args(n, plans, nb);
+  if (e) return e;
+  if (!x || !y) { set_error("blml_matvecs: bad arguments"); return BLML_ERR_ARG; }
+  const int64_t need = blml_matvecs_workspace(n, plans, nb);
+  if (wsb < need || (need > 0 && !ws)) {
+    set_error("blml_matvecs: workspace of %lld bytes, need %lld", (long long)wsb, (long long)need);
+    return BLML_ERR_WORKSPACE;
+  }
+  const bool few = few_ffts(n, plans, nb);
+  const size_t es = (plans[0]->dtype == BLML_F64 ? 8 : 4) * (xc ? 2 : 1);
+  const char* xi = reinterpret_cast<const char*>(x);
+  char* yi = reinterpret_cast<char*>(y);
+  char* wi = reinterpret_cast<char*>(ws);
+  const void* xs[8]; void* ys[8]; void* zs[8];
+  for (int i = 0; i < n; i++) {
+    size_t el = (size_t)nb[i];
+    for (int a = 0; a < plans[i]->d; a++) el *= (size_t)plans[i]->shape[a];
+    if (few) {
+      xs[i] = xi; ys[i] = yi; zs[i] = wi;
+      wi += (blml_matvec_workspace(plans[i], nb[i]) + 255) & ~(int64_t)255;
+    } else if (const int rc = blml_matvec(plans[i], xi, yi, nb[i], xc, ws, wsb, stream)) {
+      return rc;
+    }
+    xi += el * es; yi += el * es;
+  }
+  return few ? fft_matvec_few(n, plans, nb, xs, ys, zs, xc, reinterpret_cast<cudaStream_t>(stream)) : BLML_OK;
+}
+
 int blml_plan_set_route(blml_plan p, int route) {
   if (!p) { set_error("blml_plan_set_route: null plan"); return BLML_ERR_ARG; }
   if (route == BLML_ROUTE_AUTO) route = p->fft ? BLML_ROUTE_FFT : BLML_ROUTE_CONTRACT;

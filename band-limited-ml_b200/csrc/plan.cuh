@@ -30,6 +30,10 @@ int fft_plan_init(blml_plan_s* p, const double* freqs, const double* weights);
 void fft_plan_free(blml_plan_s* p);
 int64_t fft_workspace(const blml_plan_s* p, int nb);
 int fft_matvec(blml_plan_s* p, const void* x, void* y, int nb, int xc, void* ws, cudaStream_t st);
+// the same for a few plans at once, when fft_few says so (z[i]: problem i's workspace)
+bool fft_few(int n, const blml_plan* plans, const int* nb);
+int fft_matvec_few(int n, const blml_plan* plans, const int* nb, const void* const* x, void* const* y, void* const* z,
+                   int xc, cudaStream_t st);
 // a group's descriptors: problem g reads x[g], writes y[g] and keeps its spectrum in z[g] (its workspace); *out stays
 // null when a plan has no FFT route. dev: fft_group_bytes(G) bytes of device memory (kept); its first bytes are to be
 // filled from `up`

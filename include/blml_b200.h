@@ -32,6 +32,8 @@ enum { BLML_ROUTE_AUTO = 0, BLML_ROUTE_CONTRACT = 1, BLML_ROUTE_FFT = 2 };
 typedef struct blml_plan_s* blml_plan;
 
 const char* blml_last_error(void);
+/* returns when the stream's work is done (results written to mapped host memory are then there) */
+int blml_stream_wait(void* stream);
 int blml_abi_version(void);
 /* blocks of every reduction grid: `part` buffers hold nq * blml_reduce_blocks() doubles */
 int blml_reduce_blocks(void);
@@ -59,6 +61,12 @@ int blml_plan_status(blml_plan plan);
 int blml_plan_set_route(blml_plan plan, int route);
 /* the route blml_matvec takes (BLML_ROUTE_CONTRACT or BLML_ROUTE_FFT) */
 int blml_plan_route(blml_plan plan);
+
+/* n plans of one dtype on consecutive lattices of x and y (nb[i] of plan i): the modes of one fit with kernels of their
+ * own, in one launch chain where their routes allow */
+int64_t blml_matvecs_workspace(int n, const blml_plan* plans, const int* nb);
+int blml_matvecs(int n, const blml_plan* plans, const int* nb, const void* x, void* y, int x_complex, void* workspace,
+                 int64_t workspace_bytes, void* stream);
 
 /* ---- grouped mat-vecs: many plans (fits of uneven lattice size and band) applied in one launch per stage ----
  * Problem g: y_base[y_off[g] ...] = S_g x_base[x_off[g] ...] over nbatch[g] lattices of plan g (SIMT engine); every
