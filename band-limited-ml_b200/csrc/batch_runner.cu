@@ -43,11 +43,6 @@ __global__ void k_fill_int(int* a, int n, int v) {
   if (i < n) a[i] = v;
 }
 
-__global__ void k_fill_double(double* a, int64_t n, double v) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = v;
-}
-
 // one warp per quantity: out[j * nq + q] = the fixed-order sum of the fit's nblk partials, for the fits whose flag
 // is set
 __global__ void k_finish_flagged(const double* part, int nq, int nblk, const int* flag, double* out) {
@@ -153,20 +148,13 @@ __global__ void k_lb_dir(int m, const int* fid, const int* live, const double* H
   }
 }
 
-// the Armijo trials t_j = 2^-j, j0 <= j < j0 + NTG, of the fits whose flag is set (all when null): sum_occ w log F(U +
+// the Armijo trials t_j = 2^-j, j0 <= j < j0 + NTG, of every fit, or (more) of the fits whose flag is set: sum_occ w log F(U +
 // t_j S q); the first group also <q, U>, <E, S q>, <q, S q> (Q(t) = Q + t (<q, U> + <E, S q>) + t^2 <q, S q>) and <q, q>
 template <typename T, int NTG, bool FIRST>
-__global__ void __launch_bounds__(256) k_lb_trials(const blml_seg* segs, const int* flag, int j0, const void* E,
-                                                   const void* q, const void* U, const void* Sq, const T* w,
-                                                   double* part) {
-  if (flag && !flag[blockIdx.y]) return;
-  const blml_seg S = segs[blockIdx.y];
-  constexpr int NQ = NTG + (FIRST ? 4 : 0);
-  double v[NQ];
-#pragma unroll
-  for (int j = 0; j < NQ; j++) v[j] = 0.0;
+__device__ __forceinline__ void lb_trials(const blml_seg& S, int bx, int nblk, int j0, const void* E, const void* q,
+                                          const void* U, const void* Sq, const T* w, double* v) {
   const double t0 = ldexp(1.0, -j0);
-  SEG_LOOP(b, S) {
+  for (int64_t b = (int64_t)bx * blockDim.x + threadIdx.x; b < S.B; b += (int64_t)nblk * blockDim.x) {
     const double wb = (double)w[S.boff + b];
     double a = 0.0, bb = 0.0, cc = 0.0;        // F(t) = a + 2 t b + t^2 c
     for (int k = 0; k < S.K; k++) {
@@ -186,7 +174,29 @@ __global__ void __launch_bounds__(256) k_lb_trials(const blml_seg* segs, const i
       for (int j = 0; j < NTG; j++) { v[j] += wb * log(a + t * (2.0 * bb + t * cc)); t *= 0.5; }
     }
   }
-  seg_partials<NQ>(v, part);
+}
+
+template <typename T, int NTG>
+__global__ void __launch_bounds__(256) k_lb_trials(const blml_seg* segs, const void* E, const void* q, const void* U,
+                                                   const void* Sq, const T* w, double* part) {
+  double v[NTG + 4];
+#pragma unroll
+  for (int j = 0; j < NTG + 4; j++) v[j] = 0.0;
+  lb_trials<T, NTG, true>(segs[blockIdx.y], blockIdx.x, gridDim.x, 0, E, q, U, Sq, w, v);
+  seg_partials<NTG + 4>(v, part);
+}
+
+template <typename T, int NTG>
+__global__ void __launch_bounds__(256) k_lb_trials_more(const blml_seg* segs, const int* flag, int F, int nblk, int j0,
+                                                        const void* E, const void* q, const void* U, const void* Sq,
+                                                        const T* w, double* part) {
+  seg_flagged(flag, F, nblk, [&](int j, int bx) {
+    double v[NTG];
+#pragma unroll
+    for (int i = 0; i < NTG; i++) v[i] = 0.0;
+    lb_trials<T, NTG, false>(segs[j], bx, nblk, j0, E, q, U, Sq, w, v);
+    seg_partials_at<NTG>(v, part, 0u, F, j, nblk, bx);
+  });
 }
 
 constexpr int LB_T1 = 8, LB_T2 = LB_NT - LB_T1;
@@ -220,9 +230,9 @@ __global__ void k_lb_select1(int Fa, const int* fid, const int* live, const doub
 }
 
 // the remaining trials of the fits that need them, then every fit's outcome: a failed search clears the memory once
-// and stops the fit ('stall') when it fails again or had no pairs; the coefficient rows of the pair and g updates
+// and stops the fit ('stall') when it fails again or had no pairs
 __global__ void k_lb_select2(int Fa, int m, const int* fid, const int* live, const double* T1, const double* T2,
-                             const int* need2, LbState s, double* tA, double* cS, double* cY, double* cG) {
+                             const int* need2, LbState s, double* tA) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= Fa) return;
   const int f = fid[j];
@@ -248,11 +258,7 @@ __global__ void k_lb_select2(int Fa, int m, const int* fid, const int* live, con
     }
   }
   s.ok[f] = ok;
-  const double o = ok ? 1.0 : 0.0;
-  tA[j] = t;
-  cS[2 * j] = t; cS[2 * j + 1] = 1.0 - o;
-  cY[3 * j] = o; cY[3 * j + 1] = -o; cY[3 * j + 2] = 1.0 - o;
-  cG[2 * j] = o; cG[2 * j + 1] = 1.0 - o;
+  tA[j] = t;                               // 0: no step
 }
 
 // the gradient weights at the new point fused with Q: F = sum_k |U_k|^2, V = (w / F) U on occupied bins,
@@ -281,6 +287,88 @@ __global__ void __launch_bounds__(256) k_lb_weights(const blml_seg* segs, const 
     }
   }
   seg_partials<2>(v, part);
+}
+
+// the accepted step E += t q, U += t S q (float64) and k_lb_weights' quantities at the new point, with the same rounding:
+// E and U are read once (64 fits of rank 4: 198 us in two launches -> 138)
+__global__ void __launch_bounds__(256) k_lb_accept(const blml_seg* segs, void* E, const void* q, void* U, const void* Sq,
+                                                   const double* t, const double* w, void* V, double* part) {
+  const blml_seg S = segs[blockIdx.y];
+  const double tf = t[blockIdx.y];
+  double v[2] = {0.0, 0.0};
+  SEG_LOOP(b, S) {
+    double F = 0.0;
+    for (int k = 0; k < S.K; k++) {
+      const int64_t i = S.off + (int64_t)k * S.B + b;
+      double er, ei, ur, ui;
+      SAcc<double, true>::get(E, i, er, ei); SAcc<double, true>::get(U, i, ur, ui);
+      if (tf != 0.0) {
+        double qr, qi, sr, si;
+        SAcc<double, true>::get(q, i, qr, qi); SAcc<double, true>::get(Sq, i, sr, si);
+        er += tf * qr; ei += tf * qi; ur += tf * sr; ui += tf * si;
+        SAcc<double, true>::put(E, i, er, ei); SAcc<double, true>::put(U, i, ur, ui);
+      }
+      F += fma(ur, ur, __dmul_rn(ui, ui)); v[1] += fma(er, ur, __dmul_rn(ei, ui));     // as k_lb_weights compiles
+    }
+    const double wb = w[S.boff + b];
+    const bool occ = wb > 0;
+    if (occ) v[0] += wb * log(F);
+    const double fw = occ ? wb / F : 0.0;
+    for (int k = 0; k < S.K; k++) {
+      const int64_t i = S.off + (int64_t)k * S.B + b;
+      double ur, ui; SAcc<double, true>::get(U, i, ur, ui);
+      SAcc<double, true>::put(V, i, occ ? ur * fw : 0.0, occ ? ui * fw : 0.0);
+    }
+  }
+  seg_partials<2>(v, part);
+}
+
+// The end of a step in one pass: the gradient g_new = 2 (S V - n U / Q) on occupied bins; of the fits that stepped the pair
+// s = t q, y = g - g_new into slot p and g = g_new; the residual at (E, U). Five vectors read and three written, where
+// the gradient, the two pair vectors, g and the residual each by itself read ten and wrote four (64 fits of rank 4, a
+// step's share of 15: 340 us in five launches -> 223).
+template <typename T, typename TH>
+__global__ void __launch_bounds__(256) k_lb_pair(const blml_seg* segs, const void* SV, const void* U, const void* E,
+                                                 const void* q, const T* w, const T* c, const double* nq,
+                                                 const double* scale, const double* t, void* g, void* Sp,
+                                                  void* Yp, double* part) {
+  const blml_seg S = segs[blockIdx.y];
+  const double nqj = nq[blockIdx.y], sc = scale[blockIdx.y], tj = t[blockIdx.y];
+  const bool ok = tj != 0.0;
+  double v[2] = {0.0, 0.0};
+  SEG_LOOP(b, S) {
+    const bool occ = (double)w[S.boff + b] > 0;
+    double nrm2 = 0.0;
+    for (int k = 0; k < S.K; k++) {
+      const int64_t i = S.off + (int64_t)k * S.B + b;
+      double er, ei, ur, ui, sr, si;
+      SAcc<T, true>::get(E, i, er, ei);
+      if (ok) {
+        double qr, qi, gr, gi;
+        SAcc<T, true>::get(SV, i, sr, si); SAcc<T, true>::get(U, i, ur, ui);
+        SAcc<T, true>::get(q, i, qr, qi); SAcc<T, true>::get(g, i, gr, gi);
+        const double nr = (double)(T)(occ ? 2.0 * (sr - nqj * ur) : 0.0), ni = (double)(T)(occ ? 2.0 * (si - nqj * ui) : 0.0);
+        SAcc<TH, true>::put(Sp, i, fma(tj, qr, 0.0), fma(tj, qi, 0.0));
+        SAcc<TH, true>::put(Yp, i, gr - nr, gi - ni);
+        SAcc<T, true>::put(g, i, nr, ni);
+      }
+      er *= sc; ei *= sc; nrm2 += er * er + ei * ei;
+    }
+    const double cb = (double)c[S.boff + b];
+    if (!(cb > 0)) continue;
+    const double f = nrm2 / cb;
+    double r2 = 0.0;
+    for (int k = 0; k < S.K; k++) {
+      double er, ei, ur, ui;
+      const int64_t i = S.off + (int64_t)k * S.B + b;
+      SAcc<T, true>::get(E, i, er, ei); SAcc<T, true>::get(U, i, ur, ui);
+      const double dr = ur * sc * f - er * sc, di = ui * sc * f - ei * sc;
+      r2 += dr * dr + di * di;
+    }
+    const double r = sqrt(r2) / sqrt(fmax(nrm2, 1e-300));
+    if (r != r) v[1] += 1.0; else v[0] = fmax(v[0], r);
+  }
+  seg_partials<2>(v, part, 1u);
 }
 
 // Q at the new point, and the scales of the gradient finish (n / Q) and of the residual (n / sqrt Q)
@@ -481,28 +569,30 @@ __global__ void k_st_take(int Fa, int mA, const int* fid, const int* live, const
 // merit terms of E + a (E_J - E), U + a (U_J - U), formed as the linear-combination kernel forms them
 constexpr int DAMP_T1 = 4, DAMP_T2 = DAMP_NT - DAMP_T1;
 template <int NTG>
-__global__ void __launch_bounds__(256) k_st_damp_trials(const blml_seg* segs, const int* flag, int j0, const double* E,
-                                                        const double* EJ, const double* U, const double* UJ,
-                                                        const double* c, const double* sg, double* part) {
-  if (!flag[blockIdx.y]) return;
-  const blml_seg S = segs[blockIdx.y];
-  double v[3 * NTG];
+__global__ void __launch_bounds__(256) k_st_damp_trials(const blml_seg* segs, const int* flag, int F, int nblk, int j0,
+                                                        const double* E, const double* EJ, const double* U,
+                                                        const double* UJ, const double* c, const double* sg,
+                                                        double* part) {
+  seg_flagged(flag, F, nblk, [&](int j, int bx) {
+    const blml_seg S = segs[j];
+    double v[3 * NTG];
 #pragma unroll
-  for (int q = 0; q < 3 * NTG; q++) v[q] = 0.0;
-  const double a0 = ldexp(1.0, -(j0 + 1));
-  SEG_LOOP(b, S) {
-    const double e0 = E[S.off + b], e1 = EJ[S.off + b], u0 = U[S.off + b], u1 = UJ[S.off + b];
-    const double cb = c[S.boff + b], sgb = sg[S.boff + b];
-    double a = a0;
+    for (int q = 0; q < 3 * NTG; q++) v[q] = 0.0;
+    const double a0 = ldexp(1.0, -(j0 + 1));
+    for (int64_t b = (int64_t)bx * blockDim.x + threadIdx.x; b < S.B; b += (int64_t)nblk * blockDim.x) {
+      const double e0 = E[S.off + b], e1 = EJ[S.off + b], u0 = U[S.off + b], u1 = UJ[S.off + b];
+      const double cb = c[S.boff + b], sgb = sg[S.boff + b];
+      double a = a0;
 #pragma unroll
-    for (int k = 0; k < NTG; k++) {
-      const double e = fma(a, e1, (1.0 - a) * e0), u = fma(a, u1, (1.0 - a) * u0);
-      v[3 * k] += e * u;
-      if (cb > 0) { v[3 * k + 1] += cb * log(fabs(e)); if (sgb * e <= 0) v[3 * k + 2] += 1.0; }
-      a *= 0.5;
+      for (int k = 0; k < NTG; k++) {
+        const double e = fma(a, e1, (1.0 - a) * e0), u = fma(a, u1, (1.0 - a) * u0);
+        v[3 * k] += e * u;
+        if (cb > 0) { v[3 * k + 1] += cb * log(fabs(e)); if (sgb * e <= 0) v[3 * k + 2] += 1.0; }
+        a *= 0.5;
+      }
     }
-  }
-  seg_partials<3 * NTG>(v, part);
+    seg_partials_at<3 * NTG>(v, part, 0u, F, j, nblk, bx);
+  });
 }
 
 // the first damped trial (of the first 4) whose merit does not fall below the current one; the coefficients of the
@@ -858,15 +948,14 @@ struct blml_lbfgs_batch_s : Runner {
   blml_group gEU = nullptr, gq = nullptr, gV = nullptr;
   void *E = nullptr, *U = nullptr;
   const void *w = nullptr, *c = nullptr;
-  void *g = nullptr, *gn = nullptr, *q = nullptr, *Sq = nullptr, *V = nullptr, *SV = nullptr;
+  void *g = nullptr, *q = nullptr, *Sq = nullptr, *V = nullptr, *SV = nullptr;
   void *Sh[LB_MMAX] = {}, *Yh[LB_MMAX] = {};
   int h32 = 0;                           // the history (Sh, Yh) in complex64 storage (float64 state only)
   int64_t tot = 0;                       // elements of every mode array (the fits' K B summed)
   void* hvec = nullptr;                  // the history's allocation
   double *part = nullptr, *H1 = nullptr, *H2 = nullptr, *T1 = nullptr, *T2 = nullptr, *outC = nullptr,
          *outD = nullptr, *outE = nullptr;
-  double *cq = nullptr, *tA = nullptr, *cS = nullptr, *cY = nullptr, *cG = nullptr, *nqA = nullptr, *scrA = nullptr,
-         *ones = nullptr, *sc = nullptr;
+  double *cq = nullptr, *tA = nullptr, *nqA = nullptr, *scrA = nullptr, *sc = nullptr;
   int* need2 = nullptr;
   int* split = nullptr;                  // the block split of the float32 history's kernels (seg_split)
   LbState s{};
@@ -876,32 +965,28 @@ struct blml_lbfgs_batch_s : Runner {
   // over the slots that hold a pair (in set-up: none, and slot 0 is zero)
   int hist(int Fa_, const blml_seg* S, int p) {
     const HistMask hm{s.stamp, d_fid, m, p};
-    for (int h = 0; h < 2; h++) {
-      const void* a[LB_MMAX];
-      for (int i = 0; i < m; i++) a[i] = h ? Yh[i] : Sh[i];
-      const void* x = h ? nullptr : E;
-      double* out = h ? H2 : H1;
-      RC(h32 ? seg_dots2_h32(Fa_, S, split, m, a, Yh[p], g, x, part, out, hm, st)
-             : seg_dots2(dtype, Fa_, S, 1, m, a, Yh[p], g, x, part, out, hm, st));
-    }
-    return BLML_OK;
+    const void* a[LB_MMAX]; const void* a2[LB_MMAX];
+    for (int i = 0; i < m; i++) { a[i] = Sh[i]; a2[i] = Yh[i]; }
+    return h32 ? seg_dots2_h32(Fa_, S, split, m, a, a2, Yh[p], g, E, part, H1, H2, hm, st)
+               : seg_dots2(dtype, Fa_, S, 1, m, a, a2, Yh[p], g, E, part, H1, H2, hm, st);
   }
 
   template <typename T>
   int trials(int Fa_, const blml_seg* S) {
     const dim3 grid((unsigned)seg_blocks_for(Fa_), (unsigned)Fa_);
     const int nb = seg_blocks_for(Fa_);
-    k_lb_trials<T, LB_T1, true><<<grid, 256, 0, st>>>(S, nullptr, 0, E, q, U, Sq, (const T*)w, part);
+    k_lb_trials<T, LB_T1><<<grid, 256, 0, st>>>(S, E, q, U, Sq, (const T*)w, part);
     KCHECK("lbfgs trials");
     k_finish_flagged<<<Fa_, 256, 0, st>>>(part, LB_T1 + 4, nb, nullptr, T1);
     KCHECK("lbfgs trials finish");
     k_lb_select1<<<nblk(Fa_, 128), 128, 0, st>>>(Fa_, d_fid, d_live, T1, s, tA, need2);
     KCHECK("lbfgs select");
-    k_lb_trials<T, LB_T2, false><<<grid, 256, 0, st>>>(S, need2, LB_T1, E, q, U, Sq, (const T*)w, part);
+    k_lb_trials_more<T, LB_T2><<<SEG_FLAGGED_BLOCKS, 256, 0, st>>>(S, need2, Fa_, nb, LB_T1, E, q, U, Sq, (const T*)w,
+                                                                   part);
     KCHECK("lbfgs trials");
     k_finish_flagged<<<Fa_, 256, 0, st>>>(part, LB_T2, nb, need2, T2);
     KCHECK("lbfgs trials finish");
-    k_lb_select2<<<nblk(Fa_, 128), 128, 0, st>>>(Fa_, m, d_fid, d_live, T1, T2, need2, s, tA, cS, cY, cG);
+    k_lb_select2<<<nblk(Fa_, 128), 128, 0, st>>>(Fa_, m, d_fid, d_live, T1, T2, need2, s, tA);
     KCHECK("lbfgs select");
     return BLML_OK;
   }
@@ -934,25 +1019,32 @@ struct blml_lbfgs_batch_s : Runner {
     RC(blml_group_matvec_masked(gq, d_fid, Fa_, d_live, sv));
     // every fit's Armijo search (8 trials, then 32 more for the fits that need them), the accepted steps, U = S E
     RC(dt == BLML_F64 ? trials<double>(Fa_, S) : trials<float>(Fa_, S));
-    RC(blml_seg_axpy2(dt, Fa_, S, 1, E, q, U, Sq, tA, sv));
     // U + t S q is S(E + t q) up to rounding: float32 state recomputes U = S E exactly at every step (its rounding
     // would otherwise accumulate into the null space of S); float64 once per ring of m steps
-    if (dt == BLML_F32 || p == m - 1) RC(blml_group_matvec_masked(gEU, d_fid, Fa_, d_live, sv));
+    const dim3 grid((unsigned)seg_blocks_for(Fa_), (unsigned)Fa_);
+    if (dt == BLML_F32 || p == m - 1) {
+      RC(blml_seg_axpy2(dt, Fa_, S, 1, E, q, U, Sq, tA, sv));
+      RC(blml_group_matvec_masked(gEU, d_fid, Fa_, d_live, sv));
+      RC(dt == BLML_F64 ? weights<double>(Fa_, S) : weights<float>(Fa_, S));
+    } else {
+      k_lb_accept<<<grid, 256, 0, st>>>(S, E, q, U, Sq, tA, (const double*)w, V, part);
+      KCHECK("lbfgs step");
+      k_finish_flagged<<<Fa_, 256, 0, st>>>(part, 2, seg_blocks_for(Fa_), nullptr, outD);
+      KCHECK("lbfgs step finish");
+    }
     // gradient at the new point (with Q), the new pair into slot p, g, the residual, the history scan
-    RC(dt == BLML_F64 ? weights<double>(Fa_, S) : weights<float>(Fa_, S));
     k_lb_qeff<<<nblk(Fa_, 128), 128, 0, st>>>(Fa_, d_fid, d_live, outD, s, nqA, scrA);
     KCHECK("lbfgs qeff");
     RC(blml_group_matvec_masked(gV, d_fid, Fa_, d_live, sv));
-    RC(blml_seg_lgrad_finish(dt, Fa_, S, 1, SV, U, w, nqA, gn, sv));
-    terms[0] = q; terms[1] = Sh[p];
-    if (h32) RC(seg_lincomb_mixed(Fa_, S, split, Sh[p], 1, 2, cS, terms, 2ull, st));
-    else RC(blml_seg_lincomb(dt, Fa_, S, 1, Sh[p], 2, cS, terms, sv));
-    terms[0] = g; terms[1] = gn; terms[2] = Yh[p];
-    if (h32) RC(seg_lincomb_mixed(Fa_, S, split, Yh[p], 1, 3, cY, terms, 4ull, st));
-    else RC(blml_seg_lincomb(dt, Fa_, S, 1, Yh[p], 3, cY, terms, sv));
-    terms[0] = gn; terms[1] = g;
-    RC(blml_seg_lincomb(dt, Fa_, S, 1, g, 2, cG, terms, sv));
-    RC(blml_seg_resid(dt, Fa_, S, 1, E, U, c, scrA, part, outE, sv));
+    auto pair = [&](auto k, auto tag) {
+      using T = decltype(tag);
+      k<<<grid, 256, 0, st>>>(S, SV, U, E, q, (const T*)w, (const T*)c, nqA, scrA, tA, g, Sh[p], Yh[p], part);
+    };
+    if (h32) pair(k_lb_pair<double, float>, double());
+    else if (dt == BLML_F64) pair(k_lb_pair<double, double>, double());
+    else pair(k_lb_pair<float, float>, float());
+    KCHECK("lbfgs pair");
+    RC(seg_finish_resid(Fa_, part, outE, st));
     RC(hist(Fa_, S, p));
     k_lb_post<<<nblk(Fa_, 128), 128, 0, st>>>(Fa_, m, p, tol, ftol, cap, d_fid, d_live, d_segs_c, d_segs_eff, H1,
                                               H2, outD, outE, tA, s);
@@ -976,9 +1068,7 @@ struct blml_lbfgs_batch_s : Runner {
     RC(blml_seg_lincomb(dt, F, S, 1, U, 1, sc, t1, sv));
     RC(dt == BLML_F64 ? weights<double>(F, S) : weights<float>(F, S));
     RC(blml_group_matvec_masked(gV, d_fid, F, d_live, sv));
-    RC(blml_seg_lgrad_finish(dt, F, S, 1, SV, U, w, nqA, gn, sv));
-    t1[0] = gn;
-    RC(blml_seg_lincomb(dt, F, S, 1, g, 1, ones, t1, sv));
+    RC(blml_seg_lgrad_finish(dt, F, S, 1, SV, U, w, nqA, g, sv));
     RC(blml_seg_resid(dt, F, S, 1, E, U, c, scrA, part, outE, sv));
     if (h32) RC(seg_split(F, S, split, st));
     RC(hist(F, S, 0));                                  // empty history: g . g and E . E for the first direction
@@ -1067,13 +1157,13 @@ struct blml_start_batch_s : Runner {
     k_st_lin2<<<grid, 256, 0, st>>>(S, 2, cT, Terms3{{EA, EJ, nullptr}}, ET, Terms3{{UA, UJ, nullptr}}, UT);
     KCHECK("start candidate");
     // damped steps: 4 trials, then 22 more for the fits none of the 4 served
-    k_st_damp_trials<DAMP_T1><<<grid, 256, 0, st>>>(S, damp, 0, E, EJ, U, UJ, c, sg, part);
+    k_st_damp_trials<DAMP_T1><<<SEG_FLAGGED_BLOCKS, 256, 0, st>>>(S, damp, Fa_, (int)grid.x, 0, E, EJ, U, UJ, c, sg, part);
     KCHECK("start damping trials");
     k_finish_flagged<<<Fa_, 256, 0, st>>>(part, 3 * DAMP_T1, seg_blocks_for(Fa_), damp, outDT);
     KCHECK("start damping finish");
     k_st_damp_pick1<<<nblk(Fa_, 128), 128, 0, st>>>(Fa_, d_fid, d_live, damp, outDT, s, cE, need2d);
     KCHECK("start damping pick");
-    k_st_damp_trials<DAMP_T2><<<grid, 256, 0, st>>>(S, need2d, DAMP_T1, E, EJ, U, UJ, c, sg, part);
+    k_st_damp_trials<DAMP_T2><<<SEG_FLAGGED_BLOCKS, 256, 0, st>>>(S, need2d, Fa_, (int)grid.x, DAMP_T1, E, EJ, U, UJ, c, sg, part);
     KCHECK("start damping trials");
     k_finish_flagged<<<Fa_, 256, 0, st>>>(part, 3 * DAMP_T2, seg_blocks_for(Fa_), need2d, outDT2);
     KCHECK("start damping finish");
@@ -1143,13 +1233,13 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
   r->lend = lend; r->lend_ctx = ctx; r->lend_st = reinterpret_cast<cudaStream_t>(stream);
   int rc = r->base_init(F, segs);
   const size_t esz = dtype == BLML_F64 ? 16 : 8, hsz = r->h32 ? 8 : esz;
-  char* vec = rc ? nullptr : (char*)r->dalloc(6 * tot * esz);
+  char* vec = rc ? nullptr : (char*)r->dalloc(5 * tot * esz);
   char* hv = rc ? nullptr : (char*)r->dalloc(2 * (size_t)m * tot * hsz);
   if (!rc && (!vec || !hv)) { set_error("blml_lbfgs_batch_create: vector allocation"); rc = BLML_ERR_CUDA; }
   if (!rc) {
     r->tot = tot; r->hvec = hv;
-    void** v6[6] = {&r->g, &r->gn, &r->q, &r->Sq, &r->V, &r->SV};
-    for (int i = 0; i < 6; i++) *v6[i] = vec + (size_t)i * tot * esz;
+    void** v5[5] = {&r->g, &r->q, &r->Sq, &r->V, &r->SV};
+    for (int i = 0; i < 5; i++) *v5[i] = vec + (size_t)i * tot * esz;
     for (int i = 0; i < m; i++) {
       r->Sh[i] = hv + (size_t)i * tot * hsz;
       r->Yh[i] = hv + ((size_t)m + i) * tot * hsz;
@@ -1157,13 +1247,12 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
     // slot 0, which the set-up's scan reads; nothing else is read before it is written
     cudaMemsetAsync(r->Sh[0], 0, tot * hsz, r->st);
     cudaMemsetAsync(r->Yh[0], 0, tot * hsz, r->st);
-    // >= Fa * seg_blocks_for(Fa) for every Fa <= F, and 48 pw >= 43 (SEG_SPLIT_BLOCKS + Fa) for the split scan
+    // >= Fa * seg_blocks_for(Fa) and SEG_SPLIT_BLOCKS + Fa for every Fa <= F
     const size_t pw = (size_t)SEG_PART_WIDTH(F);
-    const int nq = 48;                    // the widest reduction: blml_seg_dots' 48 accumulators
+    const int nq = SEG_DOTS2_ROWS;        // the widest reduction: the history scan
     const int hs = 2 * m + 3;
     double* scr = (double*)r->dalloc(sizeof(double) * (nq * pw + (size_t)F * (2 * hs + (LB_T1 + 4) + LB_T2 + 1 + 2 + 2 +
-                                                                             (1 + 2 * m) + 1 + 2 + 3 + 2 + 1 + 1 + 1 +
-                                                                             1)));
+                                                                             (1 + 2 * m) + 1 + 1 + 1 + 1)));
     double* stt = (double*)r->dalloc(sizeof(double) * (size_t)F * (7 + (LB_FWIN + 1) + 2 * (size_t)m * m));
     int* ist = (int*)r->dalloc(sizeof(int) * ((size_t)F * (8 + m) + 1));
     r->split = (int*)r->dalloc(sizeof(int) * (size_t)seg_split_ints(F));   // >= seg_split_ints(Fa) for Fa <= F
@@ -1173,8 +1262,8 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
       double* x = scr + nq * pw;
       auto take = [&](size_t k) { double* p = x; x += k * F; return p; };
       r->H1 = take(hs); r->H2 = take(hs); r->T1 = take(LB_T1 + 4); r->T2 = take(LB_T2); r->outC = take(1);
-      r->outD = take(2); r->outE = take(2); r->cq = take(1 + 2 * m); r->tA = take(1); r->cS = take(2);
-      r->cY = take(3); r->cG = take(2); r->nqA = take(1); r->scrA = take(1); r->ones = take(1); r->sc = take(1);
+      r->outD = take(2); r->outE = take(2); r->cq = take(1 + 2 * m); r->tA = take(1);
+      r->nqA = take(1); r->scrA = take(1); r->sc = take(1);
       double* y = stt;
       auto tk = [&](size_t k) { double* p = y; y += k * F; return p; };
       r->s.L = tk(1); r->s.Q = tk(1); r->s.Qn = tk(1); r->s.n = tk(1); r->s.res = tk(1); r->s.slope = tk(1);
@@ -1186,7 +1275,6 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
       r->need2 = ti(1); ti(1);
       r->s.stamp = ti(m); r->s.step = z;
       cudaMemsetAsync(r->s.stamp, 0xff, sizeof(int) * (size_t)F * m, r->st);     // -1: no pair
-      k_fill_double<<<nblk(F, 256), 256, 0, r->st>>>(r->ones, F, 1.0);
       rc = cuda_status(cudaMemcpyAsync(r->s.n, n, F * sizeof(double), cudaMemcpyHostToDevice, r->st), "lbfgs n");
       if (!rc) rc = cuda_status(cudaStreamSynchronize(r->st), "lbfgs create");
     }

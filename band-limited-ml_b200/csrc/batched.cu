@@ -158,7 +158,7 @@ __global__ void k_seg_dots(const blml_seg* segs, int cplx, int np, SegPairs pp, 
   seg_partials<NP>(v, part);
 }
 
-struct SegList { const void* a[20]; };
+struct SegList { const void* a[40]; };              // a second list from 20 on
 
 // the history scan of the batched L-BFGS: per fit, for the np <= 20 vectors a_q, out = [a_q . b0 (np), a_q . b1 (np),
 // b0 . b0, b1 . b1, x . x] (x may be null: 0); b0, b1, x read once per element whatever np is
@@ -193,89 +193,103 @@ __global__ void __launch_bounds__(256) k_seg_dots2(const blml_seg* segs, int cpl
 // the same scan for float64 complex vectors, one (re, im) load per element and vector -- the stored vectors (TA)
 // and the first shared one (TB0) complex128 (the plain fits' history; the float32 history has its own scan,
 // k_seg_dots2_h32, with twice the elements per thread and a block split by fit size). The block's 8 warps
-// split the stored vectors (warp w takes q = w, w + 8, w + 16) and walk the same 64-element tiles, so each thread
+// split the stored vectors and walk the same 64-element tiles, so each thread
 // holds at most 6 accumulators (full occupancy, many loads in flight) and the two shared vectors are read from HBM
 // once per tile and from L1 by the other warps; the last warp also sums the three squared norms. Each quantity's
 // block partial comes from one warp (warp_sum, fixed order), in seg_partials' layout.
 // The stored vectors are those of the mask's slots, the i-th of them for warp i mod 8 (a slot's sum does not depend on
 // which warp forms it): the first iterations of a fit, whose memory is still filling, read only what it holds. 64 fits of
-// rank 4 over their first 12 iterations (20 slots): 12.9 ms of scans -> 9.3.
-__device__ __forceinline__ int nth_slot(unsigned on, int i) {
+// rank 4 over their first 12 iterations (20 slots): 12.9 ms of scans -> 9.3, -> 7.1 with both lists (S and Y) in one scan.
+__device__ __forceinline__ int nth_slot(unsigned long long on, int i) {
   for (; i > 0 && on; i--) on &= on - 1;
-  return __ffs(on) - 1;
+  return __ffsll((long long)on) - 1;
 }
+// the slots of both lists that the scan covers (bit q, and 20 + q of the second list)
+__device__ __forceinline__ unsigned long long slots_on(const HistMask& hm, int j, int np, bool two) {
+  const int q = threadIdx.x & 31;
+  const unsigned long long b = __ballot_sync(0xffffffffu, q < np && hm.on(j, q));
+  return two ? b | b << 20 : b;
+}
+// the partials' row of slot s: its product with b0; the one with b1 is 20 rows on
+__device__ __forceinline__ int slot_row(int s) { return s < 20 ? s : 23 + s; }
 
 // one complex128 element as (re, im)
 __device__ __forceinline__ double2 ld_c2(const double2* p) { return __ldg(p); }
 
-template <typename TA, typename TB0>
-__global__ void __launch_bounds__(256, 3) k_seg_dots2_c128(const blml_seg* segs, int np, SegList al, const void* b0,
-                                                           const void* b1, const void* x, double* part, HistMask hm) {
+__global__ void __launch_bounds__(256, 3) k_seg_dots2_c128(const blml_seg* segs, int np, int two, SegList al,
+                                                           const void* b0, const void* b1, const void* x, double* part,
+                                                           HistMask hm) {
   const blml_seg S = segs[blockIdx.y];
   const int64_t o = S.off, n = (int64_t)S.K * S.B;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const unsigned on = __ballot_sync(0xffffffffu, lane < np && hm.on(blockIdx.y, lane));
-  const TB0* B0 = reinterpret_cast<const TB0*>(b0) + o;
+  const unsigned long long on = slots_on(hm, blockIdx.y, np, two);
+  const int total = __popcll(on);
+  const double2* B0 = reinterpret_cast<const double2*>(b0) + o;
   const double2* B1 = reinterpret_cast<const double2*>(b1) + o;
   const double2* X = x ? reinterpret_cast<const double2*>(x) + o : nullptr;
-  const TA* A[3];
-  int na = 0, qs_[3];
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    qs_[j] = nth_slot(on, warp + nw * j);
-    A[j] = qs_[j] >= 0 ? reinterpret_cast<const TA*>(al.a[qs_[j]]) + o : nullptr;
-    na += qs_[j] >= 0;
-  }
-  const bool norms = warp == nw - 1;
-  double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
-  const double2 zero = make_double2(0.0, 0.0);
-  for (int64_t t = (int64_t)blockIdx.x * 64; t < n && (na || norms); t += (int64_t)gridDim.x * 64) {
-    // both elements' loads issued together: out-of-range lanes read element 0 and zero its shared values, so their
-    // products and norms add nothing
-    const int64_t i0 = t + lane, i1 = t + 32 + lane;
-    const bool v0 = i0 < n, v1 = i1 < n;
-    const int64_t j0 = v0 ? i0 : 0, j1 = v1 ? i1 : 0;
-    double2 y00 = ld_c2(B0 + j0), y01 = ld_c2(B0 + j1), y10 = __ldg(B1 + j0), y11 = __ldg(B1 + j1);
-    double2 a[3][2];
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-      if (j < na) { a[j][0] = ld_c2(A[j] + j0); a[j][1] = ld_c2(A[j] + j1); }
-    double2 z0 = zero, z1 = zero;
-    if (norms && X) { z0 = __ldg(X + j0); z1 = __ldg(X + j1); }
-    if (!v0) { y00 = zero; y10 = zero; z0 = zero; }
-    if (!v1) { y01 = zero; y11 = zero; z1 = zero; }
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-      if (j < na) {
-        a0[j] += a[j][0].x * y00.x + a[j][0].y * y00.y; a1[j] += a[j][0].x * y10.x + a[j][0].y * y10.y;
-        a0[j] += a[j][1].x * y01.x + a[j][1].y * y01.y; a1[j] += a[j][1].x * y11.x + a[j][1].y * y11.y;
-      }
-    if (norms) {
-      n0 += y00.x * y00.x + y00.y * y00.y; n1 += y10.x * y10.x + y10.y * y10.y; nx += z0.x * z0.x + z0.y * z0.y;
-      n0 += y01.x * y01.x + y01.y * y01.y; n1 += y11.x * y11.x + y11.y * y11.y; nx += z1.x * z1.x + z1.y * z1.y;
-    }
-  }
   const int64_t slot = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, qs = (int64_t)gridDim.y * gridDim.x;
+  const double2 zero = make_double2(0.0, 0.0);
+  // three vectors per warp and pass over the block's tiles
+  for (int first = 0; first == 0 || first < total; first += 3 * nw) {
+    const double2* A[3];
+    int na = 0, sl[3];
 #pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
-    if (j < na && lane == 0) {
-      const int q = qs_[j];
-      part[q * qs + slot] = s0; part[(20 + q) * qs + slot] = s1;
+    for (int j = 0; j < 3; j++) {
+      sl[j] = nth_slot(on, first + warp + nw * j);
+      A[j] = sl[j] >= 0 ? reinterpret_cast<const double2*>(al.a[sl[j]]) + o : nullptr;
+      na += sl[j] >= 0;
     }
-  }
-  if (norms) {
-    n0 = warp_sum(n0); n1 = warp_sum(n1); nx = warp_sum(nx);
-    if (lane == 0) { part[40 * qs + slot] = n0; part[41 * qs + slot] = n1; part[42 * qs + slot] = nx; }
+    const bool norms = first == 0 && warp == nw - 1;
+    double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
+    for (int64_t t = (int64_t)blockIdx.x * 64; t < n && (na || norms); t += (int64_t)gridDim.x * 64) {
+      // both elements' loads issued together: out-of-range lanes read element 0 and zero its shared values, so their
+      // products and norms add nothing
+      const int64_t i0 = t + lane, i1 = t + 32 + lane;
+      const bool v0 = i0 < n, v1 = i1 < n;
+      const int64_t j0 = v0 ? i0 : 0, j1 = v1 ? i1 : 0;
+      double2 y00 = ld_c2(B0 + j0), y01 = ld_c2(B0 + j1), y10 = __ldg(B1 + j0), y11 = __ldg(B1 + j1);
+      double2 a[3][2];
+#pragma unroll
+      for (int j = 0; j < 3; j++)
+        if (j < na) { a[j][0] = ld_c2(A[j] + j0); a[j][1] = ld_c2(A[j] + j1); }
+      double2 z0 = zero, z1 = zero;
+      if (norms && X) { z0 = __ldg(X + j0); z1 = __ldg(X + j1); }
+      if (!v0) { y00 = zero; y10 = zero; z0 = zero; }
+      if (!v1) { y01 = zero; y11 = zero; z1 = zero; }
+#pragma unroll
+      for (int j = 0; j < 3; j++)
+        if (j < na) {
+          a0[j] += a[j][0].x * y00.x + a[j][0].y * y00.y; a1[j] += a[j][0].x * y10.x + a[j][0].y * y10.y;
+          a0[j] += a[j][1].x * y01.x + a[j][1].y * y01.y; a1[j] += a[j][1].x * y11.x + a[j][1].y * y11.y;
+        }
+      if (norms) {
+        n0 += y00.x * y00.x + y00.y * y00.y; n1 += y10.x * y10.x + y10.y * y10.y; nx += z0.x * z0.x + z0.y * z0.y;
+        n0 += y01.x * y01.x + y01.y * y01.y; n1 += y11.x * y11.x + y11.y * y11.y; nx += z1.x * z1.x + z1.y * z1.y;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
+      if (j < na && lane == 0) {
+        const int q = slot_row(sl[j]);
+        part[q * qs + slot] = s0; part[(20 + q) * qs + slot] = s1;
+      }
+    }
+    if (norms) {
+      n0 = warp_sum(n0); n1 = warp_sum(n1); nx = warp_sum(nx);
+      if (lane == 0) { part[40 * qs + slot] = n0; part[41 * qs + slot] = n1; part[42 * qs + slot] = nx; }
+    }
   }
 }
 
 // out[f * (2 np + 3) + q] from the 43-quantity partials (quantities 20.. shifted down when np < 20)
-__global__ void k_seg_finish_dots2(const double* part, int np, int nblk, double* out, HistMask hm) {
-  const int f = blockIdx.x, F = gridDim.x, nq = 2 * np + 3;
+__global__ void k_seg_finish_dots2(const double* part, int np, int nblk, double* out_, double* out2, HistMask hm) {
+  // blockIdx.y = 1: the second list's products
+  double* out = blockIdx.y ? out2 : out_;
+  const int f = blockIdx.x, F = gridDim.x, nq = 2 * np + 3, row0 = blockIdx.y ? 43 : 0;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int q = wid; q < nq; q += nw) {
-    const int src = q < np ? q : (q < 2 * np ? 20 + (q - np) : 40 + (q - 2 * np));
+    const int src = q < np ? row0 + q : (q < 2 * np ? row0 + 20 + (q - np) : 40 + (q - 2 * np));
     double acc = 0.0;
     if (q >= 2 * np || hm.on(f, q % np))
       for (int i = lane; i < nblk; i += 32) acc += part[((int64_t)src * F + f) * nblk + i];
@@ -419,12 +433,13 @@ __device__ __forceinline__ void h32_tile(int64_t t, int64_t n, int lane, const f
   }
 }
 
-__global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, const int* split, int F, int np,
+__global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, const int* split, int F, int np, int two,
                                                           SegList al, const float2* b0, const double2* b1,
                                                           const double2* x, double* part, HistMask hm) {
   const int b = blockIdx.x, W = gridDim.x, f = split[F + 1 + b];
   if (f < 0) return;
-  const unsigned on = __ballot_sync(0xffffffffu, (threadIdx.x & 31) < np && hm.on(f, threadIdx.x & 31));
+  const unsigned long long on = slots_on(hm, f, np, two);
+  const int total = __popcll(on);
   const int lb = b - split[f], nb = split[f + 1] - split[f];
   const blml_seg S = segs[f];
   const int64_t o = S.off, n = (int64_t)S.K * S.B;
@@ -432,43 +447,47 @@ __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, 
   const float2* B0 = b0 + o;
   const double2* B1 = b1 + o;
   const double2* X = x ? x + o : nullptr;
-  const float2* A[3];
-  int na = 0, qs_[3];
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    qs_[j] = nth_slot(on, warp + nw * j);
-    A[j] = qs_[j] >= 0 ? reinterpret_cast<const float2*>(al.a[qs_[j]]) + o : nullptr;
-    na += qs_[j] >= 0;
-  }
-  const bool norms = warp == nw - 1;
-  double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
   constexpr int64_t T = 128;
   const int64_t stride = (int64_t)nb * T;
-  int64_t t = (int64_t)lb * T;
-  if (!na && !norms) t = n;
-  for (; t + T <= n; t += stride) h32_tile<false>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
-  for (; t < n; t += stride) h32_tile<true>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
+  for (int first = 0; first == 0 || first < total; first += 3 * nw) {
+    const float2* A[3];
+    int na = 0, sl[3];
 #pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
-    if (j < na && lane == 0) {
-      const int q = qs_[j];
-      part[(int64_t)q * W + b] = s0; part[(int64_t)(20 + q) * W + b] = s1;
+    for (int j = 0; j < 3; j++) {
+      sl[j] = nth_slot(on, first + warp + nw * j);
+      A[j] = sl[j] >= 0 ? reinterpret_cast<const float2*>(al.a[sl[j]]) + o : nullptr;
+      na += sl[j] >= 0;
     }
-  }
-  if (norms) {
-    n0 = warp_sum(n0); n1 = warp_sum(n1); nx = warp_sum(nx);
-    if (lane == 0) { part[40LL * W + b] = n0; part[41LL * W + b] = n1; part[42LL * W + b] = nx; }
+    const bool norms = first == 0 && warp == nw - 1;
+    double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
+    int64_t t = (int64_t)lb * T;
+    if (!na && !norms) t = n;
+    for (; t + T <= n; t += stride) h32_tile<false>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
+    for (; t < n; t += stride) h32_tile<true>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
+      if (j < na && lane == 0) {
+        const int q = slot_row(sl[j]);
+        part[(int64_t)q * W + b] = s0; part[(int64_t)(20 + q) * W + b] = s1;
+      }
+    }
+    if (norms) {
+      n0 = warp_sum(n0); n1 = warp_sum(n1); nx = warp_sum(nx);
+      if (lane == 0) { part[40LL * W + b] = n0; part[41LL * W + b] = n1; part[42LL * W + b] = nx; }
+    }
   }
 }
 
 // out[f * (2 np + 3) + q] from a split scan's partials: fit f's blocks [bstart[f], bstart[f + 1]), fixed order
-__global__ void k_seg_finish_dots2_split(const double* part, int W, const int* split, int np, double* out, HistMask hm) {
-  const int f = blockIdx.x, nq = 2 * np + 3;
+__global__ void k_seg_finish_dots2_split(const double* part, int W, const int* split, int np, double* out_, double* out2,
+                                         HistMask hm) {
+  double* out = blockIdx.y ? out2 : out_;
+  const int f = blockIdx.x, nq = 2 * np + 3, row0 = blockIdx.y ? 43 : 0;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int b0 = split[f], b1 = split[f + 1];
   for (int q = wid; q < nq; q += nw) {
-    const int src = q < np ? q : (q < 2 * np ? 20 + (q - np) : 40 + (q - 2 * np));
+    const int src = q < np ? row0 + q : (q < 2 * np ? row0 + 20 + (q - np) : 40 + (q - 2 * np));
     double acc = 0.0;
     if (q >= 2 * np || hm.on(f, q % np))
       for (int i = b0 + lane; i < b1; i += 32) acc += part[(int64_t)src * W + i];
@@ -878,33 +897,43 @@ int seg_split(int F, const blml_seg* segs, int* split, cudaStream_t st) {
   return BLML_OK;
 }
 
-int seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, const void* const* a, const void* b0,
-              const void* b1, const void* x, double* part, double* out, HistMask hm, cudaStream_t st) {
-  SegList al;
-  for (int q = 0; q < 20; q++) al.a[q] = q < np ? a[q] : nullptr;
+int seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, const void* const* a, const void* const* a2,
+              const void* b0, const void* b1, const void* x, double* part, double* out, double* out2, HistMask hm,
+              cudaStream_t st) {
   const int nb = seg_blocks_for(F);
   const dim3 g((unsigned)nb, (unsigned)F);
-  if (dtype == BLML_F64 && cplx)
-    k_seg_dots2_c128<double2, double2><<<g, 256, 0, st>>>(segs, np, al, b0, b1, x, part, hm);
-  else if (dtype == BLML_F64) k_seg_dots2<double><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
-  else k_seg_dots2<float><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
-  BLML_CHECK_LAUNCH("blml_seg_dots2");
-  k_seg_finish_dots2<<<F, 256, 0, st>>>(part, np, nb, out, hm);
-  BLML_CHECK_LAUNCH("blml_seg_dots2 finish");
+  const bool one = dtype == BLML_F64 && cplx;              // both lists in one scan; the general kernel takes one
+  for (int h = 0; h < (a2 && !one ? 2 : 1); h++) {
+    SegList al{};
+    for (int q = 0; q < np; q++) { al.a[q] = h ? a2[q] : a[q]; if (one && a2) al.a[20 + q] = a2[q]; }
+    if (one) k_seg_dots2_c128<<<g, 256, 0, st>>>(segs, np, a2 != nullptr, al, b0, b1, x, part, hm);
+    else if (dtype == BLML_F64) k_seg_dots2<double><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
+    else k_seg_dots2<float><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
+    BLML_CHECK_LAUNCH("blml_seg_dots2");
+    k_seg_finish_dots2<<<dim3(F, one && a2 ? 2 : 1), 256, 0, st>>>(part, np, nb, h ? out2 : out, out2, hm);
+    BLML_CHECK_LAUNCH("blml_seg_dots2 finish");
+  }
   return BLML_OK;
 }
 
-int seg_dots2_h32(int F, const blml_seg* segs, const int* split, int np, const void* const* a, const void* b0,
-                  const void* b1, const void* x, double* part, double* out, HistMask hm, cudaStream_t st) {
+int seg_dots2_h32(int F, const blml_seg* segs, const int* split, int np, const void* const* a, const void* const* a2,
+                  const void* b0, const void* b1, const void* x, double* part, double* out, double* out2, HistMask hm,
+                  cudaStream_t st) {
   if (np < 1 || np > 20 || !a || !b0 || !b1) { set_error("history scan: 1..20 vectors, b0 and b1"); return BLML_ERR_ARG; }
-  SegList al;
-  for (int q = 0; q < 20; q++) al.a[q] = q < np ? a[q] : nullptr;
+  SegList al{};
+  for (int q = 0; q < np; q++) { al.a[q] = a[q]; if (a2) al.a[20 + q] = a2[q]; }
   const int W = SEG_SPLIT_BLOCKS + F;
-  k_seg_dots2_h32<<<W, 256, 0, st>>>(segs, split, F, np, al, (const float2*)b0, (const double2*)b1,
+  k_seg_dots2_h32<<<W, 256, 0, st>>>(segs, split, F, np, a2 != nullptr, al, (const float2*)b0, (const double2*)b1,
                                      (const double2*)x, part, hm);
   BLML_CHECK_LAUNCH("history scan (float32 history)");
-  k_seg_finish_dots2_split<<<F, 256, 0, st>>>(part, W, split, np, out, hm);
+  k_seg_finish_dots2_split<<<dim3(F, a2 ? 2 : 1), 256, 0, st>>>(part, W, split, np, out, out2, hm);
   BLML_CHECK_LAUNCH("history scan finish");
+  return BLML_OK;
+}
+
+int seg_finish_resid(int F, const double* part, double* out, cudaStream_t st) {
+  k_seg_finish<<<F, 256, 0, st>>>(part, 2, seg_blocks_for(F), 1u, out);
+  BLML_CHECK_LAUNCH("residual finish");
   return BLML_OK;
 }
 
@@ -1008,7 +1037,7 @@ int blml_seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, con
                    const void* b1, const void* x, double* part, double* out, void* stream) {
   if (seg_args(dtype, F, segs, "blml_seg_dots2")) return BLML_ERR_ARG;
   if (np < 1 || np > 20 || !a || !b0 || !b1) { set_error("blml_seg_dots2: 1..20 vectors, b0 and b1"); return BLML_ERR_ARG; }
-  return seg_dots2(dtype, F, segs, cplx, np, a, b0, b1, x, part, out, HistMask{}, SST);
+  return seg_dots2(dtype, F, segs, cplx, np, a, nullptr, b0, b1, x, part, out, nullptr, HistMask{}, SST);
 }
 
 int blml_seg_lincomb(int dtype, int F, const blml_seg* segs, int cplx, void* out, int nterms, const double* coef,
@@ -1174,7 +1203,7 @@ int blml_seg_dots2_h32(int F, const blml_seg* segs, int* split, int np, const vo
     set_error("blml_seg_dots2_h32: bad arguments"); return BLML_ERR_ARG;
   }
   if (seg_split(F, segs, split, SST)) return BLML_ERR_CUDA;
-  return seg_dots2_h32(F, segs, split, np, a, b0, b1, x, part, out, HistMask{}, SST);
+  return seg_dots2_h32(F, segs, split, np, a, nullptr, b0, b1, x, part, out, nullptr, HistMask{}, SST);
 }
 
 int64_t blml_seg_split_ints(int F) { return F < 1 ? 0 : seg_split_ints(F); }

@@ -39,10 +39,16 @@ struct HistMask {
 };
 
 // the L-BFGS runner's history scans (batched.cu): state of dtype, or complex64 storage (split: seg_split's output)
-int seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, const void* const* a, const void* b0,
-              const void* b1, const void* x, double* part, double* out, HistMask hm, cudaStream_t st);
-int seg_dots2_h32(int F, const blml_seg* segs, const int* split, int np, const void* const* a, const void* b0,
-                  const void* b1, const void* x, double* part, double* out, HistMask hm, cudaStream_t st);
+// out: blml_seg_dots2's quantities of the vectors a; out2 (or null): those of a second list a2 of as many
+int seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, const void* const* a, const void* const* a2,
+              const void* b0, const void* b1, const void* x, double* part, double* out, double* out2, HistMask hm,
+              cudaStream_t st);
+int seg_dots2_h32(int F, const blml_seg* segs, const int* split, int np, const void* const* a, const void* const* a2,
+                  const void* b0, const void* b1, const void* x, double* part, double* out, double* out2, HistMask hm,
+                  cudaStream_t st);
+// the two quantities of blml_seg_resid from their partials
+int seg_finish_resid(int F, const double* part, double* out, cudaStream_t st);
+constexpr int SEG_DOTS2_ROWS = 83;         // partials per block: two lists of 20 twice, three norms
 int seg_lincomb_mixed(int F, const blml_seg* segs, const int* split, void* out, int out_f32, int nterms,
                       const double* coef, const void* const* v, unsigned long long f32mask, cudaStream_t st);
 
@@ -62,9 +68,10 @@ struct SAcc {
                              b += (int64_t)gridDim.x * blockDim.x)
 
 // partials layout, quantity-major so it does not depend on how many accumulators a kernel carries:
-// part[((q * F) + f) * gridDim.x + blockIdx.x], F = gridDim.y fits
+// part[((q * F) + j) * nblk + bx] for block bx of the nblk blocks of row j of F
 template <int NQ>
-__device__ __forceinline__ void seg_partials(double (&v)[NQ], double* part, unsigned maxmask = 0u) {
+__device__ __forceinline__ void seg_partials_at(double (&v)[NQ], double* part, unsigned maxmask, int F, int j, int nblk,
+                                                int bx) {
   __shared__ double sh[NQ][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
@@ -79,8 +86,30 @@ __device__ __forceinline__ void seg_partials(double (&v)[NQ], double* part, unsi
       const bool mx = (maxmask >> q) & 1u;
       double x = lane < nw ? sh[q][lane] : (mx ? -INFINITY : 0.0);
       x = mx ? warp_max(x) : warp_sum(x);
-      if (lane == 0) part[((int64_t)q * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = x;
+      if (lane == 0) part[((int64_t)q * F + j) * nblk + bx] = x;
     }
+  }
+}
+
+template <int NQ>
+__device__ __forceinline__ void seg_partials(double (&v)[NQ], double* part, unsigned maxmask = 0u) {
+  seg_partials_at<NQ>(v, part, maxmask, gridDim.y, blockIdx.y, gridDim.x, blockIdx.x);
+}
+
+// body(j, bx) for the nblk blocks bx of every row j whose flag is set, shared out among the launch's blocks: a launch of
+// nblk blocks for each of F rows costs 25 to 40 us of blocks that leave at once when few flags or none are set
+constexpr int SEG_FLAGGED_BLOCKS = 148 * 3;
+template <typename Body>
+__device__ __forceinline__ void seg_flagged(const int* flag, int F, int nblk, Body body) {
+  int64_t base = 0;
+  for (int j = 0; j < F; j++) {
+    if (!flag[j]) continue;
+    const int64_t g = gridDim.x, d = (int64_t)blockIdx.x - base % g;
+    for (int64_t i = d < 0 ? d + g : d; i < nblk; i += g) {
+      body(j, (int)i);
+      __syncthreads();                     // seg_partials_at's shared memory
+    }
+    base += nblk;
   }
 }
 
