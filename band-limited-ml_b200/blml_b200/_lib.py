@@ -124,6 +124,7 @@ _SIGS = {
     'blml_seg_dots2_h32': (_I, [_I, _P, _P, _I, _P, _P, _P, _P, _P, _P, _P]),
     'blml_seg_split_ints': (_L, [_I]),
     'blml_seg_lincomb_h32': (_I, [_I, _P, _P, _P, _I, _I, _P, _P, C.c_uint64, _P]),
+    'blml_lanczos_check': (_I, [_I, _P, _I, _P, _I, _P, _P, _P]),
     'blml_lanczos_step': (_I, [_I, _P, _P, _I, _P, _I, _P, _P, _L, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     'blml_lanczos_coef': (_I, [_I, _I, _P, _P, _P, _I, _P]),
     'blml_lanczos_beta': (_I, [_I, _P, _P, _P, _P]),

@@ -79,7 +79,7 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
     (blml_binned.py:501-518), D = sum_k |e_k|^2 / w on occupied bins, by float64 Lanczos with full
     reorthogonalisation, all fits in lockstep: one grouped mat-vec, segmented inner products and linear combinations
     per step with their coefficients formed on the device (no host round trip inside a step), each fit's tridiagonal
-    problem on the host (every third step, when alpha and beta are read back), restarts from the Ritz vector until
+    problem on the device too, looked at every third step while the next one runs, restarts from the Ritz vector until
     every fit's Ritz residual |beta_j y_j| <= tol |theta|, or its Ritz value moved by less than 1e-8 relative between
     two checks (at a certified optimum the top eigenvalue is K-fold, so the residual of its Ritz vector converges far
     more slowly than the value; 1e-8 is far below any certification bar). above: per-fit thresholds; a Ritz value is
@@ -171,8 +171,10 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
     coef_d = torch.empty(64 * F, dtype=torch.float64, device=dev)
     scale_d = torch.empty(F, dtype=torch.float64, device=dev)
     ab_d = torch.zeros((nb, 2, F), dtype=torch.float64, device=dev)
-    ab_h = torch.empty((nb, 2, F), dtype=torch.float64, pin_memory=True)
+    chk_h = torch.empty((F, 4), dtype=torch.float64, pin_memory=True)      # written by the checks themselves
+    chk = chk_h.numpy()
     part = torch.empty(64 * every.nblocks, dtype=torch.float64, device=dev)
+    work = torch.empty(4 * nb * F, dtype=torch.float64, device=dev)
     read = torch.cuda.Event()
 
     def step(S, j):
@@ -182,42 +184,48 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
 
     steps = 0
     for rnd in range(max_restarts + 1):
-        alphas = np.zeros((F, nb)); betas = np.zeros((F, nb))
-        conv = np.zeros(F, bool); yr = [None] * F; yr2 = [None] * F
+        conv = np.zeros(F, bool)
+        size = np.zeros(F, np.int64)                  # the steps each fit's last Ritz vector is made of
         S = every if not done.any() else Subset(np.where(~done)[0])
         j_end = nb
-        fetched = 0                                   # steps whose alpha / beta the host holds or has asked for
-        waiting = None                                # the step whose check is still to be made
+        waiting = None                                # the step whose check is still to be read
 
         def check(j):
-            """Every open fit's tridiagonal problem after step j; True when all have converged."""
+            """The open fits' Ritz values after step j; True when all have converged."""
             t0 = time.perf_counter()
             read.synchronize()
             clock['wait_s'] += time.perf_counter() - t0
-            t0 = time.perf_counter()
-            ab = ab_h.numpy()
             of = np.where(~(done | conv))[0]
-            alphas[of, :j + 1] = ab[:j + 1, 0, of].T
-            betas[of, :j + 1] = ab[:j + 1, 1, of].T
-            beta = betas[:, j]
-            # the largest eigenpair of each T_f (j + 1 square), all at once
-            T = np.zeros((len(of), j + 1, j + 1))
-            ii = np.arange(j + 1)
-            T[:, ii, ii] = alphas[of, :j + 1]
-            T[:, ii[:-1], ii[1:]] = betas[of, :j]
-            T[:, ii[1:], ii[:-1]] = betas[of, :j]
-            ev_all, evec_all = np.linalg.eigh(T)
-            for t_, f in enumerate(of):
-                th = float(ev_all[t_, -1]); y = evec_all[t_, :, -1].copy()
-                theta[f] = th; yr[f] = y
-                if j > 0:
-                    yr2[f] = evec_all[t_, :, -2].copy(); theta2[f] = float(ev_all[t_, -2])
-                if (abs(beta[f] * y[-1]) <= tol * max(abs(th), 1e-300) or beta[f] <= 1e-14 * max(abs(th), 1e-300)
-                        or th > above[f] or abs(th - prev[f]) <= 1e-8 * abs(th)):
-                    conv[f] = True
-                prev[f] = th
-            clock['host_s'] += time.perf_counter() - t0
+            th, th2, y, beta = chk[of].T
+            if np.isnan(th).any():
+                raise np.linalg.LinAlgError("Eigenvalues did not converge")
+            theta[of] = th; size[of] = j + 1
+            if j > 0:
+                theta2[of] = th2
+            bar = np.maximum(np.abs(th), 1e-300)
+            with np.errstate(invalid='ignore'):
+                conv[of] = ((np.abs(beta * y) <= tol * bar) | (beta <= 1e-14 * bar) | (th > above[of]) |
+                            (np.abs(th - prev[of]) <= 1e-8 * np.abs(th)))
+            prev[of] = th
             return bool(np.all(done | conv))
+
+        def ritz():
+            """Every open fit's top two Ritz vectors in its Krylov basis, from its steps' alpha and beta."""
+            ab = ab_d[:j_end].cpu().numpy()
+            yr, yr2 = [None] * F, [None] * F
+            for n in np.unique(size[~done]):
+                of = np.where(~done & (size == n))[0]
+                if n == 0:
+                    continue
+                T = np.zeros((len(of), n, n))
+                ii = np.arange(n)
+                T[:, ii, ii] = ab[:n, 0, of].T
+                T[:, ii[:-1], ii[1:]] = T[:, ii[1:], ii[:-1]] = ab[:n - 1, 1, of].T
+                vec_all = np.linalg.eigh(T)[1]
+                for t_, f in enumerate(of):
+                    yr[f] = vec_all[t_, :, -1]
+                    yr2[f] = vec_all[t_, :, -2] if n > 1 else None
+            return yr, yr2
 
         for j in range(nb):
             step(S, j)
@@ -232,14 +240,20 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
                     # the steps go on over the open fits only; the converged ones keep V[0..pj], all their Ritz vectors use
                     S = Subset(still)
             if j == nb - 1 or (j >= 5 and j % 3 == 2):
-                ab_h[fetched:j + 1].copy_(ab_d[fetched:j + 1], non_blocking=True)
+                call('blml_lanczos_check', len(S.idx), S.fid, F, ab_d.data_ptr(), j, work.data_ptr(),
+                     chk_h.data_ptr(), st)
                 read.record(torch.cuda.current_stream(dev))
-                fetched = j + 1
                 waiting = j
                 if j == nb - 1:
                     check(j)
         # the Ritz vector of every fit still open at the start of this round: R = sum_i y_i V[i]
         act = ~done
+        if not vectors and np.all(done | conv):                   # no one asks for them
+            done |= conv
+            break
+        t0 = time.perf_counter()
+        yr, yr2 = ritz()
+        clock['host_s'] += time.perf_counter() - t0
         SA = every if act.all() else Subset(np.where(act)[0])
         R.zero_()
         for c0 in range(0, j_end, 47):

@@ -219,6 +219,124 @@ __global__ void __launch_bounds__(LZ_T) k_lz_sub(LzArgs A, const double* __restr
   }
 }
 
+// The two largest eigenvalues of each row's tridiagonal matrix (n square) and the last component of the top eigenvector.
+// One warp a row. An eigenvalue by multisection with Sturm counts: each lane counts the eigenvalues above one of 32 points
+// of the bracket from the signs of the leading minors p_k = (a_k - x) p_{k-1} - b_{k-1}^2 p_{k-2}, five bits a round. The
+// last component from the twisted factorisation of T - theta (Dhillon and Parlett): the pivots d_k from the top and u_k
+// from the bottom, the twist m at the smallest |d_m + u_m - (a_m - theta)|, y_m = 1, ratios b_k / d_k above and
+// b_k / u_{k+1} below it; from the top alone it is lost where the vector has died out before the last step.
+// Bound: the chain of n dependent multiply-adds a round (78 us for 64 fits at up to 64 square, behind which the next
+// step is queued), where the host took 0.75 ms for the full decompositions, mostly with the GPU idle.
+struct LzMat { const double* a; const double* b; int sa; int n; double inv; };     // entries sa apart, scaled by inv
+
+__device__ __forceinline__ int lz_above(const LzMat& M, double x) {
+  double p1 = 1.0, p = M.a[0] * M.inv - x;
+  if (p == 0.0) p = -1e-290;
+  int c = p > 0.0;
+  for (int k = 1; k < M.n; k++) {
+    const double b = M.b[(int64_t)(k - 1) * M.sa] * M.inv;
+    double q = fma(M.a[(int64_t)k * M.sa] * M.inv - x, p, -(b * b) * p1);
+    if (q == 0.0) q = p > 0.0 ? -1e-290 : 1e-290;
+    c += (q > 0.0) == (p > 0.0);
+    p1 = p; p = q;
+    if ((k & 7) == 0) {                                   // back to order one (a power of two: exact)
+      const double f = ldexp(1.0, -ilogb(fmax(fabs(p), fabs(p1))));
+      p *= f; p1 *= f;
+    }
+  }
+  return c;
+}
+
+// the largest x with at least `want` eigenvalues above it, in [lo, hi]
+__device__ double lz_section(const LzMat& M, int want, double lo, double hi) {
+  const int lane = threadIdx.x & 31;
+  for (int r = 0; r < 16 && hi - lo > 2.3e-16 * fmax(fabs(lo), fabs(hi)); r++) {
+    const double w = (hi - lo) / 33.0, x = lo + w * (lane + 1);
+    const unsigned m = __ballot_sync(0xffffffffu, x > lo && x < hi && lz_above(M, x) >= want);
+    const int top = 31 - __clz((int)m);                   // -1: none
+    const double l = lo + w * (top + 1), h = lo + w * (top + 2);
+    if (top >= 0) lo = l;
+    if (top < 31 && h < hi) hi = h;
+  }
+  return 0.5 * (lo + hi);
+}
+
+constexpr int LZ_SHARED_N = 1024;
+__global__ void __launch_bounds__(32) k_lz_check(const int* fid, int stride, const double* ab, int j, double* work,
+                                                 double* out) {
+  __shared__ double as[LZ_SHARED_N], bs[LZ_SHARED_N];
+  const int f = fid[blockIdx.x], lane = threadIdx.x, n = j + 1;
+  const double *a = ab + f, *b = ab + stride + f;         // alpha_i, beta_i at i * 2 stride
+  LzMat M{a, b, 2 * stride, n, 1.0};
+  if (n <= LZ_SHARED_N) {
+    for (int i = lane; i < n; i += 32) { as[i] = a[(int64_t)i * M.sa]; bs[i] = b[(int64_t)i * M.sa]; }
+    M.a = as; M.b = bs; M.sa = 1;
+  }
+  __syncwarp();
+  double lo = INFINITY, hi = -INFINITY;                   // Gershgorin
+  bool bad = false;
+  for (int i = lane; i < n; i += 32) {
+    const double d = M.a[(int64_t)i * M.sa];
+    const double r = (i > 0 ? fabs(M.b[(int64_t)(i - 1) * M.sa]) : 0.0) + (i < n - 1 ? fabs(M.b[(int64_t)i * M.sa]) : 0.0);
+    lo = fmin(lo, d - r); hi = fmax(hi, d + r);
+    bad |= !isfinite(d) || !isfinite(r);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o)); hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  const double size = fmax(fabs(lo), fabs(hi));
+  double t1 = bad ? NAN : 0.0, t2 = bad || n == 1 ? NAN : 0.0, y = 1.0;       // (the zero matrix)
+  if (!bad && size > 0.0) {
+    M.inv = 1.0 / size;
+    const double pad = 4e-16, l = lo * M.inv - pad, h = hi * M.inv + pad;
+    t1 = lz_section(M, 1, l, h);
+    if (n > 1) t2 = lz_section(M, 2, l, h);
+    // lane 0 from the top, lane 1 from the bottom: pivots and the sums of (y_i / y_k)^2 up to k
+    double* W = work + 4 * (int64_t)n * blockIdx.x;
+    if (lane < 2) {
+      double S = 1.0, d = 0.0;
+      for (int k = 0; k < n; k++) {
+        const int i = lane ? n - 1 - k : k;
+        if (k == 0) d = M.a[(int64_t)i * M.sa] * M.inv - t1;
+        else {
+          const double bk = M.b[(int64_t)(lane ? i : i - 1) * M.sa] * M.inv;
+          if (fabs(d) < 1e-30) d = -1e-30;
+          const double r = bk / d;
+          S = 1.0 + r * r * S;
+          d = M.a[(int64_t)i * M.sa] * M.inv - t1 - bk * r;
+        }
+        W[(2 * lane) * n + i] = d; W[(2 * lane + 1) * n + i] = S;
+      }
+    }
+    __syncwarp();
+    double best = INFINITY;
+    int m = n - 1;
+    for (int i = lane; i < n; i += 32) {
+      const double g = fabs(W[i] + W[2 * n + i] - (M.a[(int64_t)i * M.sa] * M.inv - t1));
+      if (g < best) { best = g; m = i; }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double g = __shfl_xor_sync(0xffffffffu, best, o);
+      const int i = __shfl_xor_sync(0xffffffffu, m, o);
+      if (g < best || (g == best && i < m)) { best = g; m = i; }
+    }
+    y = 1.0;
+    for (int i = m + lane; i < n - 1; i += 32) {
+      double u = W[2 * n + i + 1];
+      if (fabs(u) < 1e-30) u = -1e-30;
+      y *= fabs(M.b[(int64_t)i * M.sa] * M.inv / u);
+    }
+    for (int o = 16; o > 0; o >>= 1) y *= __shfl_xor_sync(0xffffffffu, y, o);
+    y /= sqrt(W[n + m] + W[3 * n + m] - 1.0);
+    t1 *= size; t2 *= size;
+  }
+  if (lane == 0) {
+    double* o = out + 4 * (int64_t)f;
+    o[0] = t1; o[1] = t2; o[2] = y; o[3] = M.b[(int64_t)j * M.sa];
+  }
+}
+
 template <bool FIRST>
 static void lz_dots(int nblocks, cudaStream_t st, const LzArgs& A, const double* V, int64_t ldv, int nq, const double* sv,
                     const double* dh, double* w, double* alpha, int acol) {
@@ -283,6 +401,14 @@ int blml_lanczos_step(int F, const blml_seg* segs, const int* fid, int nblocks, 
       k_lz_sub<false><<<nblocks, LZ_T, 0, st>>>(A, Vq, ldv, nq, w, last ? beta : nullptr, last ? scale : nullptr);
       BLML_CHECK_LAUNCH("lanczos subtraction");
     }
+  return BLML_OK;
+}
+
+int blml_lanczos_check(int F, const int* fid, int stride, const double* alpha_beta, int j, double* work,
+                       double* out, void* stream) {
+  if (F < 1 || !fid || stride < 1 || !alpha_beta || j < 0 || !work || !out) { set_error("blml_lanczos_check: bad arguments"); return BLML_ERR_ARG; }
+  k_lz_check<<<F, 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(fid, stride, alpha_beta, j, work, out);
+  BLML_CHECK_LAUNCH("lanczos check");
   return BLML_OK;
 }
 

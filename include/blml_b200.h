@@ -320,6 +320,11 @@ int blml_lanczos_step(int F, const blml_seg* segs, const int* fid, int nblocks, 
                       blml_group group, double* V, int64_t ldv, int j, const double* dh, double* tmp, const double* sv,
                       double* w, double* part, int* counters, double* coef, double* alpha, double* beta, double* scale,
                       void* stream);
+/* After step j: out[4 fit ..] = the two largest eigenvalues of the fit's tridiagonal matrix (the second NaN for j = 0), the
+ * last component of the top eigenvector (its size) and beta_j; alpha_beta holds alpha_i, then beta_i, as rows of `stride`
+ * fits; work: 4 (j + 1) F doubles. The eigenvalues are NaN where an entry is not finite. out may be mapped host memory. */
+int blml_lanczos_check(int F, const int* fid, int stride, const double* alpha_beta, int j, double* work, double* out,
+                       void* stream);
 
 /* ---- batched solver phases with device-side control: the per-fit decisions of every
  *      iteration run as kernels, a ring of iterations is one CUDA graph replayed until every fit has stopped, the

@@ -93,3 +93,43 @@ def test_launches_over_any_number_of_fits(cuda_device):
         one = BLMLBinnedBatch(tol=1e-9, max_sweeps=2)
         one.fit(counts[i:i + 1], modes[i:i + 1])
         assert abs(one.certificate()[0] - both[i]) <= 1e-5 * abs(both[i])
+
+
+@pytest.mark.parametrize('n', [1, 2, 3, 6, 33, 64, 130, 1500])
+def test_check(cuda_device, n):
+    """The two top eigenvalues within 4 n eps of the largest in size, the last component (exact up to the eigenvalue's
+    error over the gap) within 1e-7, for random, graded, split, repeated and zero matrices, of some of the fits."""
+    from blml_b200 import _lib
+    rng = np.random.default_rng(n)
+    F = 7
+    a, b = rng.standard_normal((n, F)), np.abs(rng.standard_normal((n, F))) + 0.1
+    a[:, 1] *= 1e-150; b[:, 1] *= 1e-150
+    a[:, 2] = 1e5 * 0.5 ** np.arange(n); b[:, 2] = 1e3 * 0.5 ** np.arange(n)
+    b[n // 2, 3] = 0.0                                        # two blocks
+    a[:, 4] = 2.0; b[:, 4] = 1e-9                             # a cluster
+    a[:, 5] = 0.0; b[:, 5] = 0.0
+    a[:, 6] = np.abs(a[:, 6]) + 1e6                           # close to a multiple of the identity
+    ab = torch.as_tensor(np.stack([a, b], 1)).cuda()
+    rows = np.array([6, 0, 1, 2, 3, 4, 5], np.int32)[:7 if n % 2 else 6]
+    fid = torch.as_tensor(rows).cuda()
+    out = torch.full((F, 4), 9.0, dtype=torch.float64, device='cuda')
+    work = torch.empty(4 * n * F, dtype=torch.float64, device='cuda')
+    _lib.call('blml_lanczos_check', len(rows), fid.data_ptr(), F, ab.data_ptr(), n - 1, work.data_ptr(), out.data_ptr(),
+              torch.cuda.current_stream().cuda_stream)
+    got = out.cpu().numpy()
+    for f in range(F):
+        if f not in rows:
+            assert np.all(got[f] == 9.0)
+            continue
+        T = np.diag(a[:, f]) + np.diag(b[:-1, f], 1) + np.diag(b[:-1, f], -1)
+        ev, vec = np.linalg.eigh(T)
+        big = np.abs(ev).max()
+        assert abs(got[f, 0] - ev[-1]) <= 4 * n * 2.3e-16 * big + 1e-300
+        if n > 1:
+            assert abs(got[f, 1] - ev[-2]) <= 4 * n * 2.3e-16 * big + 1e-300
+        else:
+            assert np.isnan(got[f, 1]) or f == 5
+        assert got[f, 3] == b[n - 1, f]
+        gap = (ev[-1] - ev[-2]) / big if n > 1 and big > 0 else 1.0
+        if f not in (4, 5) and gap > 1e-6:
+            assert abs(got[f, 2] - abs(vec[-1, -1])) <= 1e-7
