@@ -569,29 +569,45 @@ __global__ void k_st_take(int Fa, int mA, const int* fid, const int* live, const
 // merit terms of E + a (E_J - E), U + a (U_J - U), formed as the linear-combination kernel forms them
 constexpr int DAMP_T1 = 4, DAMP_T2 = DAMP_NT - DAMP_T1;
 template <int NTG>
-__global__ void __launch_bounds__(256) k_st_damp_trials(const blml_seg* segs, const int* flag, int F, int nblk, int j0,
-                                                        const double* E, const double* EJ, const double* U,
-                                                        const double* UJ, const double* c, const double* sg,
-                                                        double* part) {
-  seg_flagged(flag, F, nblk, [&](int j, int bx) {
-    const blml_seg S = segs[j];
-    double v[3 * NTG];
+__device__ __forceinline__ void damp_trials(const blml_seg& S, int bx, int nblk, int j0, const double* E, const double* EJ,
+                                            const double* U, const double* UJ, const double* c, const double* sg,
+                                            double* v) {
+  const double a0 = ldexp(1.0, -(j0 + 1));
+  for (int64_t b = (int64_t)bx * blockDim.x + threadIdx.x; b < S.B; b += (int64_t)nblk * blockDim.x) {
+    const double e0 = E[S.off + b], e1 = EJ[S.off + b], u0 = U[S.off + b], u1 = UJ[S.off + b];
+    const double cb = c[S.boff + b], sgb = sg[S.boff + b];
+    double a = a0;
 #pragma unroll
-    for (int q = 0; q < 3 * NTG; q++) v[q] = 0.0;
-    const double a0 = ldexp(1.0, -(j0 + 1));
-    for (int64_t b = (int64_t)bx * blockDim.x + threadIdx.x; b < S.B; b += (int64_t)nblk * blockDim.x) {
-      const double e0 = E[S.off + b], e1 = EJ[S.off + b], u0 = U[S.off + b], u1 = UJ[S.off + b];
-      const double cb = c[S.boff + b], sgb = sg[S.boff + b];
-      double a = a0;
-#pragma unroll
-      for (int k = 0; k < NTG; k++) {
-        const double e = fma(a, e1, (1.0 - a) * e0), u = fma(a, u1, (1.0 - a) * u0);
-        v[3 * k] += e * u;
-        if (cb > 0) { v[3 * k + 1] += cb * log(fabs(e)); if (sgb * e <= 0) v[3 * k + 2] += 1.0; }
-        a *= 0.5;
-      }
+    for (int k = 0; k < NTG; k++) {
+      const double e = fma(a, e1, (1.0 - a) * e0), u = fma(a, u1, (1.0 - a) * u0);
+      v[3 * k] += e * u;
+      if (cb > 0) { v[3 * k + 1] += cb * log(fabs(e)); if (sgb * e <= 0) v[3 * k + 2] += 1.0; }
+      a *= 0.5;
     }
-    seg_partials_at<3 * NTG>(v, part, 0u, F, j, nblk, bx);
+  }
+}
+
+// the first trials, of most fits (64 fits: 65 us a launch, 112 when shared out), and the further ones, of few (105 -> 86)
+__global__ void __launch_bounds__(256) k_st_damp_trials(const blml_seg* segs, const int* flag, const double* E,
+                                                        const double* EJ, const double* U, const double* UJ,
+                                                        const double* c, const double* sg, double* part) {
+  if (!flag[blockIdx.y]) return;
+  double v[3 * DAMP_T1];
+#pragma unroll
+  for (int q = 0; q < 3 * DAMP_T1; q++) v[q] = 0.0;
+  damp_trials<DAMP_T1>(segs[blockIdx.y], blockIdx.x, gridDim.x, 0, E, EJ, U, UJ, c, sg, v);
+  seg_partials<3 * DAMP_T1>(v, part);
+}
+
+__global__ void __launch_bounds__(256) k_st_damp_more(const blml_seg* segs, const int* flag, int F, int nblk,
+                                                      const double* E, const double* EJ, const double* U,
+                                                      const double* UJ, const double* c, const double* sg, double* part) {
+  seg_flagged(flag, F, nblk, [&](int j, int bx) {
+    double v[3 * DAMP_T2];
+#pragma unroll
+    for (int q = 0; q < 3 * DAMP_T2; q++) v[q] = 0.0;
+    damp_trials<DAMP_T2>(segs[j], bx, nblk, DAMP_T1, E, EJ, U, UJ, c, sg, v);
+    seg_partials_at<3 * DAMP_T2>(v, part, 0u, F, j, nblk, bx);
   });
 }
 
@@ -1157,13 +1173,13 @@ struct blml_start_batch_s : Runner {
     k_st_lin2<<<grid, 256, 0, st>>>(S, 2, cT, Terms3{{EA, EJ, nullptr}}, ET, Terms3{{UA, UJ, nullptr}}, UT);
     KCHECK("start candidate");
     // damped steps: 4 trials, then 22 more for the fits none of the 4 served
-    k_st_damp_trials<DAMP_T1><<<SEG_FLAGGED_BLOCKS, 256, 0, st>>>(S, damp, Fa_, (int)grid.x, 0, E, EJ, U, UJ, c, sg, part);
+    k_st_damp_trials<<<grid, 256, 0, st>>>(S, damp, E, EJ, U, UJ, c, sg, part);
     KCHECK("start damping trials");
     k_finish_flagged<<<Fa_, 256, 0, st>>>(part, 3 * DAMP_T1, seg_blocks_for(Fa_), damp, outDT);
     KCHECK("start damping finish");
     k_st_damp_pick1<<<nblk(Fa_, 128), 128, 0, st>>>(Fa_, d_fid, d_live, damp, outDT, s, cE, need2d);
     KCHECK("start damping pick");
-    k_st_damp_trials<DAMP_T2><<<SEG_FLAGGED_BLOCKS, 256, 0, st>>>(S, need2d, Fa_, (int)grid.x, DAMP_T1, E, EJ, U, UJ, c, sg, part);
+    k_st_damp_more<<<SEG_FLAGGED_BLOCKS, 256, 0, st>>>(S, need2d, Fa_, (int)grid.x, E, EJ, U, UJ, c, sg, part);
     KCHECK("start damping trials");
     k_finish_flagged<<<Fa_, 256, 0, st>>>(part, 3 * DAMP_T2, seg_blocks_for(Fa_), need2d, outDT2);
     KCHECK("start damping finish");

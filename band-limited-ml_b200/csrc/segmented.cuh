@@ -96,20 +96,31 @@ __device__ __forceinline__ void seg_partials(double (&v)[NQ], double* part, unsi
   seg_partials_at<NQ>(v, part, maxmask, gridDim.y, blockIdx.y, gridDim.x, blockIdx.x);
 }
 
-// body(j, bx) for the nblk blocks bx of every row j whose flag is set, shared out among the launch's blocks: a launch of
-// nblk blocks for each of F rows costs 25 to 40 us of blocks that leave at once when few flags or none are set
-constexpr int SEG_FLAGGED_BLOCKS = 148 * 3;
+// body(j, bx) for the nblk blocks bx of every row j whose flag is set, shared out among the launch's blocks (256 threads);
+// the flags are listed 256 at a time. A launch of nblk blocks for each of F rows costs 25 to 40 us of blocks that leave at
+// once when few flags or none are set, this one 4.
+constexpr int SEG_FLAGGED_BLOCKS = 148 * 8;
 template <typename Body>
 __device__ __forceinline__ void seg_flagged(const int* flag, int F, int nblk, Body body) {
+  __shared__ int list[256], cnt[8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int64_t base = 0;
-  for (int j = 0; j < F; j++) {
-    if (!flag[j]) continue;
-    const int64_t g = gridDim.x, d = (int64_t)blockIdx.x - base % g;
-    for (int64_t i = d < 0 ? d + g : d; i < nblk; i += g) {
-      body(j, (int)i);
+  for (int j0 = 0; j0 < F; j0 += 256) {
+    const bool on = j0 + tid < F && flag[j0 + tid];
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) cnt[warp] = __popc(m);
+    __syncthreads();
+    int at = __popc(m & ((1u << lane) - 1u)), total = 0;
+    for (int w = 0; w < 8; w++) { at += w < warp ? cnt[w] : 0; total += cnt[w]; }
+    if (on) list[at] = j0 + tid;
+    __syncthreads();
+    const int64_t n = (int64_t)total * nblk, g = gridDim.x, d = (int64_t)blockIdx.x - base % g;
+    for (int64_t i = d < 0 ? d + g : d; i < n; i += g) {
+      body(list[i / nblk], (int)(i % nblk));
       __syncthreads();                     // seg_partials_at's shared memory
     }
-    base += nblk;
+    base += n;
+    __syncthreads();                       // list and cnt
   }
 }
 
