@@ -223,62 +223,61 @@ __global__ void __launch_bounds__(256, 3) k_seg_dots2_c128(const blml_seg* segs,
   const int64_t o = S.off, n = (int64_t)S.K * S.B;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const unsigned long long on = slots_on(hm, blockIdx.y, np, two);
-  const int total = __popcll(on);
+  const int first = blockIdx.z * 3 * nw;                  // three vectors per warp: 24 slots per launch layer
+  if (first && first >= __popcll(on)) return;
   const double2* B0 = reinterpret_cast<const double2*>(b0) + o;
   const double2* B1 = reinterpret_cast<const double2*>(b1) + o;
   const double2* X = x ? reinterpret_cast<const double2*>(x) + o : nullptr;
-  const int64_t slot = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, qs = (int64_t)gridDim.y * gridDim.x;
   const double2 zero = make_double2(0.0, 0.0);
-  // three vectors per warp and pass over the block's tiles
-  for (int first = 0; first == 0 || first < total; first += 3 * nw) {
-    const double2* A[3];
-    int na = 0, sl[3];
+  const double2* A[3];
+  int na = 0;
 #pragma unroll
-    for (int j = 0; j < 3; j++) {
-      sl[j] = nth_slot(on, first + warp + nw * j);
-      A[j] = sl[j] >= 0 ? reinterpret_cast<const double2*>(al.a[sl[j]]) + o : nullptr;
-      na += sl[j] >= 0;
-    }
-    const bool norms = first == 0 && warp == nw - 1;
-    double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
-    for (int64_t t = (int64_t)blockIdx.x * 64; t < n && (na || norms); t += (int64_t)gridDim.x * 64) {
-      // both elements' loads issued together: out-of-range lanes read element 0 and zero its shared values, so their
-      // products and norms add nothing
-      const int64_t i0 = t + lane, i1 = t + 32 + lane;
-      const bool v0 = i0 < n, v1 = i1 < n;
-      const int64_t j0 = v0 ? i0 : 0, j1 = v1 ? i1 : 0;
-      double2 y00 = ld_c2(B0 + j0), y01 = ld_c2(B0 + j1), y10 = __ldg(B1 + j0), y11 = __ldg(B1 + j1);
-      double2 a[3][2];
+  for (int j = 0; j < 3; j++) {
+    const int sl = nth_slot(on, first + warp + nw * j);
+    A[j] = sl >= 0 ? reinterpret_cast<const double2*>(al.a[sl]) + o : nullptr;
+    na += sl >= 0;
+  }
+  const bool norms = first == 0 && warp == nw - 1;
+  double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
+  for (int64_t t = (int64_t)blockIdx.x * 64; t < n && (na || norms); t += (int64_t)gridDim.x * 64) {
+    // both elements' loads issued together: out-of-range lanes read element 0 and zero its shared values, so their
+    // products and norms add nothing
+    const int64_t i0 = t + lane, i1 = t + 32 + lane;
+    const bool v0 = i0 < n, v1 = i1 < n;
+    const int64_t j0 = v0 ? i0 : 0, j1 = v1 ? i1 : 0;
+    double2 y00 = ld_c2(B0 + j0), y01 = ld_c2(B0 + j1), y10 = __ldg(B1 + j0), y11 = __ldg(B1 + j1);
+    double2 a[3][2];
 #pragma unroll
-      for (int j = 0; j < 3; j++)
-        if (j < na) { a[j][0] = ld_c2(A[j] + j0); a[j][1] = ld_c2(A[j] + j1); }
-      double2 z0 = zero, z1 = zero;
-      if (norms && X) { z0 = __ldg(X + j0); z1 = __ldg(X + j1); }
-      if (!v0) { y00 = zero; y10 = zero; z0 = zero; }
-      if (!v1) { y01 = zero; y11 = zero; z1 = zero; }
+    for (int j = 0; j < 3; j++)
+      if (j < na) { a[j][0] = ld_c2(A[j] + j0); a[j][1] = ld_c2(A[j] + j1); }
+    double2 z0 = zero, z1 = zero;
+    if (norms && X) { z0 = __ldg(X + j0); z1 = __ldg(X + j1); }
+    if (!v0) { y00 = zero; y10 = zero; z0 = zero; }
+    if (!v1) { y01 = zero; y11 = zero; z1 = zero; }
 #pragma unroll
-      for (int j = 0; j < 3; j++)
-        if (j < na) {
-          a0[j] += a[j][0].x * y00.x + a[j][0].y * y00.y; a1[j] += a[j][0].x * y10.x + a[j][0].y * y10.y;
-          a0[j] += a[j][1].x * y01.x + a[j][1].y * y01.y; a1[j] += a[j][1].x * y11.x + a[j][1].y * y11.y;
-        }
-      if (norms) {
-        n0 += y00.x * y00.x + y00.y * y00.y; n1 += y10.x * y10.x + y10.y * y10.y; nx += z0.x * z0.x + z0.y * z0.y;
-        n0 += y01.x * y01.x + y01.y * y01.y; n1 += y11.x * y11.x + y11.y * y11.y; nx += z1.x * z1.x + z1.y * z1.y;
+    for (int j = 0; j < 3; j++)
+      if (j < na) {
+        a0[j] += a[j][0].x * y00.x + a[j][0].y * y00.y; a1[j] += a[j][0].x * y10.x + a[j][0].y * y10.y;
+        a0[j] += a[j][1].x * y01.x + a[j][1].y * y01.y; a1[j] += a[j][1].x * y11.x + a[j][1].y * y11.y;
       }
-    }
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
-      if (j < na && lane == 0) {
-        const int q = slot_row(sl[j]);
-        part[q * qs + slot] = s0; part[(20 + q) * qs + slot] = s1;
-      }
-    }
     if (norms) {
-      n0 = warp_sum(n0); n1 = warp_sum(n1); nx = warp_sum(nx);
-      if (lane == 0) { part[40 * qs + slot] = n0; part[41 * qs + slot] = n1; part[42 * qs + slot] = nx; }
+      n0 += y00.x * y00.x + y00.y * y00.y; n1 += y10.x * y10.x + y10.y * y10.y; nx += z0.x * z0.x + z0.y * z0.y;
+      n0 += y01.x * y01.x + y01.y * y01.y; n1 += y11.x * y11.x + y11.y * y11.y; nx += z1.x * z1.x + z1.y * z1.y;
     }
+  }
+  const int64_t slot = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, qs = (int64_t)gridDim.y * gridDim.x;
+  const unsigned long long on2 = slots_on(hm, blockIdx.y, np, two);
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
+    if (j < na && lane == 0) {
+      const int q = slot_row(nth_slot(on2, first + warp + nw * j));
+      part[q * qs + slot] = s0; part[(20 + q) * qs + slot] = s1;
+    }
+  }
+  if (norms) {
+    n0 = warp_sum(n0); n1 = warp_sum(n1); nx = warp_sum(nx);
+    if (lane == 0) { part[40 * qs + slot] = n0; part[41 * qs + slot] = n1; part[42 * qs + slot] = nx; }
   }
 }
 
@@ -439,7 +438,6 @@ __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, 
   const int b = blockIdx.x, W = gridDim.x, f = split[F + 1 + b];
   if (f < 0) return;
   const unsigned long long on = slots_on(hm, f, np, two);
-  const int total = __popcll(on);
   const int lb = b - split[f], nb = split[f + 1] - split[f];
   const blml_seg S = segs[f];
   const int64_t o = S.off, n = (int64_t)S.K * S.B;
@@ -449,33 +447,34 @@ __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, 
   const double2* X = x ? x + o : nullptr;
   constexpr int64_t T = 128;
   const int64_t stride = (int64_t)nb * T;
-  for (int first = 0; first == 0 || first < total; first += 3 * nw) {
-    const float2* A[3];
-    int na = 0, sl[3];
+  const int first = blockIdx.y * 3 * nw;
+  if (first && first >= __popcll(on)) return;
+  const float2* A[3];
+  int na = 0;
 #pragma unroll
-    for (int j = 0; j < 3; j++) {
-      sl[j] = nth_slot(on, first + warp + nw * j);
-      A[j] = sl[j] >= 0 ? reinterpret_cast<const float2*>(al.a[sl[j]]) + o : nullptr;
-      na += sl[j] >= 0;
-    }
-    const bool norms = first == 0 && warp == nw - 1;
-    double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
-    int64_t t = (int64_t)lb * T;
-    if (!na && !norms) t = n;
-    for (; t + T <= n; t += stride) h32_tile<false>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
-    for (; t < n; t += stride) h32_tile<true>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
+  for (int j = 0; j < 3; j++) {
+    const int sl = nth_slot(on, first + warp + nw * j);
+    A[j] = sl >= 0 ? reinterpret_cast<const float2*>(al.a[sl]) + o : nullptr;
+    na += sl >= 0;
+  }
+  const bool norms = first == 0 && warp == nw - 1;
+  double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
+  int64_t t = (int64_t)lb * T;
+  if (!na && !norms) t = n;
+  for (; t + T <= n; t += stride) h32_tile<false>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
+  for (; t < n; t += stride) h32_tile<true>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
+  const unsigned long long on2 = slots_on(hm, f, np, two);
 #pragma unroll
-    for (int j = 0; j < 3; j++) {
-      const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
-      if (j < na && lane == 0) {
-        const int q = slot_row(sl[j]);
-        part[(int64_t)q * W + b] = s0; part[(int64_t)(20 + q) * W + b] = s1;
-      }
+  for (int j = 0; j < 3; j++) {
+    const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
+    if (j < na && lane == 0) {
+      const int q = slot_row(nth_slot(on2, first + warp + nw * j));
+      part[(int64_t)q * W + b] = s0; part[(int64_t)(20 + q) * W + b] = s1;
     }
-    if (norms) {
-      n0 = warp_sum(n0); n1 = warp_sum(n1); nx = warp_sum(nx);
-      if (lane == 0) { part[40LL * W + b] = n0; part[41LL * W + b] = n1; part[42LL * W + b] = nx; }
-    }
+  }
+  if (norms) {
+    n0 = warp_sum(n0); n1 = warp_sum(n1); nx = warp_sum(nx);
+    if (lane == 0) { part[40LL * W + b] = n0; part[41LL * W + b] = n1; part[42LL * W + b] = nx; }
   }
 }
 
@@ -906,7 +905,7 @@ int seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, const vo
   for (int h = 0; h < (a2 && !one ? 2 : 1); h++) {
     SegList al{};
     for (int q = 0; q < np; q++) { al.a[q] = h ? a2[q] : a[q]; if (one && a2) al.a[20 + q] = a2[q]; }
-    if (one) k_seg_dots2_c128<<<g, 256, 0, st>>>(segs, np, a2 != nullptr, al, b0, b1, x, part, hm);
+    if (one) k_seg_dots2_c128<<<dim3((unsigned)nb, (unsigned)F, a2 && 2 * np > 24 ? 2 : 1), 256, 0, st>>>(segs, np, a2 != nullptr, al, b0, b1, x, part, hm);
     else if (dtype == BLML_F64) k_seg_dots2<double><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
     else k_seg_dots2<float><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
     BLML_CHECK_LAUNCH("blml_seg_dots2");
@@ -923,7 +922,7 @@ int seg_dots2_h32(int F, const blml_seg* segs, const int* split, int np, const v
   SegList al{};
   for (int q = 0; q < np; q++) { al.a[q] = a[q]; if (a2) al.a[20 + q] = a2[q]; }
   const int W = SEG_SPLIT_BLOCKS + F;
-  k_seg_dots2_h32<<<W, 256, 0, st>>>(segs, split, F, np, a2 != nullptr, al, (const float2*)b0, (const double2*)b1,
+  k_seg_dots2_h32<<<dim3((unsigned)W, a2 && 2 * np > 24 ? 2 : 1), 256, 0, st>>>(segs, split, F, np, a2 != nullptr, al, (const float2*)b0, (const double2*)b1,
                                      (const double2*)x, part, hm);
   BLML_CHECK_LAUNCH("history scan (float32 history)");
   k_seg_finish_dots2_split<<<dim3(F, a2 ? 2 : 1), 256, 0, st>>>(part, W, split, np, out, out2, hm);
