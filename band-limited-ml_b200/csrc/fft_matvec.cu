@@ -143,9 +143,15 @@ template <typename T, int R, bool INV> __device__ __forceinline__ void butterfly
 // (j - j mod ns) R + j mod ns + s ns: to shared memory, or in the last pass (where that is j + s ns) to
 // store(t, j, s, ns, value). TF: consecutive threads take consecutive transforms (the side whose global accesses are
 // contiguous over transforms), else consecutive butterflies.
+// ldg_c: constants of the plan, through the read-only path. ld_c: what the kernel before may have written -- the stages may
+// be resident while it still writes (stage_wait), and only ordinary loads are ordered behind that wait.
 template <typename T> __device__ __forceinline__ cpx<T> ldg_c(const cpx<T>* p) {
   if constexpr (sizeof(T) == 8) { const double2 v = __ldg(reinterpret_cast<const double2*>(p)); return {v.x, v.y}; }
   else { const float2 v = __ldg(reinterpret_cast<const float2*>(p)); return {v.x, v.y}; }
+}
+template <typename T> __device__ __forceinline__ cpx<T> ld_c(const cpx<T>* p) {
+  if constexpr (sizeof(T) == 8) { const double2 v = *reinterpret_cast<const double2*>(p); return {v.x, v.y}; }
+  else { const float2 v = *reinterpret_cast<const float2*>(p); return {v.x, v.y}; }
 }
 
 // the band position of DFT index k of axis 1, or -1
@@ -294,10 +300,10 @@ __device__ __forceinline__ void rows_fwd_body(const FftDesc& D, int cta, unsigne
   if (D.flags & 1) {
     const T* X = reinterpret_cast<const T*>(D.X) + base;
     transform<T, false, false, true>(ax, tw, nr, mnr, a, b,
-                                     [&](int t, int i) { return cpx<T>{__ldg(X + t * N + i), T(0)}; }, keep);
+                                     [&](int t, int i) { return cpx<T>{X[t * N + i], T(0)}; }, keep);
   } else {
     const cpx<T>* X = reinterpret_cast<const cpx<T>*>(D.X) + base;
-    transform<T, false, false, true>(ax, tw, nr, mnr, a, b, [&](int t, int i) { return ldg_c(X + t * N + i); }, keep);
+    transform<T, false, false, true>(ax, tw, nr, mnr, a, b, [&](int t, int i) { return ld_c(X + t * N + i); }, keep);
   }
 }
 
@@ -361,7 +367,7 @@ __device__ __forceinline__ void rows_inv_body(const FftDesc& D, int cta, unsigne
     const int q2 = band_pos(D, k);
     if (q2 < 0) return cpx<T>{T(0), T(0)};
     const int row = r0 + t, bt = lattice_of(D, row);
-    return ldg_c(Z + ((int64_t)bt * H2 + q2) * M1 + (row - bt * M1));
+    return ld_c(Z + ((int64_t)bt * H2 + q2) * M1 + (row - bt * M1));
   };
   const int64_t base = (int64_t)r0 * N;
   if (D.flags & 4) {
@@ -374,7 +380,9 @@ __device__ __forceinline__ void rows_inv_body(const FftDesc& D, int cta, unsigne
 }
 
 // the stages are launched with programmatic dependent launch: a stage's CTAs may be placed while the one before drains,
-// and wait here for its results; every stage lets the next one in as soon as all its own CTAs have started
+// and wait here for its results; every stage lets the next one in as soon as all its own CTAs have started. No memory that
+// another kernel writes is read before the wait or through the read-only path (no __ldg, no const __restrict__ parameter:
+// such loads are not ordered behind it)
 __device__ __forceinline__ void stage_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -425,10 +433,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_fft_cluster(const __grid_cons
     if (D.flags & 1) {
       const T* X = reinterpret_cast<const T*>(D.X) + base + (int64_t)r0 * N;
       transform<T, false, false, true>(D.ax2, tw2, nr, mnr, a, b,
-                                       [&](int t, int i) { return cpx<T>{__ldg(X + t * N + i), T(0)}; }, keep);
+                                       [&](int t, int i) { return cpx<T>{X[t * N + i], T(0)}; }, keep);
     } else {
       const cpx<T>* X = reinterpret_cast<const cpx<T>*>(D.X) + base + (int64_t)r0 * N;
-      transform<T, false, false, true>(D.ax2, tw2, nr, mnr, a, b, [&](int t, int i) { return ldg_c(X + t * N + i); },
+      transform<T, false, false, true>(D.ax2, tw2, nr, mnr, a, b, [&](int t, int i) { return ld_c(X + t * N + i); },
                                        keep);
     }
     __syncthreads();
@@ -526,8 +534,7 @@ struct FftFew { FftDesc d[kFew]; int n, offA[kFew + 1], offB[kFew + 1]; };
 // (384 x 384 x 8: 36.1 -> 34.0 us)
 #define FFT_STAGE(NAME, BODY, OFF)                                                                                \
   template <typename T>                                                                                          \
-  __global__ void __launch_bounds__(kFT, 4) NAME##_grp(const FftDesc* __restrict__ descs,                           \
-                                                    const FftSched* __restrict__ sch) {                          \
+  __global__ void __launch_bounds__(kFT, 4) NAME##_grp(const FftDesc* descs, const FftSched* sch) {                 \
     extern __shared__ __align__(16) unsigned char fft_smem[];                                                    \
     __shared__ __align__(16) FftDesc Ds;                                                                         \
     stage_wait();                                                                                                \

@@ -198,7 +198,8 @@ using TileS = StageTile<1, 1, 2, 2, 32, 4>;              // 16 x 16
 using TileD = StageTile<1, 1, 2, 2, 64, 3>;              // 16 x 16, deeper slices: fewer of them, two CTAs per SM
 using TileM = StageTile<2, 2, 2, 2, 16, 4>;              // 32 x 32
 
-// dependent launches: the CTAs may be placed while the stage before drains, and wait here for its results
+// dependent launches: the CTAs may be placed while the stage before drains, and wait here for its results (read by ordinary
+// loads alone: the read-only path, which const __restrict__ parameters may take, is not ordered behind the wait)
 __device__ __forceinline__ void stage_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -214,9 +215,7 @@ __global__ void __launch_bounds__(TL::THREADS) k_stage(const __grid_constant__ S
 
 // the same stage of many mat-vecs: problem blockIdx.z of the subset
 template <typename TL>
-__global__ void __launch_bounds__(TL::THREADS) k_stage_grouped(const StageDesc* __restrict__ descs,
-                                                               const int* __restrict__ subset,
-                                                               const int* __restrict__ live) {
+__global__ void __launch_bounds__(TL::THREADS) k_stage_grouped(const StageDesc* descs, const int* subset, const int* live) {
   extern __shared__ __align__(16) unsigned char stage_smem[];
   stage_wait();
   const int gi = subset ? subset[blockIdx.z] : blockIdx.z;
