@@ -83,7 +83,7 @@ constexpr int kConvStages = 20;
 struct ConvPipe {
   uint64_t full[kConvStages], empty[kConvStages], tfull[2], tempty[2], once;
   uint32_t tslot;
-  int abort;
+  int abort, once_issued;               // (once_issued: the load behind `once` has been started)
   long long issued, consumed;           // slices loaded by the producer / taken by the MMA issuer
 };
 
@@ -99,7 +99,7 @@ __device__ __forceinline__ uint32_t conv_begin(ConvPipe* sh, int stages, int col
     for (int s = 0; s < stages; s++) { nn_mbar_init(&sh->full[s], 1); nn_mbar_init(&sh->empty[s], 1); }
     for (int a = 0; a < 2; a++) { nn_mbar_init(&sh->tfull[a], 1); nn_mbar_init(&sh->tempty[a], 4); }
     nn_mbar_init(&sh->once, 1);
-    sh->abort = 0; sh->issued = 0; sh->consumed = 0;
+    sh->abort = 0; sh->once_issued = 0; sh->issued = 0; sh->consumed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -112,8 +112,9 @@ __device__ __forceinline__ void conv_end(ConvPipe* sh, int stages, int columns, 
   const int tid = threadIdx.x;
   __syncthreads();
   if (*(volatile int*)&sh->abort && tid == 0) {
-    // a bounded wait gave up: the slices still loading and the MMAs last committed get one more bounded wait each
-    // before the shared and tensor memory are released
+    // a bounded wait gave up: the resident operand and the slices still loading and the MMAs last committed get one more
+    // bounded wait each before the shared and tensor memory are released
+    if (*(volatile int*)&sh->once_issued) nn_wait_or_abort(&sh->once, 0, nullptr);
     const long long iss = *(volatile long long*)&sh->issued, con = *(volatile long long*)&sh->consumed;
     for (long long g = con; g < iss; g++)
       nn_wait_or_abort(&sh->full[g % stages], (uint32_t)((g / stages) & 1), nullptr);
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(NN_PIPE_THREADS, 1) k_conv3x3(const __grid_con
     bool ok = true;
     if (wonce) {
       nn_mbar_expect_tx(&sh->once, (uint32_t)nslice * b_bytes);
+      *(volatile int*)&sh->once_issued = 1;
       for (int tap = 0, sl = 0; sl < nslice; tap++)
         for (int c = 0; c < C; c += CK, sl++) load_w(wbase + (size_t)sl * b_bytes, tap, c, &sh->once);
     }
