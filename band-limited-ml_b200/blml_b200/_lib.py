@@ -232,18 +232,19 @@ def current_stream(device):
 
 class Lender:
     """Device memory lent to the library (blml_alloc_fn) from torch's allocator, on the device's current stream. Keep it
-    until the objects created with it are destroyed."""
+    until the objects created with it are destroyed; the memory goes back to the allocator with it (the callback holds
+    the list alone, not this object: a cycle would keep the memory until Python's collector ran)."""
 
     def __init__(self, device):
         import torch
-        self.tensors = []
+        self.tensors = tensors = []
 
         def alloc(nbytes, ctx):
             try:
                 t = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
             except Exception:                      # none left: the library reports it (nothing may unwind through it)
                 return None
-            self.tensors.append(t)
+            tensors.append(t)
             return t.data_ptr()
 
         self.fn = ALLOC_FN(alloc)

@@ -73,6 +73,27 @@ def lanczos_max(plan, dh, red, stream, tol=1e-6, seed=0, max_basis=96, max_resta
     return theta
 
 
+class _Subset:
+    """The fits a launch covers: their segment list (offsets into the full vectors), grouped mat-vec and blocks."""
+
+    def __init__(self, batch, idx, chunk, tmp, sv):
+        from .sweep import _Group, _Seg
+        self.idx = np.asarray(idx, np.int64)
+        segs = (_Seg * len(self.idx))(*[_Seg(int(batch.boff[f]), int(batch.boff[f]), int(batch.B[f]), 1, 0)
+                                        for f in self.idx])
+        nc = -(-np.asarray(batch.B)[self.idx] // chunk)
+        row = np.repeat(np.arange(len(self.idx)), nc)
+        tab = np.stack([row, np.arange(len(row)) - np.repeat(np.cumsum(nc) - nc, nc)], 1).astype(np.int32)
+        self.nblocks = len(tab)
+        ints = np.concatenate([np.frombuffer(bytes(segs), np.int32), self.idx.astype(np.int32),
+                               np.zeros(len(self.idx), np.int32)])      # 10 ints a row: tab stays 8-byte aligned
+        self.segs_t = torch.from_numpy(np.concatenate([ints, tab.ravel()])).to(batch.device)
+        at = self.segs_t.data_ptr()
+        self.fid, self.cnt, self.tab = at + len(bytes(segs)), at + len(bytes(segs)) + 4 * len(self.idx), at + 4 * len(ints)
+        off = np.asarray(batch.boff[:-1])[self.idx]
+        self.grp = _Group([batch.p64[f] for f in self.idx], tmp, off, sv, off, False)
+
+
 def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, vectors=False, above=None,
                         second=False):
     """The certificate of every fit of a fitted BLMLBinnedBatch at once: lambda_max(D^1/2 S D^1/2) per fit
@@ -90,7 +111,6 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
     dh, v): dh the per-bin scaling and v the top Ritz vectors (float64 per bin over all fits, None unless vectors)
     -- d = dh v is the direction of a new mode. second (with vectors): v is a pair (top, next) -- the Ritz vector of
     each fit's second Ritz value from the same Krylov basis, a second ascent direction while that value is above n."""
-    from .sweep import _Group, _Seg
     clock = {'wait_s': 0.0, 'host_s': 0.0}
     F, dev, st, B = batch.F, batch.device, batch.st, batch.Btot
     code = _lib.F64
@@ -103,24 +123,8 @@ def lanczos_max_batched(batch, tol=1e-6, seed=0, max_basis=64, max_restarts=12, 
     # bins per block of a step: at least 512, at most 256 blocks a fit
     chunk = max(512, -(-int(batch.B.max()) // (256 * 256)) * 256)
 
-    class Subset:
-        """The fits a launch covers: their segment list (offsets into the full vectors), grouped mat-vec and blocks."""
-
-        def __init__(self, idx):
-            self.idx = np.asarray(idx, np.int64)
-            segs = (_Seg * len(self.idx))(*[_Seg(int(batch.boff[f]), int(batch.boff[f]), int(batch.B[f]), 1, 0)
-                                            for f in self.idx])
-            nc = -(-np.asarray(batch.B)[self.idx] // chunk)
-            row = np.repeat(np.arange(len(self.idx)), nc)
-            tab = np.stack([row, np.arange(len(row)) - np.repeat(np.cumsum(nc) - nc, nc)], 1).astype(np.int32)
-            self.nblocks = len(tab)
-            ints = np.concatenate([np.frombuffer(bytes(segs), np.int32), self.idx.astype(np.int32),
-                                   np.zeros(len(self.idx), np.int32)])      # 10 ints a row: tab stays 8-byte aligned
-            self.segs_t = torch.from_numpy(np.concatenate([ints, tab.ravel()])).to(dev)
-            at = self.segs_t.data_ptr()
-            self.fid, self.cnt, self.tab = at + len(bytes(segs)), at + len(bytes(segs)) + 4 * len(self.idx), at + 4 * len(ints)
-            off = np.asarray(batch.boff[:-1])[self.idx]
-            self.grp = _Group([batch.p64[f] for f in self.idx], tmp, off, sv, off, False)
+    def Subset(idx):
+        return _Subset(batch, idx, chunk, tmp, sv)
 
     def dots(S, pairs):
         n = len(S.idx)
