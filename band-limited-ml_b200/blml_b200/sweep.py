@@ -70,7 +70,9 @@ class _Group:
         """The handle, its lent memory ready for a launch on `stream`."""
         if (stream or 0) != self._st:                       # lent memory on another stream than its own
             other = torch.cuda.ExternalStream(stream or 0, device=self._keep[1].device)
-            other.wait_stream(torch.cuda.ExternalStream(self._st, device=other.device))
+            with torch.cuda.stream(other):
+                if not torch.cuda.is_current_stream_capturing():     # (a capture cannot wait for a stream outside it: the
+                    other.wait_stream(torch.cuda.ExternalStream(self._st, device=other.device))   # capturer has waited)
             for t in self._mem.tensors:
                 t.record_stream(other)
         return self._h

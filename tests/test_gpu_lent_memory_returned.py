@@ -85,3 +85,24 @@ def test_memory_of_a_group_pending_on_another_stream_is_not_reused(cuda_device, 
     assert not other.query() and len(taken) == 4 * len(sizes)         # (the test's premise)
     torch.cuda.synchronize()
     torch.testing.assert_close(y, ref, rtol=1e-13, atol=0)
+
+
+@pytest.mark.parametrize('own', [False, True])
+def test_group_inside_a_stream_capture(cuda_device, own):
+    """A group made on the default stream, captured on a stream of its own and replayed on new input (own: made on the
+    capturing stream)."""
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st) if own else torch.cuda.stream(torch.cuda.current_stream()):
+        g, x, y, ref = _group(3)
+    g((st if own else torch.cuda.current_stream()).cuda_stream)
+    torch.cuda.synchronize()
+    torch.testing.assert_close(y, ref, rtol=1e-13, atol=0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        g(st.cuda_stream)
+    x.mul_(2.0)
+    y.zero_()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    torch.testing.assert_close(y, 2.0 * ref, rtol=1e-13, atol=0)
