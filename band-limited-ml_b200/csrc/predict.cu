@@ -25,8 +25,8 @@ __device__ __forceinline__ cpx<double> phase(double nu, double u) {
 }
 
 // spec (H1 x H2 complex, row-major), f1 (H1), f2 (H2) cycles per lattice index, U (m x 2) lattice coordinates; C
-// axis-1 frequencies per lane and chunk
-template <int C>
+// axis-1 frequencies per lane and chunk; V: spec's coefficients in one 16-byte load (16-byte aligned), else in two
+template <int C, bool V>
 __global__ void __launch_bounds__(32 * kPwWarps, 2) k_planewave_points(int H1, int H2, const double* __restrict__ f1,
                                                                         const double* __restrict__ f2,
                                                                         const cpx<double>* __restrict__ spec, int64_t m,
@@ -75,9 +75,11 @@ __global__ void __launch_bounds__(32 * kPwWarps, 2) k_planewave_points(int H1, i
         for (int p = 0; p < kPwPts; p++) part[p] = {0.0, 0.0};
 #pragma unroll
         for (int c = 0; c < C; c++) {
-          const double2 s = __ldg(reinterpret_cast<const double2*>(row + q2[c]));
+          cpx<double> s;
+          if (V) { const double2 v = __ldg(reinterpret_cast<const double2*>(row + q2[c])); s = {v.x, v.y}; }
+          else s = row[q2[c]];
 #pragma unroll
-          for (int p = 0; p < kPwPts; p++) part[p] = cfma(cpx<double>{s.x, s.y}, ph2[c][p], part[p]);
+          for (int p = 0; p < kPwPts; p++) part[p] = cfma(s, ph2[c][p], part[p]);
         }
 #pragma unroll
         for (int p = 0; p < kPwPts; p++) {
@@ -117,10 +119,11 @@ int blml_planewave_points(int H1, int H2, const double* f1, const double* f2, co
     kern<<<blocks, 32 * kPwWarps, 0, st>>>(H1, H2, f1, f2, reinterpret_cast<const cpx<double>*>(spec), m, U,
                                            reinterpret_cast<cpx<double>*>(g));
   };
-  if (c <= 1) run(k_planewave_points<1>);
-  else if (c == 2) run(k_planewave_points<2>);
-  else if (c == 3) run(k_planewave_points<3>);
-  else run(k_planewave_points<4>);
+  const bool v = (reinterpret_cast<uintptr_t>(spec) & 15) == 0;
+  if (c <= 1) v ? run(k_planewave_points<1, true>) : run(k_planewave_points<1, false>);
+  else if (c == 2) v ? run(k_planewave_points<2, true>) : run(k_planewave_points<2, false>);
+  else if (c == 3) v ? run(k_planewave_points<3, true>) : run(k_planewave_points<3, false>);
+  else v ? run(k_planewave_points<4, true>) : run(k_planewave_points<4, false>);
   BLML_CHECK_LAUNCH("blml_planewave_points");
   return BLML_OK;
 }
