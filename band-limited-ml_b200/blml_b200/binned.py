@@ -733,20 +733,22 @@ class BLMLBinned:
     def _spectrum_plan(self, k):
         """Mode k's float64 contraction plan, its frequencies, and (frequencies per axis, origin, steps) on the device,
         for sums over its spectrum: the fit's own plan where it is one, else one made for it. Kept by the fit, per kernel,
-        lattice and stream."""
+        lattice, device and stream."""
         held = self.__dict__.setdefault('_spec_plans', {})
-        key = (spec_key(self.specs_[k]), self.shape_, tuple(self.h_), tuple(self.origin_), self._code, self._st)
-        if key not in held:
+        key = (spec_key(self.specs_[k]), self.shape_, tuple(self.h_), tuple(self.origin_), self._code, str(self.dev_),
+               self._st)
+        entry = held.get(key)
+        if entry is None:
             plan, _, (freqs, W) = self.kern_[k]
             if self._code != _lib.F64 or plan.engine != _lib.ENGINE_SIMT:
                 with torch.cuda.device(self.dev_):
                     plan = Plan(freqs, W, self.shape_, _lib.F64, _lib.ENGINE_SIMT)
             f1, f2 = (np.zeros(1), freqs[0]) if self.d_ == 1 else freqs
-            held[key] = plan, freqs, tuple(torch.as_tensor(np.array(a, np.float64)).to(self.dev_)
-                                           for a in (f1, f2, self.origin_, self.h_))
-            while len(held) > 8:
-                held.pop(next(iter(held)))
-        return held[key]
+            entry = held[key] = plan, freqs, tuple(torch.as_tensor(np.array(a, np.float64)).to(self.dev_)
+                                                   for a in (f1, f2, self.origin_, self.h_))
+            for old in list(held)[:-8]:                   # (another thread may have dropped it by now)
+                held.pop(old, None)
+        return entry
 
     def sqrt_density(self, X, chunk=65536):
         """g_k(x) = (1/n) sum_b e_bk K_k(x - z_b) at arbitrary points X (m, d) (blml_binned.py:451-465): (m,) for
