@@ -568,7 +568,7 @@ static int check_extents(const ColMeta& cm, const int64_t* ZA, int64_t R, const 
   return extents_ok(cm, hr);
 }
 
-// column slices of a rows launch: about 16 blocks of 128 rows per SM, at least 256 columns each
+// column slices of a rows launch (R, M >= 1): about 16 blocks of 128 rows per SM, at least 256 columns each
 static void rows_slices(int64_t R, int64_t M, int64_t& nsl, int64_t& slice, int64_t most = 65535) {
   const int64_t rblocks = (R + PR_THREADS - 1) / PR_THREADS;
   nsl = std::max<int64_t>(1, std::min<int64_t>((16 * 148 + rblocks - 1) / rblocks, (M + 255) / 256));
@@ -752,6 +752,7 @@ int blml_rows_plan_create(const blml_tables* tb, const int64_t* Z, int64_t n, vo
 
 int64_t blml_rows_plan_workspace(blml_rows_plan p, int64_t R, int64_t M) {
   if (!p || R < 0 || M < 1) return -1;
+  if (R == 0) return 0;
   int64_t nsl, slice;
   rows_slices(R, M, nsl, slice);
   return nsl * R * (int64_t)sizeof(double);
@@ -787,14 +788,15 @@ int64_t blml_rows_workspace(int64_t R, int64_t M, int nW) {
 int blml_rows_ws(const blml_tables* tb, const int64_t* ZA, int64_t R, const int64_t* ZB, int64_t M, const double* w,
                  int grad, double* s, double* ds, void* ws, int64_t ws_bytes, void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (!tb || R < 0 || M < 0) { set_error("blml_rows: no tables, or a negative count of rows or columns"); return BLML_ERR_ARG; }
   ColMeta cm;
   if (R == 0 || M == 0) {                    // nothing to sum: the tables are checked all the same
     const int e = read_meta(tb, cm, st);
     if (e || R == 0) return e;
     return cuda_status(cudaMemsetAsync(s, 0, R * sizeof(double), st), "blml_rows");
   }
-  if (tb && tb->nW == 0) grad = 0;
-  const int64_t need = rows_bytes(R, M, grad && tb ? tb->nW : 0);
+  if (tb->nW == 0) grad = 0;
+  const int64_t need = rows_bytes(R, M, grad ? tb->nW : 0);
   if (!ws || ws_bytes < need) {
     set_error("blml_rows: workspace of %lld bytes, need %lld", (long long)ws_bytes, (long long)need);
     return BLML_ERR_WORKSPACE;
@@ -855,6 +857,7 @@ int blml_rows_multi(const blml_tables* tb, const int64_t* ZA, int64_t R, const i
                     const double* W, int Mm, const unsigned* umask, double* s, void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (Mm < 1 || Mm > MAXM || !umask) { set_error("blml_rows_multi: 1 to %d densities with a unit mask each", MAXM); return BLML_ERR_ARG; }
+  if (R < 0 || M < 0) { set_error("blml_rows_multi: a negative count of rows or columns"); return BLML_ERR_ARG; }
   ColMeta cm;
   int e = read_meta(tb, cm, st);
   if (e) return e;
