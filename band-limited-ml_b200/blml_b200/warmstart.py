@@ -141,6 +141,8 @@ class WarmStartNet:
         """x: BF16 (N, H, W, 8) on the device -> u FP32 (N, H, W, 2); keeps the activations for backward."""
         if H % 8 or W % 8:
             raise ValueError("WarmStartNet: lattice sides must be multiples of 8")
+        if x.data_ptr() % 16:
+            x = x.clone()                                  # (the convolutions' copies start on 16-byte boundaries)
         self.shape_ = (N, H, W)
         P1, P2, P3, P4 = N * H * W, N * H * W // 4, N * H * W // 16, N * H * W // 64
         H2, W2, H4, W4, H8, W8 = H // 2, W // 2, H // 4, W // 4, H // 8, W // 8

@@ -530,16 +530,21 @@ __global__ void __launch_bounds__(256) k_head_bwd_weight32(const float* __restri
 //   l_s = min over (t, conj t) and a global phase of |u - e^{i th} t|^2 / |t|^2
 //       = (|u|^2 + |t|^2 - 2 max(|<t, u>|, |<conj t, u>|)) / |t|^2
 // stats[s] = [|u|^2, |t|^2, Re a, Im a, Re b, Im b] with a = sum conj(t) u, b = sum t u: a cluster of 8 blocks per
-// sample, the blocks' sums joined in block order through distributed shared memory
+// sample, the blocks' sums joined in block order through distributed shared memory. V: a pair in one load (u and t on
+// 8-byte boundaries), else in two
 constexpr int kLossBlocks = 8;
+template <bool V>
 __global__ void __cluster_dims__(kLossBlocks, 1, 1) __launch_bounds__(256)
-    k_loss_stats(const float2* __restrict__ u, const float2* __restrict__ t, int64_t HW, double* __restrict__ stats) {
+    k_loss_stats(const float* __restrict__ u, const float* __restrict__ t, int64_t HW, double* __restrict__ stats) {
   const int s = blockIdx.x / kLossBlocks, part = blockIdx.x % kLossBlocks;
-  const float2* us = u + (size_t)s * HW;
-  const float2* ts = t + (size_t)s * HW;
+  const float* us = u + (size_t)s * HW * 2;
+  const float* ts = t + (size_t)s * HW * 2;
+  auto pair = [](const float* p, int64_t i) {
+    return V ? reinterpret_cast<const float2*>(p)[i] : make_float2(p[2 * i], p[2 * i + 1]);
+  };
   double v[6] = {0, 0, 0, 0, 0, 0};
   for (int64_t i = (int64_t)part * blockDim.x + threadIdx.x; i < HW; i += kLossBlocks * blockDim.x) {
-    const float2 a = us[i], b = ts[i];
+    const float2 a = pair(us, i), b = pair(ts, i);
     const double ur = a.x, ui = a.y, tr = b.x, ti = b.y;
     v[0] += ur * ur + ui * ui; v[1] += tr * tr + ti * ti;
     v[2] += tr * ur + ti * ui; v[3] += tr * ui - ti * ur;       // conj(t) u
@@ -876,11 +881,8 @@ int blml_nn_phase_loss(const float* u, const float* t, int64_t HW, int S, double
   if (!u || !t || !stats || !du || !loss || HW < 1 || S < 1 || S > 65535) {
     set_error("blml_nn_phase_loss: bad arguments"); return BLML_ERR_ARG;
   }
-  if ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(t)) & 7) {
-    set_error("blml_nn_phase_loss: u and t are complex pairs (8-byte aligned)"); return BLML_ERR_ARG;
-  }
-  k_loss_stats<<<S * kLossBlocks, 256, 0, NST>>>(reinterpret_cast<const float2*>(u), reinterpret_cast<const float2*>(t),
-                                               HW, stats);
+  const bool v = ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(t)) & 7) == 0;
+  (v ? k_loss_stats<true> : k_loss_stats<false>)<<<S * kLossBlocks, 256, 0, NST>>>(u, t, HW, stats);
   BLML_CHECK_LAUNCH("blml_nn_phase_loss");
   k_loss_grad<<<dim3(g1(HW), (unsigned)S), 256, 0, NST>>>(u, t, HW, S, stats, du, loss);
   BLML_CHECK_LAUNCH("blml_nn_phase_loss");
