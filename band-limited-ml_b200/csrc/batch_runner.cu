@@ -980,7 +980,8 @@ struct blml_lbfgs_batch_s : Runner {
   // the history scan: H1 = [S_q . y_p, S_q . g, y_p . y_p, g . g, E . E], H2 = [Y_q . y_p, Y_q . g, ...]
   // over the slots that hold a pair (in set-up: none, and slot 0 is zero)
   int hist(int Fa_, const blml_seg* S, int p) {
-    const HistMask hm{s.stamp, d_fid, m, p};
+    // (a pair an iteration, and slot p)
+    const HistMask hm{s.stamp, d_fid, m, p, (int)std::min<long long>(m, most < LLONG_MAX ? most + 1 : m)};
     const void* a[LB_MMAX]; const void* a2[LB_MMAX];
     for (int i = 0; i < m; i++) { a[i] = Sh[i]; a2[i] = Yh[i]; }
     return h32 ? seg_dots2_h32(Fa_, S, split, m, a, a2, Yh[p], g, E, part, H1, H2, hm, st)

@@ -190,25 +190,35 @@ __global__ void __launch_bounds__(256) k_seg_dots2(const blml_seg* segs, int cpl
   seg_partials<43>(v, part);
 }
 
-// the same scan for float64 complex vectors, one (re, im) load per element and vector -- the stored vectors (TA)
-// and the first shared one (TB0) complex128 (the plain fits' history; the float32 history has its own scan,
+// the same scan for float64 complex vectors, one (re, im) load per element and vector -- the stored vectors
+// and the first shared one complex128 (the plain fits' history; the float32 history has its own scan,
 // k_seg_dots2_h32, with twice the elements per thread and a block split by fit size). The block's 8 warps
-// split the stored vectors and walk the same 64-element tiles, so each thread
-// holds at most 6 accumulators (full occupancy, many loads in flight) and the two shared vectors are read from HBM
+// split the stored vectors, up to NV each, and walk the same 64-element tiles, so each thread
+// holds at most 2 NV accumulators with many loads in flight, and the two shared vectors are read from HBM
 // once per tile and from L1 by the other warps; the last warp also sums the three squared norms. Each quantity's
 // block partial comes from one warp (warp_sum, fixed order), in seg_partials' layout.
-// The stored vectors are those of the mask's slots, the i-th of them for warp i mod 8 (a slot's sum does not depend on
-// which warp forms it): the first iterations of a fit, whose memory is still filling, read only what it holds. 64 fits of
-// rank 4 over their first 12 iterations (20 slots): 12.9 ms of scans -> 9.3, -> 7.1 with both lists (S and Y) in one scan.
-__device__ __forceinline__ int nth_slot(unsigned long long on, int i) {
-  for (; i > 0 && on; i--) on &= on - 1;
-  return __ffsll((long long)on) - 1;
-}
-// the slots of both lists that the scan covers (bit q, and 20 + q of the second list)
-__device__ __forceinline__ unsigned long long slots_on(const HistMask& hm, int j, int np, bool two) {
-  const int q = threadIdx.x & 31;
-  const unsigned long long b = __ballot_sync(0xffffffffu, q < np && hm.on(j, q));
-  return two ? b | b << 20 : b;
+// LISTED: the stored vectors are those of the mask's slots, of one list or two, the i-th of them for warp i mod 8 (a slot's
+// sum does not depend on which warp forms it): the first iterations of a fit, whose memory is still filling, read only what
+// it holds (64 fits of rank 4 over their first 12 iterations, 20 slots: 12.9 ms of scans -> 7.4).
+// Up to 24 vectors take three per warp and three blocks per SM, more take five and two blocks: at full history, 64 fits of
+// rank 4 (a step's two lists of 20, bound by HBM), two scans of one list 927 us, both lists in layers of 24 with the shared
+// vectors read twice and spills 1,310, this 899; two lists of 12 639 -> 547. One list of 20 by itself (not LISTED) 546 us,
+// 6.83 TB/s. Five per warp are slower while few slots hold a pair (a cold sweep's scans 130 -> 196 us), so a run of few
+// iterations takes three.
+//
+// list_slots: the slots that the scan covers, in list[0 ..] (a second list's from 20 on), and their number; called by the
+// whole block. In shared memory: walked as a bit mask by every warp before and after the loop they cost the loop registers
+// that it then spilled (one list of 20: 639 us).
+__device__ __forceinline__ int list_slots(const HistMask& hm, int j, int np, bool two, int* list) {
+  if (threadIdx.x < 32) {
+    const int q = threadIdx.x;
+    const unsigned b = __ballot_sync(0xffffffffu, q < np && hm.on(j, q));
+    const int n = __popc(b), at = __popc(b & ((1u << q) - 1u));
+    if (b >> q & 1u) { list[at] = q; if (two) list[n + at] = 20 + q; }
+    if (q == 0) list[40] = two ? 2 * n : n;
+  }
+  __syncthreads();
+  return list[40];
 }
 // the partials' row of slot s: its product with b0; the one with b1 is 20 rows on
 __device__ __forceinline__ int slot_row(int s) { return s < 20 ? s : 23 + s; }
@@ -216,46 +226,47 @@ __device__ __forceinline__ int slot_row(int s) { return s < 20 ? s : 23 + s; }
 // one complex128 element as (re, im)
 __device__ __forceinline__ double2 ld_c2(const double2* p) { return __ldg(p); }
 
-__global__ void __launch_bounds__(256, 3) k_seg_dots2_c128(const blml_seg* segs, int np, int two, SegList al,
+template <int NV, int NB, bool LISTED>
+__global__ void __launch_bounds__(256, NB) k_seg_dots2_c128(const blml_seg* segs, int np, int two, SegList al,
                                                            const void* b0, const void* b1, const void* x, double* part,
                                                            HistMask hm) {
+  __shared__ int list[41];                                // (LISTED; else the np vectors of one list, unmasked)
   const blml_seg S = segs[blockIdx.y];
   const int64_t o = S.off, n = (int64_t)S.K * S.B;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const unsigned long long on = slots_on(hm, blockIdx.y, np, two);
-  const int first = blockIdx.z * 3 * nw;                  // three vectors per warp: 24 slots per launch layer
-  if (first && first >= __popcll(on)) return;
+  const int ns = LISTED ? list_slots(hm, blockIdx.y, np, two, list) : np;
   const double2* B0 = reinterpret_cast<const double2*>(b0) + o;
   const double2* B1 = reinterpret_cast<const double2*>(b1) + o;
   const double2* X = x ? reinterpret_cast<const double2*>(x) + o : nullptr;
   const double2 zero = make_double2(0.0, 0.0);
-  const double2* A[3];
+  const double2* A[NV];
   int na = 0;
 #pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const int sl = nth_slot(on, first + warp + nw * j);
-    A[j] = sl >= 0 ? reinterpret_cast<const double2*>(al.a[sl]) + o : nullptr;
-    na += sl >= 0;
+  for (int j = 0; j < NV; j++) {
+    const int i = warp + nw * j;
+    A[j] = i < ns ? reinterpret_cast<const double2*>(al.a[LISTED ? list[i] : i]) + o : nullptr;
+    na += i < ns;
   }
-  const bool norms = first == 0 && warp == nw - 1;
-  double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
-  for (int64_t t = (int64_t)blockIdx.x * 64; t < n && (na || norms); t += (int64_t)gridDim.x * 64) {
+  const bool norms = warp == nw - 1;
+  double a0[NV] = {}, a1[NV] = {}, n0 = 0.0, n1 = 0.0, nx = 0.0;
+  // (three vectors: a warp without any walks along, the test for it costs registers that spill)
+  for (int64_t t = (int64_t)blockIdx.x * 64; t < n && (NV == 3 || na || norms); t += (int64_t)gridDim.x * 64) {
     // both elements' loads issued together: out-of-range lanes read element 0 and zero its shared values, so their
     // products and norms add nothing
     const int64_t i0 = t + lane, i1 = t + 32 + lane;
     const bool v0 = i0 < n, v1 = i1 < n;
     const int64_t j0 = v0 ? i0 : 0, j1 = v1 ? i1 : 0;
     double2 y00 = ld_c2(B0 + j0), y01 = ld_c2(B0 + j1), y10 = __ldg(B1 + j0), y11 = __ldg(B1 + j1);
-    double2 a[3][2];
+    double2 a[NV][2];
 #pragma unroll
-    for (int j = 0; j < 3; j++)
+    for (int j = 0; j < NV; j++)
       if (j < na) { a[j][0] = ld_c2(A[j] + j0); a[j][1] = ld_c2(A[j] + j1); }
     double2 z0 = zero, z1 = zero;
     if (norms && X) { z0 = __ldg(X + j0); z1 = __ldg(X + j1); }
     if (!v0) { y00 = zero; y10 = zero; z0 = zero; }
     if (!v1) { y01 = zero; y11 = zero; z1 = zero; }
 #pragma unroll
-    for (int j = 0; j < 3; j++)
+    for (int j = 0; j < NV; j++)
       if (j < na) {
         a0[j] += a[j][0].x * y00.x + a[j][0].y * y00.y; a1[j] += a[j][0].x * y10.x + a[j][0].y * y10.y;
         a0[j] += a[j][1].x * y01.x + a[j][1].y * y01.y; a1[j] += a[j][1].x * y11.x + a[j][1].y * y11.y;
@@ -266,12 +277,11 @@ __global__ void __launch_bounds__(256, 3) k_seg_dots2_c128(const blml_seg* segs,
     }
   }
   const int64_t slot = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, qs = (int64_t)gridDim.y * gridDim.x;
-  const unsigned long long on2 = slots_on(hm, blockIdx.y, np, two);
 #pragma unroll
-  for (int j = 0; j < 3; j++) {
+  for (int j = 0; j < NV; j++) {
     const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
     if (j < na && lane == 0) {
-      const int q = slot_row(nth_slot(on2, first + warp + nw * j));
+      const int q = LISTED ? slot_row(list[warp + nw * j]) : warp + nw * j;
       part[q * qs + slot] = s0; part[(20 + q) * qs + slot] = s1;
     }
   }
@@ -432,12 +442,14 @@ __device__ __forceinline__ void h32_tile(int64_t t, int64_t n, int lane, const f
   }
 }
 
+template <bool LISTED>
 __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, const int* split, int F, int np, int two,
                                                           SegList al, const float2* b0, const double2* b1,
                                                           const double2* x, double* part, HistMask hm) {
   const int b = blockIdx.x, W = gridDim.x, f = split[F + 1 + b];
   if (f < 0) return;
-  const unsigned long long on = slots_on(hm, f, np, two);
+  __shared__ int list[41];
+  const int ns = LISTED ? list_slots(hm, f, np, two, list) : np;
   const int lb = b - split[f], nb = split[f + 1] - split[f];
   const blml_seg S = segs[f];
   const int64_t o = S.off, n = (int64_t)S.K * S.B;
@@ -447,15 +459,15 @@ __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, 
   const double2* X = x ? x + o : nullptr;
   constexpr int64_t T = 128;
   const int64_t stride = (int64_t)nb * T;
-  const int first = blockIdx.y * 3 * nw;
-  if (first && first >= __popcll(on)) return;
+  const int first = LISTED ? blockIdx.y * 3 * nw : 0;     // three vectors per warp: 24 slots per launch layer
+  if (first && first >= ns) return;
   const float2* A[3];
   int na = 0;
 #pragma unroll
   for (int j = 0; j < 3; j++) {
-    const int sl = nth_slot(on, first + warp + nw * j);
-    A[j] = sl >= 0 ? reinterpret_cast<const float2*>(al.a[sl]) + o : nullptr;
-    na += sl >= 0;
+    const int i = first + warp + nw * j;
+    A[j] = i < ns ? reinterpret_cast<const float2*>(al.a[LISTED ? list[i] : i]) + o : nullptr;
+    na += i < ns;
   }
   const bool norms = first == 0 && warp == nw - 1;
   double a0[3] = {0.0, 0.0, 0.0}, a1[3] = {0.0, 0.0, 0.0}, n0 = 0.0, n1 = 0.0, nx = 0.0;
@@ -463,12 +475,11 @@ __global__ void __launch_bounds__(256, 2) k_seg_dots2_h32(const blml_seg* segs, 
   if (!na && !norms) t = n;
   for (; t + T <= n; t += stride) h32_tile<false>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
   for (; t < n; t += stride) h32_tile<true>(t, n, lane, A, na, B0, B1, X, norms, a0, a1, n0, n1, nx);
-  const unsigned long long on2 = slots_on(hm, f, np, two);
 #pragma unroll
   for (int j = 0; j < 3; j++) {
     const double s0 = warp_sum(a0[j]), s1 = warp_sum(a1[j]);
     if (j < na && lane == 0) {
-      const int q = slot_row(nth_slot(on2, first + warp + nw * j));
+      const int q = LISTED ? slot_row(list[first + warp + nw * j]) : warp + nw * j;
       part[(int64_t)q * W + b] = s0; part[(int64_t)(20 + q) * W + b] = s1;
     }
   }
@@ -905,7 +916,11 @@ int seg_dots2(int dtype, int F, const blml_seg* segs, int cplx, int np, const vo
   for (int h = 0; h < (a2 && !one ? 2 : 1); h++) {
     SegList al{};
     for (int q = 0; q < np; q++) { al.a[q] = h ? a2[q] : a[q]; if (one && a2) al.a[20 + q] = a2[q]; }
-    if (one) k_seg_dots2_c128<<<dim3((unsigned)nb, (unsigned)F, a2 && 2 * np > 24 ? 2 : 1), 256, 0, st>>>(segs, np, a2 != nullptr, al, b0, b1, x, part, hm);
+    if (one)
+      (!a2 && !hm.stamp ? k_seg_dots2_c128<3, 3, false>
+       : (a2 ? 2 : 1) * (hm.stamp ? std::min(np, hm.most) : np) <= 24 ? k_seg_dots2_c128<3, 3, true>
+                                                                      : k_seg_dots2_c128<5, 2, true>)
+          <<<g, 256, 0, st>>>(segs, np, a2 != nullptr, al, b0, b1, x, part, hm);
     else if (dtype == BLML_F64) k_seg_dots2<double><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
     else k_seg_dots2<float><<<g, 256, 0, st>>>(segs, cplx, np, al, b0, b1, x, part, hm);
     BLML_CHECK_LAUNCH("blml_seg_dots2");
@@ -922,8 +937,9 @@ int seg_dots2_h32(int F, const blml_seg* segs, const int* split, int np, const v
   SegList al{};
   for (int q = 0; q < np; q++) { al.a[q] = a[q]; if (a2) al.a[20 + q] = a2[q]; }
   const int W = SEG_SPLIT_BLOCKS + F;
-  k_seg_dots2_h32<<<dim3((unsigned)W, a2 && 2 * np > 24 ? 2 : 1), 256, 0, st>>>(segs, split, F, np, a2 != nullptr, al, (const float2*)b0, (const double2*)b1,
-                                     (const double2*)x, part, hm);
+  const int layers = a2 && 2 * np > 24 ? 2 : 1;
+  (a2 || hm.stamp ? k_seg_dots2_h32<true> : k_seg_dots2_h32<false>)<<<dim3((unsigned)W, (unsigned)layers), 256, 0, st>>>(
+      segs, split, F, np, a2 != nullptr, al, (const float2*)b0, (const double2*)b1, (const double2*)x, part, hm);
   BLML_CHECK_LAUNCH("history scan (float32 history)");
   k_seg_finish_dots2_split<<<dim3(F, a2 ? 2 : 1), 256, 0, st>>>(part, W, split, np, out, out2, hm);
   BLML_CHECK_LAUNCH("history scan finish");

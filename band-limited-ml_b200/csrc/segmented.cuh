@@ -32,9 +32,9 @@ __host__ __device__ inline int64_t seg_split_ints(int F) { return 2 * (int64_t)F
 int seg_split(int F, const blml_seg* segs, int* split, cudaStream_t st);
 
 // The history slots a scan covers: slot p and the slots that hold a pair (stamp >= 0) of launch row j's fit fid[j]; the
-// other slots' products are 0 and their memory is not read. stamp null: every slot.
+// other slots' products are 0 and their memory is not read. stamp null: every slot. most: no fit has more slots than that.
 struct HistMask {
-  const int* stamp; const int* fid; int m, p;
+  const int* stamp; const int* fid; int m, p, most;
   __device__ __forceinline__ bool on(int j, int q) const { return !stamp || q == p || stamp[(int64_t)fid[j] * m + q] >= 0; }
 };
 
