@@ -1261,7 +1261,8 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
       r->Sh[i] = hv + (size_t)i * tot * hsz;
       r->Yh[i] = hv + ((size_t)m + i) * tot * hsz;
     }
-    // slot 0, which the set-up's scan reads; nothing else is read before it is written
+    // slot 0, which the set-up's scan reads. (Of what is read before it is written nothing is used: a fit whose line search
+    // failed has the iteration's slot scanned whatever it holds, and k_lb_post drops those products)
     cudaMemsetAsync(r->Sh[0], 0, tot * hsz, r->st);
     cudaMemsetAsync(r->Yh[0], 0, tot * hsz, r->st);
     // >= Fa * seg_blocks_for(Fa) and SEG_SPLIT_BLOCKS + Fa for every Fa <= F

@@ -373,7 +373,9 @@ __global__ void __launch_bounds__(1024) k_seg_split(int F, const blml_seg* segs,
 // quantities of k_seg_dots2_c128 (same warp roles: warp w takes q = w, w + 8, w + 16, the last warp the norms). Each
 // thread loads 4 elements per tile (128-element tiles), twice the complex128 kernel's 2 at half the bytes each, so as
 // many bytes are in flight per thread; full tiles take unchecked loads at fixed offsets from one base, the fit's last
-// tile the checked ones. Two blocks per SM leave the registers for that without spills.
+// tile the checked ones. Two blocks per SM leave the registers for that without spills. LISTED: the slots of one list or
+// both, from the 25th on in a second layer of blocks. 64 fits of rank 4, 20 slots: one list 367 us, both 597 (two launches of
+// one list 596).
 template <bool CHECK>
 __device__ __forceinline__ void h32_tile(int64_t t, int64_t n, int lane, const float2* const* A, int na,
                                          const float2* B0, const double2* B1, const double2* X, bool norms,

@@ -530,8 +530,8 @@ __device__ __forceinline__ int sched_find(const int* off, int n, int x, int& loc
 constexpr int kFew = 4;
 struct FftFew { FftDesc d[kFew]; int n, offA[kFew + 1], offB[kFew + 1]; };
 
-// 4 CTAs per SM over many problems (the sweep's lattices 78 -> 73 us), 3 and more registers for one plan's lattices
-// (384 x 384 x 8: 36.1 -> 34.0 us)
+// 4 CTAs per SM over many problems (the sweep's lattices 78 -> 73 us, although the float64 column stage then spills 8 bytes
+// at 64 registers), 3 and more registers for one plan's lattices (384 x 384 x 8: 36.1 -> 34.0 us; 80 registers, 4 bytes)
 #define FFT_STAGE(NAME, BODY, OFF)                                                                                \
   template <typename T>                                                                                          \
   __global__ void __launch_bounds__(kFT, 4) NAME##_grp(const FftDesc* descs, const FftSched* sch) {                 \

@@ -568,7 +568,12 @@ static int check_extents(const ColMeta& cm, const int64_t* ZA, int64_t R, const 
   return extents_ok(cm, hr);
 }
 
-// column slices of a rows launch (R, M >= 1): about 16 blocks of 128 rows per SM, at least 256 columns each
+// column slices of a rows launch (R, M >= 1): about 16 blocks of 128 rows per SM, at least 256 columns each, whichever kernel
+// runs. 4 blocks per SM and 1,024 columns were slower for each, though a block of the general and multi-density kernels copies
+// all tables for its slice (us, float64, three-column bins by themselves; 600, 3,000, 12,000 bins): a ball of three columns
+// 694, 1,194, 2,385 -> 236, 314, 1,955, with tables of 133 KB 705, 1,199, 4,399 -> 239, 379, 4,182; pball x sinc 726, 1,260,
+// 2,752 -> 247, 329, 2,380; three densities of ball x sinc 1,094, 1,875, 4,105 -> 372, 485, 2,660. The partials: at most
+// 16 x 148 x 128 + R sums a density or derivative entry.
 static void rows_slices(int64_t R, int64_t M, int64_t& nsl, int64_t& slice, int64_t most = 65535) {
   const int64_t rblocks = (R + PR_THREADS - 1) / PR_THREADS;
   nsl = std::max<int64_t>(1, std::min<int64_t>((16 * 148 + rblocks - 1) / rblocks, (M + 255) / 256));

@@ -931,7 +931,7 @@ def main():
                             'peak_source': 'MEASURED_PEAKS.json hbm_gbs (of measured)' if pk else 'fallback'},
                'roofline_scan_c128': {'bound': 'hbm', 'achieved': scan['dots2']['GB/s'], 'peak': peak, 'unit': 'GB/s',
                                       'frac': scan['dots2']['GB/s'] / peak, 'traffic': scan_traffic(4),
-                                      'kernel': f"k_seg_dots2_c128<double2, double2>, the complex128 history scan of "
+                                      'kernel': f"k_seg_dots2_c128, the complex128 history scan of "
                                                 f"plain fits, {scan['dots2']['us']:.1f} us per launch"},
                'roofline_lincomb': {'bound': 'hbm', 'achieved': scan['lincomb']['GB/s'], 'peak': peak,
                                     'unit': 'GB/s', 'frac': scan['lincomb']['GB/s'] / peak,
