@@ -1088,7 +1088,9 @@ struct blml_lbfgs_batch_s : Runner {
     RC(blml_seg_lgrad_finish(dt, F, S, 1, SV, U, w, nqA, g, sv));
     RC(blml_seg_resid(dt, F, S, 1, E, U, c, scrA, part, outE, sv));
     if (h32) RC(seg_split(F, S, split, st));
-    RC(hist(F, S, 0));                                  // empty history: g . g and E . E for the first direction
+    // empty history (no slot holds a pair, whatever an earlier run left): g . g and E . E for the first direction
+    RC(cuda_status(cudaMemsetAsync(s.stamp, 0xff, sizeof(int) * (size_t)F * m, st), "lbfgs set-up"));
+    RC(hist(F, S, 0));
     k_lbi_state<<<nblk(F, 128), 128, 0, st>>>(F, m, tol, cap, d_fid, d_live, d_segs_c, d_segs_eff, outD, outE, s);
     KCHECK("lbfgs set-up");
     return BLML_OK;
@@ -1292,7 +1294,6 @@ static int lbfgs_create(int dtype, int F, const blml_seg* segs, const blml_plan*
       r->s.active = ti(1); r->s.it = ti(1); r->s.stop = ti(1); r->s.reset = ti(1); r->s.nh = ti(1); r->s.ok = ti(1);
       r->need2 = ti(1); ti(1);
       r->s.stamp = ti(m); r->s.step = z;
-      cudaMemsetAsync(r->s.stamp, 0xff, sizeof(int) * (size_t)F * m, r->st);     // -1: no pair
       rc = cuda_status(cudaMemcpyAsync(r->s.n, n, F * sizeof(double), cudaMemcpyHostToDevice, r->st), "lbfgs n");
       if (!rc) rc = cuda_status(cudaStreamSynchronize(r->st), "lbfgs create");
     }
